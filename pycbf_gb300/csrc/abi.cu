@@ -71,9 +71,23 @@ void fill_time_axis(DasArgs &a, const pycbf_gb_rfinfo *rf) {
     a.xend = rf->t0 + span2;
     a.eps = boundary_eps(rf->nt);
     {
+        // fast quotient q' = d * inv_dt (fma, one rounding) against fl(d / dt), both
+        // below 2^k: q' - 1/2 is rounded by at most 2^(k-25), inv_dt is off by the
+        // known share |inv_dt dt - 1|, and fl(d / dt) lies at most 2^(k-25) above d / dt
         int k = 0;
-        while ((1LL << k) < (long long)rf->nt) ++k;
-        a.eps_fast = std::ldexp(1.25f * 1.5f, k - 23);
+        while ((1LL << k) < (long long)rf->nt + 1) ++k;
+        const double share = std::fabs((double)a.inv_dt * (double)a.dt - 1.0);
+        a.eps_fast = std::nextafter(
+            (float)(std::ldexp(1.0, k - 24) * 1.0625 + share * (double)(rf->nt + 1)), 1.0f);
+    }
+    a.neg_zero = -0.0f;
+    {
+        // the knot cubic_taps takes for x = xmax: fma, then rounded to an integer
+        const volatile float d = a.xmax - a.t0;
+        const volatile float s = std::fmaf(d, a.inv_dt, -0.5f);
+        const volatile float r = s + 12582912.f;
+        a.fast_axis = r - 12582912.f <= (float)(rf->nt - 1) &&
+                              (long long)rf->nrx * rf->nt < (1LL << 29);
     }
     // the last knot as NVRTC compiles x0 + dx*(nx-1) in the reference's CUDA kernels
     a.xfma = std::fmaf(rf->dt, (float)(rf->nt - 1), rf->t0);

@@ -21,36 +21,42 @@ namespace {
 
 template <int GEOM, typename T, int TXC>
 __device__ __forceinline__ void batch_tile(const DasArgs &a, long long tile) {
-    using K = Kind<PYCBF_GB_INTERP_CUBIC, T>;
-    constexpr int G = (TXC < kGroup) ? TXC : kGroup;  // taps whose gathers are in flight together
+    using Rec = typename CoefRec<T>::raw;
     const long long i = tile * kBlock + threadIdx.x;
     if (i >= a.np) return;
     const long long np = a.np;
     const int ntx = a.ntx, nrx = a.nrx;
     const long long op = a.pixel_index ? (long long)__ldg(a.pixel_index + i) : i;
     const long long chs = (long long)nrx * a.nt;
+    const float inf = __int_as_float(0x7f800000);
+    const TapConst tc(a);
     float pnt[3] = {0.f, 0.f, 0.f};
     if (GEOM == GEOM_SYNTH)
         for (int k = 0; k < 3; ++k) if (k < a.ndim) pnt[k] = __ldg(a.geo.pnts + i * a.ndim + k);
 
     float acc = 0.f;
     for (int t0 = 0; t0 < ntx; t0 += TXC) {
-        float rtau[TXC], rapod[TXC];
+        float2 tt2[TXC / 2], at2[TXC / 2];
         float amax = 0.f;
 #pragma unroll
         for (int k = 0; k < TXC; ++k) {
-            rtau[k] = 0.f;
-            rapod[k] = 0.f;
+            float tau = inf, apod = 0.f;  // padding: an infinite delay never counts
             const int t = t0 + k;
             if (t < ntx) {
                 if (GEOM == GEOM_TABBED) {
-                    rtau[k] = __ldg(a.tautx + (long long)t * np + i);
-                    rapod[k] = __ldg(a.apodtx + (long long)t * np + i);
-                    amax = fmaxf(amax, fabsf(rapod[k]));
+                    tau = __ldg(a.tautx + (long long)t * np + i);
+                    apod = __ldg(a.apodtx + (long long)t * np + i);
+                    amax = fmaxf(amax, fabsf(apod));
                 } else {
-                    rtau[k] = synth_tx_delay(a, t, pnt);
-                    rapod[k] = 1.f;
+                    tau = synth_tx_delay(a, t, pnt);
                 }
+            }
+            if (k & 1) {
+                tt2[k >> 1].y = tau;
+                at2[k >> 1].y = apod;
+            } else {
+                tt2[k >> 1].x = tau;
+                at2[k >> 1].x = apod;
             }
         }
         const int nk_chunk = min(TXC, ntx - t0);
@@ -69,62 +75,24 @@ __device__ __forceinline__ void batch_tile(const DasArgs &a, long long tile) {
             } else {
                 trx = synth_rx_delay(a, r, pnt);
                 arx = 1.f;
-                live = trx != __int_as_float(0x7f800000);
+                live = trx != inf;
             }
             if (!live) continue;
-            const long long ch0 = ((long long)t0 * nrx + r) * a.nt;
-            float accr = 0.f;
+            const Rec *rec = static_cast<const Rec *>(a.data) + ((long long)t0 * nrx + r) * a.nt;
+            auto sum = CubicAcc<T>::zero();
 #pragma unroll
-            for (int g = 0; g < TXC; g += G) {
-                if (g >= nk_chunk) break;
-                const int nk = min(G, nk_chunk - g);
-                float xs[G], ap[G];
-                int ix[G];
-                unsigned hit = 0u, fix = 0u;
-#pragma unroll
-                for (int k = 0; k < G; ++k) {
-                    xs[k] = 0.f;
-                    ap[k] = 0.f;
-                    ix[k] = 0;
-                    if (k < nk) {
-                        const float x = __fadd_rn(rtau[g + k], trx);
-                        float apod = 1.f;
-                        bool h = true;
-                        if (GEOM == GEOM_TABBED) {
-                            apod = __fmul_rn(rapod[g + k], arx);
-                            h = fabsf(apod) >= a.thresh;
-                        }
-                        bool fx;
-                        int idx;
-                        const bool inr = K::index(x, a, idx, fx);
-                        xs[k] = x;
-                        ap[k] = apod;
-                        ix[k] = idx;
-                        hit |= (unsigned)(h && inr) << k;
-                        fix |= (unsigned)(h && fx) << k;
-                    }
+            for (int g = 0; g < TXC; g += kCubicGroup) {
+                if (g < nk_chunk) {
+                    const Rec *rg = rec + (long long)g * chs;
+                    if (a.fast_axis)
+                        sum = cubic_taps<GEOM, T, kCubicGroup>(a, tc, tt2 + g / 2, at2 + g / 2, trx,
+                                                               arx, rg, (unsigned)chs, sum);
+                    else
+                        sum = cubic_taps_clamped<GEOM, T, kCubicGroup>(
+                            a, tt2 + g / 2, at2 + g / 2, trx, arx, rg, chs, sum);
                 }
-                if (fix) {
-#pragma unroll
-                    for (int k = 0; k < G; ++k) {
-                        if ((fix >> k) & 1u) {
-                            int idx;
-                            const bool inr = K::index_exact(xs[k], a, idx);
-                            ix[k] = idx;
-                            hit = inr ? (hit | (1u << k)) : (hit & ~(1u << k));
-                        }
-                    }
-                }
-                typename K::P pv[G];
-#pragma unroll
-                for (int k = 0; k < G; ++k)
-                    if ((hit >> k) & 1u) pv[k] = K::load(a.data, ch0 + (long long)(g + k) * chs, ix[k], a);
-#pragma unroll
-                for (int k = 0; k < G; ++k)
-                    if ((hit >> k) & 1u)
-                        accr = fmaf(ap[k], K::value(pv[k], xs[k], (float)ix[k], a), accr);
             }
-            bacc += accr;
+            bacc += CubicAcc<T>::total(sum);
         }
         acc += bacc;
     }
@@ -165,6 +133,16 @@ batch_das_kernel(const BatchJob *__restrict__ jobs, const int2 *__restrict__ ite
     }
 }
 
+// One pixel by the single-frame kernels' cubic body in its shared-memory column
+// form, whatever the job's ntx (per-receive sums are sequential over transmits
+// either way, so the images are those of the single-frame calls bit for bit),
+// behind a call of its own so that the compiler allocates each geometry's and
+// type's registers apart from the others'.
+template <int GEOM, typename T>
+__device__ __noinline__ void batch_pixel(const DasArgs &a, long long i, float *sm) {
+    das_pixel<GEOM, PYCBF_GB_INTERP_CUBIC, PYCBF_GB_SUM_TX_AND_RX, T, false, kTxSmem>(a, i, 0, sm);
+}
+
 // The same queue, each pixel run by the single-frame kernel's body
 // (das_pixel): transmits in registers up to kTxReg, in the thread's column of
 // shared memory beyond, every receive's delay and reject computed once.  The
@@ -176,7 +154,6 @@ batch_das_full_kernel(const BatchJob *__restrict__ jobs, const int2 *__restrict_
     __shared__ __align__(16) BatchJob s_job;
     __shared__ long long s_k;
     constexpr int kWords = (int)(sizeof(BatchJob) / sizeof(int));
-    constexpr int CUB = PYCBF_GB_INTERP_CUBIC, SUM = PYCBF_GB_SUM_TX_AND_RX;
     for (;;) {
         if (threadIdx.x == 0) s_k = (long long)atomicAdd(counter, 1ULL);
         __syncthreads();
@@ -191,35 +168,23 @@ batch_das_full_kernel(const BatchJob *__restrict__ jobs, const int2 *__restrict_
         for (int sub = 0; sub < tiles_per_item; ++sub) {
             const long long i = ((long long)it.y * tiles_per_item + sub) * kBlock + threadIdx.x;
             if (geom == GEOM_TABBED) {
-                if (dtype == PYCBF_GB_F32) das_pixel<GEOM_TABBED, CUB, SUM, float, false>(s_job.a, i, 0, sm);
-                else if (dtype == PYCBF_GB_F16) das_pixel<GEOM_TABBED, CUB, SUM, __half, false>(s_job.a, i, 0, sm);
-                else das_pixel<GEOM_TABBED, CUB, SUM, __nv_bfloat16, false>(s_job.a, i, 0, sm);
+                if (dtype == PYCBF_GB_F32) batch_pixel<GEOM_TABBED, float>(s_job.a, i, sm);
+                else if (dtype == PYCBF_GB_F16) batch_pixel<GEOM_TABBED, __half>(s_job.a, i, sm);
+                else batch_pixel<GEOM_TABBED, __nv_bfloat16>(s_job.a, i, sm);
             } else {
-                if (dtype == PYCBF_GB_F32) das_pixel<GEOM_SYNTH, CUB, SUM, float, false>(s_job.a, i, 0, sm);
-                else if (dtype == PYCBF_GB_F16) das_pixel<GEOM_SYNTH, CUB, SUM, __half, false>(s_job.a, i, 0, sm);
-                else das_pixel<GEOM_SYNTH, CUB, SUM, __nv_bfloat16, false>(s_job.a, i, 0, sm);
+                if (dtype == PYCBF_GB_F32) batch_pixel<GEOM_SYNTH, float>(s_job.a, i, sm);
+                else if (dtype == PYCBF_GB_F16) batch_pixel<GEOM_SYNTH, __half>(s_job.a, i, sm);
+                else batch_pixel<GEOM_SYNTH, __nv_bfloat16>(s_job.a, i, sm);
             }
         }
         __syncthreads();  // every thread is done with s_job and s_k
     }
 }
 
-// The same for a batch of one storage type T: each pixel runs the single-frame
-// kernels' cubic body in its shared-memory column form, whatever the job's
-// ntx (the column is sized for the batch's largest ntx; per-receive sums are
-// sequential over transmits either way, so the images are those of the
-// single-frame calls bit for bit).  The kernel carries the paths of one
-// storage type only -- the mixed kernel above spills -- and each geometry's
-// body sits behind a call of its own, so the compiler allocates its registers
-// apart from the other's (one call per pixel, not per tap).  A CTA copies a
-// job's descriptor only when its next item belongs to another job.  Measured
-// on the 64-frame batch: with the register form as well for ntx <= 12 the
-// float32 kernel took 43 ms, without it 38 ms.
-template <int GEOM, typename T>
-__device__ __noinline__ void batch_pixel(const DasArgs &a, long long i, float *sm) {
-    das_pixel<GEOM, PYCBF_GB_INTERP_CUBIC, PYCBF_GB_SUM_TX_AND_RX, T, false, kTxSmem>(a, i, 0, sm);
-}
-
+// The same for a batch of one storage type T: the kernel carries the paths of
+// that type only, and a CTA copies a job's descriptor only when its next item
+// belongs to another job.  Measured on the 64-frame batch with the register form
+// as well for ntx <= 12: 43 ms, without it 38 ms.
 // five CTAs per SM for 16-bit records (42 against 43 ms), four for float32
 // records, whose body spills under five's register cap (47 against 38 ms)
 template <typename T>
@@ -259,7 +224,7 @@ batch_das_typed_kernel(const BatchJob *__restrict__ jobs, const int2 *__restrict
 // the column of every job's transmit delays (the typed kernel uses the column
 // form for every ntx, so this holds even when max_ntx <= kTxReg)
 size_t batch_full_smem_bytes(int max_ntx) {
-    return (size_t)std::max(max_ntx, 1) * kBlock * sizeof(float);
+    return (size_t)cubic_column_padded(std::max(max_ntx, 1)) * kBlock * sizeof(float);
 }
 
 cudaError_t prepare_batch_das(int max_ntx) {

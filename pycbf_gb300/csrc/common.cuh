@@ -193,9 +193,13 @@ struct DasArgs {
     long long np;
     int ntx, nrx, nt, ndim, nframes;
     float t0, dt, inv_dt, xmax, xend, thresh, eps;
-    // the staged cubic taps' floor test: 1.25 x the largest gap 1.5 |q| 2^-23
-    // between the reciprocal quotient and the IEEE quotient for |q| < nt
+    // cubic taps: a fast quotient farther than this from every integer has the floor
+    // of the IEEE quotient
     float eps_fast;
+    float neg_zero;     // -0: added to a product in an fma it keeps the product's own rounding
+    // cubic_taps applies: the fast knot of every x <= xmax is at most nt - 1, and a
+    // group's transmits are less than 2^32 records apart
+    int fast_axis;
     const float *slow;  // GEOM_SYNTH_SLOW: slowness per pixel (s/m), kernel pixel order
     float xfma;         // fma(dt, nt-1, t0): the last knot as the reference's CUDA kernels round it
     // staged kernel: SM cycles after which an mbarrier wait gives up (0: 2^31,

@@ -22,6 +22,7 @@
 //   IEEE division is taken instead.
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -335,15 +336,48 @@ __device__ __forceinline__ float synth_rx_delay(const DasArgs &a, int r, const f
     return off ? __int_as_float(0x7f800000) : __fdiv_rn(mag, a.geo.c0);
 }
 
+// synth_rx_delay for a whole warp: most receives mask every pixel of a tile, and
+// there the projection alone shows it (proj < cos(ala) |d| from the squares, with
+// a margin far above their rounding), so no root or quotient is taken.
+__device__ __forceinline__ float synth_rx_delay_warp(const DasArgs &a, int r, const float *p) {
+    const int nd = a.ndim;
+    const float *o = a.geo.ovecrx + r * nd, *n = a.geo.nvecrx + r * nd;
+    const float cosala = __ldg(a.geo.cosalarx + r);
+    float m2 = 0.f, pr = 0.f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (k < nd) {
+            const float d = __fsub_rn(p[k], __ldg(o + k));
+            m2 = __fadd_rn(m2, __fmul_rn(d, d));
+            pr = __fadd_rn(pr, __fmul_rn(d, __ldg(n + k)));
+        }
+    }
+    const bool far = (m2 > 1e-20f) && (cosala > 1e-3f) &&
+                     (pr <= 0.f || pr * pr < cosala * cosala * m2 * 0.9999f);
+    if (__all_sync(0xffffffffu, far)) return __int_as_float(0x7f800000);
+    const float mag = __fsqrt_rn(m2);
+    const bool off = (mag > kDxMin) && (__fdiv_rn(pr, mag) < cosala);
+    return off ? __int_as_float(0x7f800000) : __fdiv_rn(mag, a.geo.c0);
+}
+
 // ---------------------------------------------------------------------------
 // the kernel
 // ---------------------------------------------------------------------------
 constexpr int kGroup = 6;  // taps whose gathers a thread keeps in flight together
-// the same for the fast cubic group over transmits in shared memory: six
-// for float32 records; four for 16-bit records, whose (y, z) interpolation
-// needs more registers (groups of six cost the 3-D 25-transmit launch 11 %
-// in occupancy)
-template <typename T> constexpr int kGroupSmem = CoefRec<T>::kPoly ? 6 : 4;
+// the same for cubic sums over transmits: at six, 3.76 against 3.91 ms for 75
+// float32 transmits, but 0.83 against 0.74 ms for 31 and 122 against 112 ms for
+// 25 in float16 (registers); at eight slower throughout
+constexpr int kCubicGroup = 4;
+
+// The transmit delays of a pixel beyond kTxReg: a column of shared memory per
+// thread.  Cubic sums keep them as pairs, padded with infinite delays to whole
+// groups of kCubicGroup where that still fits; the padding of the last few
+// sizes below the limit does not, and their last transmits go one by one.
+constexpr size_t kColumnSmemMax = 227 * 1024;
+__host__ __device__ inline int cubic_column_padded(int ntx) {
+    const int full = (ntx + kCubicGroup - 1) / kCubicGroup * kCubicGroup;
+    return (size_t)full * kBlock * sizeof(float) <= kColumnSmemMax ? full : (ntx + 1) / 2 * 2;
+}
 
 // Fast knots of N cubic taps x_k = fl(tt_k + trx), decided as the staged
 // kernel decides them: delay sums and quotients q = fl(fl(x - t0) * fl(1/dt))
@@ -403,81 +437,231 @@ __device__ __forceinline__ void cubic_knots_exact(const DasArgs &a, const float 
     }
 }
 
-// Cubic taps of up to N transmits k0.. k0+nk-1 of one receive (trx, arx)
-// for the generic kernel, the decisions made as the staged kernel makes them:
-// delay sums, weights and fast quotients q = fl(fl(x - t0) * fl(1/dt)) two
-// taps per instruction; s = q - 1/2 plus 1.5 * 2^23 rounds to the knot j in
-// the sum's low bits, and where |s - j| <= 1/2 - eps_fast the fast quotient
-// and the reference's correctly rounded one floor to the same j.  A tap that
-// contributes (in range, weight past the threshold) with its quotient closer
-// to an integer is redone with the IEEE division.  Records are gathered from
-// global memory (rec: the receive's channel of transmit k0, chs elements
-// between transmits); values and the running sum are those of the generic
-// group (Kind::value, one fma per contributing tap, in transmit order), so
-// the image bits do not change.
-template <int GEOM, typename T, int N>
-__device__ __forceinline__ float generic_cubic_group(const DasArgs &a, const float *tt,
-                                                     const float *at, int nk, float trx, float arx,
-                                                     const typename CoefRec<T>::raw *rec,
-                                                     long long chs, float accr) {
-    using K = Kind<PYCBF_GB_INTERP_CUBIC, T>;
-    constexpr int NP = (N + 1) / 2;
-    const float2 trx2 = make_float2(trx, trx), arx2 = make_float2(arx, arx);
-    const float2 t02 = make_float2(a.t0, a.t0), inv2 = make_float2(a.inv_dt, a.inv_dt);
-    const float2 half2 = make_float2(0.5f, 0.5f), mag2 = make_float2(12582912.f, 12582912.f);
-    const float hmax = 0.5f - a.eps_fast;
-    float xs[N], ap[N], fj[N];
-    int jj[N];
-    unsigned hit = 0u, fix = 0u;
+// ---------------------------------------------------------------------------
+// Cubic taps summed over the transmits of one receive, for every kernel
+// (generic, batched, staged): the same operations, so the same bits.
+//
+// What bounds them is the issue rate: a tap is one gather and a handful of
+// float operations, and the L1 or shared-memory pipe is busy about a third of
+// the time.  So a tap is kept to ~14 instructions:
+//   x   = fl(tautx + taurx)                      packed, two transmits each
+//   s   = (x - t0) * 1/dt - 1/2                  packed subtract, packed fma
+//   j   = s rounded to an integer: s + 1.5 * 2^23 holds it in its low bits,
+//         and those bits scaled by the record size are the gather address
+//   xlo = fl(t0 + fl(dt j)), b = (x - xlo) / dt  packed, as the reference rounds
+//   three multiply-adds, and one into the running sum where the tap counts.
+// 192 elements x 75 transmits x 4096 samples, 512 x 1024 pixels: 2.11e9 warp
+// instructions and 3.6 ms (20 a tap, half the issue slots; the rest waits on the
+// gathers), against 3.84e9 and 4.9 ms with the tests and knots kept as bit masks,
+// 64-bit addresses and every constant fetched again.
+// Every decision is the reference's: t0 <= x <= xmax and |w| >= thresh on the
+// rounded x and w, and the knot of the correctly rounded quotient.  h = s - j is
+// within 1/2 - eps_fast of zero unless the quotient is so near an integer that
+// the two roundings could differ; a group with such a tap (a few in a hundred of
+// a warp's groups at nt = 2048) takes those taps' knots from the IEEE quotient.
+//
+// A tap that counts has 0 <= j: x >= t0 gives s >= -1/2, which rounds to 0 or
+// more; and j <= nt - 1 where the fast quotient of xmax rounds to at most nt -
+// 1, which the host checks (DasArgs::fast_axis).  On the other time axes (one
+// float step of the delay longer than half a sample) the taps go one by one
+// through cubic_tap_clamped.
+// ---------------------------------------------------------------------------
+constexpr unsigned kKnotBits = 0x4B400000u;  // 1.5 * 2^23 as an integer
+
+// the running sum over transmits: float32 records one value; 16-bit records the
+// y and the z terms of the two ends of the interval side by side
+template <typename T> struct CubicAcc {
+    using type = float2;
+    static __device__ __forceinline__ type zero() { return make_float2(0.f, 0.f); }
+    static __device__ __forceinline__ float total(type v) { return v.x + v.y; }
+};
+template <> struct CubicAcc<float> {
+    using type = float;
+    static __device__ __forceinline__ type zero() { return 0.f; }
+    static __device__ __forceinline__ float total(type v) { return v; }
+};
+
+__device__ __forceinline__ float pair_lane(const float2 *v, int k) {
+    return (k & 1) ? v[k >> 1].y : v[k >> 1].x;
+}
+
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// The constants of the taps in registers, the packed operands twice over: left
+// to itself the compiler fetches them from the argument bank for every tap.
+__device__ __forceinline__ float in_register(float v) {
+    float r;
+    asm volatile("mov.b32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float2 twice(float v) {
+    return make_float2(in_register(v), in_register(v));
+}
+struct TapConst {
+    float2 t02, inv2, dt2, nz2, mh2, mag2;
+    float t0, xmax, hmax, thresh;
+    __device__ __forceinline__ explicit TapConst(const DasArgs &a)
+        : t02(twice(a.t0)), inv2(twice(a.inv_dt)), dt2(twice(a.dt)), nz2(twice(a.neg_zero)),
+          mh2(twice(-0.5f)), mag2(twice(12582912.f)), t0(in_register(a.t0)),
+          xmax(in_register(a.xmax)), hmax(in_register(0.5f - a.eps_fast)),
+          thresh(in_register(a.thresh)) {}
+};
+
+// delay sums x, knots fj (as floats) and r (kKnotBits + j) of NP pairs of
+// transmits; a NaN or infinite x never counts, whatever its knot
+template <int NP>
+__device__ __forceinline__ void knot_pairs(const DasArgs &a, const TapConst &c, const float2 *tt2,
+                                           float trx, float2 *x2, float2 *fj2, unsigned *r) {
+    const float2 trx2 = make_float2(trx, trx);
+    float2 h2[NP];
+    float hm = 0.f;
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
-        const int k1 = (2 * p + 1 < N) ? 2 * p + 1 : 2 * p;
-        const float2 x2 = add2_rn(make_float2(tt[2 * p], tt[k1]), trx2);
-        const float2 ap2 = (GEOM == GEOM_TABBED) ? mul2_rn(make_float2(at[2 * p], at[k1]), arx2)
-                                                 : make_float2(1.f, 1.f);
-        const float2 q2 = mul2_rn(sub2_rn(x2, t02), inv2);
-        const float2 s2 = sub2_rn(q2, half2);
-        const float2 r2 = add2_rn(s2, mag2);
-        const float2 f2 = sub2_rn(r2, mag2);
-        const float2 h2 = sub2_rn(s2, f2);
+        x2[p] = add2_rn(tt2[p], trx2);
+        const float2 s2 = fma2_rn(sub2_rn(x2[p], c.t02), c.inv2, c.mh2);
+        const float2 r2 = add2_rn(s2, c.mag2);
+        fj2[p] = sub2_rn(r2, c.mag2);
+        h2[p] = sub2_rn(s2, fj2[p]);
+        hm = max3(hm, fabsf(h2[p].x), fabsf(h2[p].y));  // a NaN is passed over
+        r[2 * p] = __float_as_uint(r2.x);
+        r[2 * p + 1] = __float_as_uint(r2.y);
+    }
+    if (hm > c.hmax) {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (fabsf(h ? h2[p].y : h2[p].x) > c.hmax) {
+                    const float x = h ? x2[p].y : x2[p].x;
+                    const float fl = fminf(floorf(__fdiv_rn(__fsub_rn(x, a.t0), a.dt)),
+                                           (float)(a.nt - 1));
+                    if (h) fj2[p].y = fl;
+                    else fj2[p].x = fl;
+                    r[2 * p + h] = kKnotBits + (unsigned)(int)fl;
+                }
+            }
+        }
+    }
+}
+
+// b = (x - xlo) / dt with xlo = fl(t0 + fl(dt j)) for two transmits: the product
+// is an fma with -0 read from the arguments, so that it stays rounded on its own
+__device__ __forceinline__ float2 knot_frac2(const TapConst &c, float2 x2, float2 fj2) {
+    const float2 xlo2 = add2_rn(fma2_rn(c.dt2, fj2, c.nz2), c.t02);
+    return mul2_rn(sub2_rn(x2, xlo2), c.inv2);
+}
+
+// v(b) of a float32 record (the interval's polynomial)
+__device__ __forceinline__ float poly_value(const float4 &c, float b) {
+    return fmaf(fmaf(fmaf(c.w, b, c.z), b, c.y), b, c.x);
+}
+
+// Interpolation weights of a 16-bit record (y_j, y_j+1, z_j, z_j+1): with a =
+// (xhi - x)/dt, b = (x - xlo)/dt, wy = w (a, b) and wz = w (a^3 - a, b^3 - b).
+template <bool WEIGHTED>
+__device__ __forceinline__ void half_weights(const TapConst &c, float x, float fj, float w,
+                                             float2 &wy, float2 &wz) {
+    const float2 K = add2_rn(fma2_rn(c.dt2, make_float2(__fadd_rn(fj, 1.f), fj), c.nz2), c.t02);
+    wy = mul2_rn(sub2_rn(K, make_float2(x, x)), make_float2(c.inv2.x, -c.inv2.x));
+    const float2 t = fma2_rn(wy, wy, make_float2(-1.f, -1.f));
+    if (WEIGHTED) wy = mul2_rn(wy, make_float2(w, w));
+    wz = mul2_rn(t, wy);
+}
+
+__device__ __forceinline__ float2 half_add(const float4 &c, float2 wy, float2 wz, float2 acc) {
+    return fma2_rn(wz, make_float2(c.z, c.w), fma2_rn(wy, make_float2(c.x, c.y), acc));
+}
+
+// One tap with the IEEE quotient and its knot clamped to the channel, added
+// where it counts (time axes without fast_axis, transmits past the last whole
+// group of an unpadded column).
+template <typename T, bool WEIGHTED>
+__device__ __noinline__ typename CubicAcc<T>::type cubic_tap_clamped(
+    const DasArgs &a, float x, float w, const typename CoefRec<T>::raw *rec,
+    typename CubicAcc<T>::type acc) {
+    if (!((x >= a.t0) && (x <= a.xmax)) || (WEIGHTED && !(fabsf(w) >= a.thresh))) return acc;
+    const float fj = fminf(floorf(__fdiv_rn(__fsub_rn(x, a.t0), a.dt)), (float)(a.nt - 1));
+    const float4 c = CoefRec<T>::load(rec + (int)fj);
+    const TapConst tc(a);
+    if constexpr (CoefRec<T>::kPoly) {
+        const float v = poly_value(c, knot_frac2(tc, make_float2(x, x), make_float2(fj, fj)).x);
+        return WEIGHTED ? fmaf(w, v, acc) : acc + v;
+    } else {
+        float2 wy, wz;
+        half_weights<WEIGHTED>(tc, x, fj, w, wy, wz);
+        return half_add(c, wy, wz, acc);
+    }
+}
+
+// N taps gathered from global memory: transmits g .. g+N-1 of one receive, rec
+// the channel of transmit g, chs records between transmits (fast_axis: N chs <
+// 2^32).  Padding transmits carry infinite delays, which never count.  The
+// gather is predicated on the tap, so nothing is read for one that does not
+// count; its address is 64-bit rec plus 32-bit (j + k chs) records.
+template <int GEOM, typename T, int N>
+__device__ __forceinline__ typename CubicAcc<T>::type cubic_taps(
+    const DasArgs &a, const TapConst &c, const float2 *tt2, const float2 *at2, float trx, float arx,
+    const typename CoefRec<T>::raw *rec, unsigned chs, typename CubicAcc<T>::type acc) {
+    using raw = typename CoefRec<T>::raw;
+    constexpr int NP = (N + 1) / 2;
+    constexpr bool W = GEOM == GEOM_TABBED;
+    float2 x2[NP], fj2[NP], w2[NP];
+    unsigned r[2 * NP];
+    knot_pairs<NP>(a, c, tt2, trx, x2, fj2, r);
+    bool ok[N];
+    raw pv[N];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        if (W) w2[p] = mul2_rn(at2[p], make_float2(arx, arx));
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int k = 2 * p + h;
-            if (k < N) {
-                const float x = h ? x2.y : x2.x;
-                const float apod = h ? ap2.y : ap2.x;
-                const bool contrib = (k < nk) && (x >= a.t0) && (x <= a.xmax) &&
-                                     (GEOM != GEOM_TABBED || fabsf(apod) >= a.thresh);
-                const bool near = !(fabsf(h ? h2.y : h2.x) <= hmax);
-                xs[k] = x;
-                ap[k] = apod;
-                fj[k] = h ? f2.y : f2.x;
-                // a contributing tap has x <= xmax, so its fast knot is <= nt - 1
-                jj[k] = __float_as_int(h ? r2.y : r2.x) - 0x4B400000;
-                hit |= (unsigned)contrib << k;
-                fix |= (unsigned)(contrib && near) << k;
+            if (k >= N) continue;
+            const float x = h ? x2[p].y : x2[p].x;
+            ok[k] = (x >= c.t0) && (x <= c.xmax);
+            if (W) ok[k] = ok[k] && (fabsf(h ? w2[p].y : w2[p].x) >= c.thresh);
+            if (ok[k]) pv[k] = __ldg(rec + (r[k] + ((unsigned)k * chs - kKnotBits)));
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        float2 b2;
+        if constexpr (CoefRec<T>::kPoly) b2 = knot_frac2(c, x2[p], fj2[p]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int k = 2 * p + h;
+            if (k >= N) continue;
+            if constexpr (CoefRec<T>::kPoly) {
+                const float v = poly_value(pv[k], h ? b2.y : b2.x);
+                if (ok[k]) acc = W ? fmaf(h ? w2[p].y : w2[p].x, v, acc) : acc + v;
+            } else {
+                float2 wy, wz;
+                half_weights<W>(c, h ? x2[p].y : x2[p].x, h ? fj2[p].y : fj2[p].x,
+                                W ? (h ? w2[p].y : w2[p].x) : 1.f, wy, wz);
+                const float2 s = half_add(CoefRec<T>::unpack(pv[k]), wy, wz, acc);
+                if (ok[k]) acc = s;
             }
         }
     }
-    if (fix) {  // rare: a quotient next to a rounding boundary, redo it exactly
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-            if ((fix >> k) & 1u) {
-                int idx;
-                K::index_exact(xs[k], a, idx);
-                jj[k] = idx;
-                fj[k] = (float)idx;
-            }
-        }
-    }
-    typename K::P pv[N];
+    return acc;
+}
+
+// the same taps one by one (time axes or channel strides without fast_axis)
+template <int GEOM, typename T, int N>
+__device__ __forceinline__ typename CubicAcc<T>::type cubic_taps_clamped(
+    const DasArgs &a, const float2 *tt2, const float2 *at2, float trx, float arx,
+    const typename CoefRec<T>::raw *rec, long long chs, typename CubicAcc<T>::type acc) {
+    constexpr bool W = GEOM == GEOM_TABBED;
 #pragma unroll
     for (int k = 0; k < N; ++k)
-        if ((hit >> k) & 1u) pv[k] = CoefRec<T>::load(rec + (long long)k * chs + jj[k]);
-#pragma unroll
-    for (int k = 0; k < N; ++k)
-        if ((hit >> k) & 1u) accr = fmaf(ap[k], K::value(pv[k], xs[k], fj[k], a), accr);
-    return accr;
+        acc = cubic_tap_clamped<T, W>(a, __fadd_rn(pair_lane(tt2, k), trx),
+                                      W ? __fmul_rn(pair_lane(at2, k), arx) : 1.f,
+                                      rec + (long long)k * chs, acc);
+    return acc;
 }
 
 // Where the transmit side of a pixel lives: decided per launch from ntx
@@ -492,9 +676,17 @@ constexpr int kTxAuto = 0, kTxRegs = 1, kTxSmem = 2;
 template <int GEOM, int KIND, int SUM, typename T, bool CENSUS, int TXM = kTxAuto>
 __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, float *sm) {
     using K = Kind<KIND, T>;
+    // cubic sums over the transmits of a receive take cubic_taps; the rest (census,
+    // per-tap outputs, other kinds) the general group
+    constexpr bool kFastCubic = KIND == PYCBF_GB_INTERP_CUBIC && !CENSUS &&
+                                SUM != PYCBF_GB_SUM_NONE && SUM != PYCBF_GB_SUM_RX_ONLY;
+    constexpr unsigned kFull = 0xffffffffu;
     const int tid = threadIdx.x;
-    if (i >= a.np) return;
     const long long np = a.np;
+    // threads past the end walk the last pixel along (the receive loop votes per
+    // warp) and write nothing
+    const bool valid = i < np;
+    if (!valid) i = np - 1;
     const int ntx = a.ntx, nrx = a.nrx;
     const long long op = a.pixel_index ? (long long)__ldg(a.pixel_index + i) : i;
     const bool in_regs = TXM == kTxAuto ? ntx <= kTxReg : TXM == kTxRegs;
@@ -509,17 +701,26 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
     // transmit side: registers (ntx <= kTxReg) or this thread's column of shared memory.
     // Synthetic masks travel as +inf delays, which the range test rejects.
     float rtau[kTxReg], rapod[kTxReg], racc[kTxReg];
+    float2 tt2[kTxReg / 2], at2[kTxReg / 2];  // kFastCubic: the same in pairs
     float *stau = sm + tid;
+    float2 *spair = reinterpret_cast<float2 *>(sm) + tid;  // kFastCubic: the column in pairs
+    const int ncol = kFastCubic && !in_regs ? cubic_column_padded(ntx) : ntx;
+    const int nfast = a.fast_axis ? ncol / kCubicGroup * kCubicGroup : 0;  // taps by whole groups
+    const TapConst tc(a);
     // Tabbed transmit weights beyond kTxReg are read from the table per
     // receive (L1-resident: a tile's rows), which halves the shared memory of
     // the column form and so raises the CTAs per SM (two -> five at 75 transmits)
     float *sacc = stau + (size_t)ntx * kBlock;
     float amax = 0.f;  // max |apodtx| of this pixel, for the exact receive-level reject
+    float amin = __int_as_float(0x7f800000);  // min apodtx: the weights are all alike where it is
+    float atop = -amin;                       // also the max
     auto tx_side = [&](int t, float &tau, float &apod) {
         if (GEOM == GEOM_TABBED) {
             tau = __ldg(a.tautx + (long long)t * np + i);
             apod = __ldg(a.apodtx + (long long)t * np + i);
             amax = fmaxf(amax, fabsf(apod));
+            amin = fminf(amin, apod);
+            atop = fmaxf(atop, apod);
         } else if (GEOM == GEOM_SYNTH) {
             tau = synth_tx_delay(a, t, pnt);
             apod = 1.f;
@@ -530,24 +731,53 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
             apod = 1.f;
         }
     };
+    const float inf = __int_as_float(0x7f800000);
+    if constexpr (kFastCubic) {
+        if (in_regs) {
 #pragma unroll
-    for (int k = 0; k < kTxReg; ++k) {
-        rtau[k] = 0.f;
-        rapod[k] = 0.f;
-        racc[k] = 0.f;
-    }
-    if (in_regs) {
-#pragma unroll
-        for (int k = 0; k < kTxReg; ++k)
-            if (k < ntx) tx_side(k, rtau[k], rapod[k]);
+            for (int k = 0; k < kTxReg; ++k) {
+                float tau = inf, apod = 0.f;
+                if (k < ntx) tx_side(k, tau, apod);
+                if (k & 1) {
+                    tt2[k >> 1].y = tau;
+                    at2[k >> 1].y = apod;
+                } else {
+                    tt2[k >> 1].x = tau;
+                    at2[k >> 1].x = apod;
+                }
+            }
+        } else {
+            for (int k = 0; k < ncol; k += 2) {
+                float2 t = make_float2(inf, inf);
+                float apod;
+                if (k < ntx) tx_side(k, t.x, apod);
+                if (k + 1 < ntx) tx_side(k + 1, t.y, apod);
+                spair[(size_t)(k >> 1) * kBlock] = t;
+            }
+        }
     } else {
-        for (int k = 0; k < ntx; ++k) {
-            float tau, apod;
-            tx_side(k, tau, apod);
-            stau[(size_t)k * kBlock] = tau;
-            if (SUM == PYCBF_GB_SUM_RX_ONLY) sacc[(size_t)k * kBlock] = 0.f;
+#pragma unroll
+        for (int k = 0; k < kTxReg; ++k) {
+            rtau[k] = 0.f;
+            rapod[k] = 0.f;
+            racc[k] = 0.f;
+        }
+        if (in_regs) {
+#pragma unroll
+            for (int k = 0; k < kTxReg; ++k)
+                if (k < ntx) tx_side(k, rtau[k], rapod[k]);
+        } else {
+            for (int k = 0; k < ntx; ++k) {
+                float tau, apod;
+                tx_side(k, tau, apod);
+                stau[(size_t)k * kBlock] = tau;
+                if (SUM == PYCBF_GB_SUM_RX_ONLY) sacc[(size_t)k * kBlock] = 0.f;
+            }
         }
     }
+    // Tabbed weights beyond kTxReg: one value for every transmit of every pixel of the warp
+    // (apodtx all ones), or read from the table per tap
+    const bool one_weight = GEOM == GEOM_TABBED && __all_sync(kFull, amin == atop);
 
     float acc = 0.f, s1 = 0.f;
     float bacc = 0.f;  // TX_AND_RX: sequential sum of the current block of kRxBlockSum receives
@@ -560,7 +790,7 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
             trx = __ldg(a.taurx + (long long)r * np + i);
             arx = __ldg(a.apodrx + (long long)r * np + i);
         } else if (GEOM == GEOM_SYNTH) {
-            trx = synth_rx_delay(a, r, pnt);
+            trx = synth_rx_delay_warp(a, r, pnt);
             arx = 1.f;
         } else {
             float D;
@@ -590,9 +820,12 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
         // transmit.  A masked synthetic receive has an infinite delay.
         bool live;
         if (GEOM == GEOM_TABBED) live = __fmul_rn(amax, fabsf(arx)) >= a.thresh;
-        else live = trx != __int_as_float(0x7f800000);
-        if (!live && SUM != PYCBF_GB_SUM_NONE) {
-            if (!CENSUS && SUM == PYCBF_GB_SUM_TX_ONLY) a.out[((long long)f * nrx + r) * np + op] = 0.f;
+        else live = trx != inf;
+        // a warp leaves a receive together; the taps of a pixel that it cannot reach
+        // fail their own tests (weight below thresh, infinite delay)
+        if (SUM != PYCBF_GB_SUM_NONE && !__any_sync(kFull, live)) {
+            if (!CENSUS && SUM == PYCBF_GB_SUM_TX_ONLY && valid)
+                a.out[((long long)f * nrx + r) * np + op] = 0.f;
             continue;
         }
         const long long ch0 = (frame_ch + r) * a.nt;  // channel (tx 0, rx r)
@@ -659,7 +892,7 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
                         }
                     }
                     const int t = k0 + k;
-                    if (!CENSUS && SUM == PYCBF_GB_SUM_NONE)
+                    if (!CENSUS && SUM == PYCBF_GB_SUM_NONE && valid)
                         a.out[(((long long)f * ntx + t) * nrx + r) * np + op] = c;
                     if (SUM == PYCBF_GB_SUM_RX_ONLY) {
                         if (in_regs) {
@@ -674,57 +907,75 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
             }
         };
 
-        // cubic sums per receive: the fast-decision groups; the rest (census,
-        // per-tap outputs, other kinds) the general group
-        constexpr bool kFastCubic = KIND == PYCBF_GB_INTERP_CUBIC && !CENSUS &&
-                                    SUM != PYCBF_GB_SUM_NONE && SUM != PYCBF_GB_SUM_RX_ONLY;
-        using Rec = typename CoefRec<T>::raw;
-        const Rec *rec_r = static_cast<const Rec *>(a.data) + ch0;
-        if (in_regs) {
+        if constexpr (kFastCubic) {
+            using Rec = typename CoefRec<T>::raw;
+            const Rec *rec = static_cast<const Rec *>(a.data) + ch0;
+            auto sum = CubicAcc<T>::zero();
+            if (in_regs) {
 #pragma unroll
-            for (int g = 0; g < kTxReg; g += kGroup) {
-                if (g < ntx) {
-                    if constexpr (kFastCubic)
-                        accr = generic_cubic_group<GEOM, T, kGroup>(
-                            a, rtau + g, rapod + g, min(kGroup, ntx - g), trx, arx,
-                            rec_r + (long long)g * chs, chs, accr);
-                    else
-                        group(g, min(kGroup, ntx - g), rtau + g, rapod + g);
-                }
-            }
-        } else {
-            if constexpr (kFastCubic) {
-                for (int g = 0; g < ntx; g += kGroupSmem<T>) {
-                    const int nk = min(kGroupSmem<T>, ntx - g);
-                    float tt[kGroupSmem<T>], at[kGroupSmem<T>];
-#pragma unroll
-                    for (int k = 0; k < kGroupSmem<T>; ++k) {
-                        tt[k] = (k < nk) ? stau[(size_t)(g + k) * kBlock] : 0.f;
-                        at[k] = (GEOM == GEOM_TABBED && k < nk)
-                                    ? __ldg(a.apodtx + (long long)(g + k) * np + i)
-                                    : 1.f;
+                for (int g = 0; g < kTxReg; g += kCubicGroup) {
+                    if (g < ntx) {
+                        const Rec *rg = rec + (long long)g * chs;
+                        if (a.fast_axis)
+                            sum = cubic_taps<GEOM, T, kCubicGroup>(a, tc, tt2 + g / 2, at2 + g / 2,
+                                                                   trx, arx, rg, (unsigned)chs, sum);
+                        else
+                            sum = cubic_taps_clamped<GEOM, T, kCubicGroup>(
+                                a, tt2 + g / 2, at2 + g / 2, trx, arx, rg, chs, sum);
                     }
-                    accr = generic_cubic_group<GEOM, T, kGroupSmem<T>>(
-                        a, tt, at, nk, trx, arx, rec_r + (long long)g * chs, chs, accr);
                 }
             } else {
-                for (int g = 0; g < ntx; g += kGroup) {
-                    const int nk = min(kGroup, ntx - g);
-                    float tt[kGroup], at[kGroup];
+                int g = 0;
+                for (; g < nfast; g += kCubicGroup) {
+                    float2 t2[kCubicGroup / 2], w2[kCubicGroup / 2];
 #pragma unroll
-                    for (int k = 0; k < kGroup; ++k) {
-                        tt[k] = (k < nk) ? stau[(size_t)(g + k) * kBlock] : 0.f;
-                        at[k] = (GEOM == GEOM_TABBED && k < nk)
-                                    ? __ldg(a.apodtx + (long long)(g + k) * np + i)
-                                    : 1.f;
+                    for (int p = 0; p < kCubicGroup / 2; ++p) {
+                        t2[p] = spair[(size_t)(g / 2 + p) * kBlock];
+                        w2[p] = make_float2(amin, amin);
                     }
-                    group(g, nk, tt, at);
+                    if (GEOM == GEOM_TABBED && !one_weight) {
+                        float *w = reinterpret_cast<float *>(w2);
+#pragma unroll
+                        for (int k = 0; k < kCubicGroup; ++k)
+                            w[k] = __ldg(a.apodtx + (long long)min(g + k, ntx - 1) * np + i);
+                    }
+                    sum = cubic_taps<GEOM, T, kCubicGroup>(a, tc, t2, w2, trx, arx, rec,
+                                                           (unsigned)chs, sum);
+                    rec += kCubicGroup * chs;
                 }
+                for (; g < ntx; ++g) {  // an unpadded column's last transmits; no fast_axis: all
+                    const float2 t = spair[(size_t)(g >> 1) * kBlock];
+                    float w = 1.f;
+                    if (GEOM == GEOM_TABBED)
+                        w = __fmul_rn(__ldg(a.apodtx + (long long)g * np + i), arx);
+                    sum = cubic_tap_clamped<T, GEOM == GEOM_TABBED>(
+                        a, __fadd_rn((g & 1) ? t.y : t.x, trx), w, rec, sum);
+                    rec += chs;
+                }
+            }
+            accr = CubicAcc<T>::total(sum);
+        } else if (in_regs) {
+#pragma unroll
+            for (int g = 0; g < kTxReg; g += kGroup)
+                if (g < ntx) group(g, min(kGroup, ntx - g), rtau + g, rapod + g);
+        } else {
+            for (int g = 0; g < ntx; g += kGroup) {
+                const int nk = min(kGroup, ntx - g);
+                float tt[kGroup], at[kGroup];
+#pragma unroll
+                for (int k = 0; k < kGroup; ++k) {
+                    tt[k] = (k < nk) ? stau[(size_t)(g + k) * kBlock] : 0.f;
+                    at[k] = (GEOM == GEOM_TABBED && k < nk)
+                                ? __ldg(a.apodtx + (long long)(g + k) * np + i)
+                                : 1.f;
+                }
+                group(g, nk, tt, at);
             }
         }
 
         if (SUM == PYCBF_GB_SUM_TX_AND_RX) bacc += accr;
-        if (!CENSUS && SUM == PYCBF_GB_SUM_TX_ONLY) a.out[((long long)f * nrx + r) * np + op] = accr;
+        if (!CENSUS && SUM == PYCBF_GB_SUM_TX_ONLY && valid)
+            a.out[((long long)f * nrx + r) * np + op] = accr;
         if (SUM == PYCBF_GB_SUM_DMAS_SSR || SUM == PYCBF_GB_SUM_DMAS_POWER) {
             // pairwise sum over receives i<j of s_i s_j as sum_j s_j * (sum_{i<j} s_i):
             // no cancellation, two FMAs per receive
@@ -734,6 +985,7 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
         }
     }
 
+    if (!valid) return;
     if (SUM == PYCBF_GB_SUM_TX_AND_RX) acc += bacc;
     // census launches carry no image buffer (out is NULL): they store counts only
     if (!CENSUS && (SUM == PYCBF_GB_SUM_TX_AND_RX || SUM == PYCBF_GB_SUM_DMAS_SSR ||
@@ -768,7 +1020,8 @@ inline size_t das_smem_bytes(int geom, int sum, int ntx) {
     (void)geom;
     if (ntx <= kTxReg) return 0;
     const size_t per = 1 + (sum == PYCBF_GB_SUM_RX_ONLY ? 1 : 0);
-    return per * (size_t)ntx * kBlock * sizeof(float);
+    const size_t cols = per > 1 ? per * (size_t)ntx : (size_t)std::max(ntx, cubic_column_padded(ntx));
+    return cols * kBlock * sizeof(float);
 }
 
 template <int GEOM, int KIND, int SUM, typename T, bool CENSUS, int TXM>

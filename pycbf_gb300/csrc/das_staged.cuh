@@ -333,10 +333,6 @@ constexpr int kTapGroup = 4;
 // indices, otherwise from global memory.  A tap whose quotient lies within
 // a few ulp of a rounding boundary has its index redone with the IEEE
 // division; the group branches only when some tap needs it.
-__device__ __forceinline__ float pair_lane(const float2 *v, int k) {
-    return (k & 1) ? v[k >> 1].y : v[k >> 1].x;
-}
-
 template <int KIND, typename T, bool STAGED, int N>
 __device__ __forceinline__ float staged_group(const DasArgs &a, const float2 *tt2, const float2 *at2,
                                               float trx, float arx, const int *bk,
@@ -434,99 +430,62 @@ __device__ __forceinline__ float staged_group(const DasArgs &a, const float2 *tt
     return accr;
 }
 
-// Cubic taps from float32 polynomial records in a stage: N <= kTapGroup
-// transmits of receive (trx, arx), their delays and weights as float32 pairs
-// tt2/at2 (the pair's second lane past N is padding), sb[k] the element base
-// of transmit k's window in the stage.  The delay sums, weights and quotients
-// are formed two taps per instruction (each lane rounded as the scalar
-// operation).  The knot: for the fast quotient q = fl(fl(x - t0) * fl(1/dt)),
-// s = q - 1/2 is exact for 0 <= q < 2^22, and adding 1.5 * 2^23 rounds it to
-// an integer j held in the low bits of the sum, so h = s - j lies in
-// [-1/2, 1/2].  Where |h| <= 1/2 - eps_fast (eps_fast exceeds 1.5 |q| 2^-23,
-// the largest gap between q and the reference's correctly rounded quotient
-// fl(fl(x - t0) / dt), for every q below nt), both quotients lie strictly
-// between j and j + 1, so j is the reference's knot; the sum's bit pattern
-// minus that of 1.5 * 2^23 is j itself.  A group holding any other tap (q
-// within eps_fast of an integer; NaN and infinite delays too) takes
-// staged_cubic_exact instead, which decides every tap with the IEEE division.
-// The two paths share nothing after the branch but the running sum, so the
-// common one carries no merge of gathered records.
-template <int N>
-__device__ __forceinline__ float staged_cubic_exact(const DasArgs &a, const float2 *tt2,
-                                                 const float2 *at2, float trx, float arx,
-                                                 const int *sb, const float4 *stage, float accr) {
-    constexpr unsigned cap = kStageBytes / sizeof(float4);
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-        const float x = __fadd_rn(pair_lane(tt2, k), trx);
-        const float apod = __fmul_rn(pair_lane(at2, k), arx);
-        const float fl = floorf(__fdiv_rn(__fsub_rn(x, a.t0), a.dt));
-        const int j = (int)fminf(fmaxf(fl, -1.f), (float)a.nt);  // NaN: -1
-        const float4 c = stage[min((unsigned)(sb[k] + j), cap - 1u)];
-        const float xlo = __fadd_rn(a.t0, __fmul_rn(a.dt, fl));
-        const float b = __fmul_rn(__fsub_rn(x, xlo), a.inv_dt);
-        const float v = fmaf(fmaf(fmaf(c.w, b, c.z), b, c.y), b, c.x);
-        const bool ok = (x >= a.t0) && (x <= a.xmax) && (fabsf(apod) >= a.thresh);
-        const float r = fmaf(apod, v, accr);
-        accr = ok ? r : accr;
-    }
-    return accr;
+// a record at a byte address of the CTA's shared memory, whose last record starts at
+// `last`: a tap outside its window cannot occur, and if it did it would read a
+// wrong value inside the CTA's memory, never outside
+__device__ __forceinline__ float4 lds_record(unsigned addr, unsigned last, const float4 *) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(min(addr, last)));
+    return v;
+}
+__device__ __forceinline__ uint2 lds_record(unsigned addr, unsigned last, const uint2 *) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(min(addr, last)));
+    return v;
 }
 
-template <int N>
-__device__ __forceinline__ float staged_cubic_group(const DasArgs &a, const float2 *tt2,
-                                                    const float2 *at2, float trx, float arx,
-                                                    const int *sb, const float4 *stage,
-                                                    float accr) {
-    constexpr unsigned cap = kStageBytes / sizeof(float4);
+// cubic_taps with the records in a stage: sb[k] is the byte address of transmit
+// k's window minus (kKnotBits + its first record) records, so the knot's bits,
+// scaled, lead to the record.  Every tap gathers (at a clamped address); those
+// that count are added.
+template <typename T, int N>
+__device__ __forceinline__ typename CubicAcc<T>::type staged_taps(
+    const DasArgs &a, const TapConst &c, const float2 *tt2, const float2 *at2, float trx, float arx,
+    const unsigned *sb, unsigned last, typename CubicAcc<T>::type acc) {
+    using raw = typename CoefRec<T>::raw;
     constexpr int NP = (N + 1) / 2;
-    const float2 trx2 = make_float2(trx, trx), arx2 = make_float2(arx, arx);
-    const float2 t02 = make_float2(a.t0, a.t0), inv2 = make_float2(a.inv_dt, a.inv_dt);
-    const float2 half2 = make_float2(0.5f, 0.5f), mag2 = make_float2(12582912.f, 12582912.f);
-    const float hmax = 0.5f - a.eps_fast;
-    float2 x2[NP], ap2[NP], fj2[NP];
-    int e[2 * NP];
-    bool nearb = false;
+    float2 x2[NP], fj2[NP], w2[NP];
+    unsigned r[2 * NP];
+    knot_pairs<NP>(a, c, tt2, trx, x2, fj2, r);
+    raw pv[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+        pv[k] = lds_record(r[k] * (unsigned)sizeof(raw) + sb[k], last, static_cast<raw *>(nullptr));
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
-        x2[p] = add2_rn(tt2[p], trx2);
-        ap2[p] = mul2_rn(at2[p], arx2);
-        const float2 q2 = mul2_rn(sub2_rn(x2[p], t02), inv2);
-        const float2 s2 = sub2_rn(q2, half2);
-        const float2 r2 = add2_rn(s2, mag2);
-        fj2[p] = sub2_rn(r2, mag2);
-        const float2 h2 = sub2_rn(s2, fj2[p]);
-        e[2 * p] = sb[2 * p] + (__float_as_int(r2.x) - 0x4B400000);
-        e[2 * p + 1] = sb[2 * p + 1] + (__float_as_int(r2.y) - 0x4B400000);
-        nearb |= !(fabsf(h2.x) <= hmax);
-        if (2 * p + 1 < N) nearb |= !(fabsf(h2.y) <= hmax);
-    }
-    if (nearb) return staged_cubic_exact<N>(a, tt2, at2, trx, arx, sb, stage, accr);
-    float4 pv[N];
-#pragma unroll
-    for (int k = 0; k < N; ++k) pv[k] = stage[min((unsigned)e[k], cap - 1u)];
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        // b = (x - xlo) / dt, xlo = fl(t0 + fl(dt j)) as the reference rounds the
-        // knot (two scalar roundings: no product feeds a packed add)
-        const float2 xlo2 = make_float2(__fadd_rn(a.t0, __fmul_rn(a.dt, fj2[p].x)),
-                                        __fadd_rn(a.t0, __fmul_rn(a.dt, fj2[p].y)));
-        const float2 b2 = mul2_rn(sub2_rn(x2[p], xlo2), inv2);
+        w2[p] = mul2_rn(at2[p], make_float2(arx, arx));
+        float2 b2;
+        if constexpr (CoefRec<T>::kPoly) b2 = knot_frac2(c, x2[p], fj2[p]);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int k = 2 * p + h;
-            if (k < N) {
-                const float b = h ? b2.y : b2.x;
-                const float x = h ? x2[p].y : x2[p].x;
-                const float apod = h ? ap2[p].y : ap2[p].x;
-                const float v = fmaf(fmaf(fmaf(pv[k].w, b, pv[k].z), b, pv[k].y), b, pv[k].x);
-                const bool ok = (x >= a.t0) && (x <= a.xmax) && (fabsf(apod) >= a.thresh);
-                const float c = fmaf(apod, v, accr);
-                accr = ok ? c : accr;
+            if (k >= N) continue;
+            const float x = h ? x2[p].y : x2[p].x, w = h ? w2[p].y : w2[p].x;
+            const bool ok = (x >= c.t0) && (x <= c.xmax) && (fabsf(w) >= c.thresh);
+            if constexpr (CoefRec<T>::kPoly) {
+                const float v = poly_value(pv[k], h ? b2.y : b2.x);
+                if (ok) acc = fmaf(w, v, acc);
+            } else {
+                float2 wy, wz;
+                half_weights<true>(c, x, h ? fj2[p].y : fj2[p].x, w, wy, wz);
+                const float2 s = half_add(CoefRec<T>::unpack(pv[k]), wy, wz, acc);
+                if (ok) acc = s;
             }
         }
     }
-    return accr;
+    return acc;
 }
 
 // Delay gradients of N <= kTapGroup cubic taps of receive (trx, arx), the
@@ -536,73 +495,45 @@ __device__ __forceinline__ float staged_cubic_group(const DasArgs &a, const floa
 // polynomial record; d is added into gt[k] (this pixel's dL/dtautx of the
 // group's transmit k, over receives in order) and into the returned gr
 // (dL/dtaurx, over transmits in order).  Records come from the stage
-// (STAGED; sb the element bases of the windows in the stage) or from global memory
+// (STAGED; sb as in staged_taps) or from global memory
 // (grec: the record row of the group's first transmit, chs between
 // transmits).
 template <int N, bool STAGED>
-__device__ __forceinline__ float adj_cubic_group(const DasArgs &a, const float2 *tt2,
-                                                 const float2 *at2, float trx, float arx, float gp,
-                                                 const int *sb, const float4 *stage,
+__device__ __forceinline__ float adj_cubic_group(const DasArgs &a, const TapConst &c,
+                                                 const float2 *tt2, const float2 *at2, float trx, float arx, float gp,
+                                                 const unsigned *sb, unsigned last,
                                                  const float4 *grec, long long chs, float *gt,
                                                  float gr) {
-    constexpr unsigned cap = kStageBytes / sizeof(float4);
     constexpr int NP = (N + 1) / 2;
-    const float2 trx2 = make_float2(trx, trx), arx2 = make_float2(arx, arx);
-    const float2 t02 = make_float2(a.t0, a.t0), inv2 = make_float2(a.inv_dt, a.inv_dt);
-    const float2 half2 = make_float2(0.5f, 0.5f), mag2 = make_float2(12582912.f, 12582912.f);
-    const float hmax = 0.5f - a.eps_fast;
-    float2 x2[NP], ap2[NP], fj2[NP];
-    int jj[2 * NP];
-    bool nearb = false;
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        x2[p] = add2_rn(tt2[p], trx2);
-        ap2[p] = mul2_rn(at2[p], arx2);
-        const float2 s2 = sub2_rn(mul2_rn(sub2_rn(x2[p], t02), inv2), half2);
-        const float2 r2 = add2_rn(s2, mag2);
-        fj2[p] = sub2_rn(r2, mag2);
-        const float2 h2 = sub2_rn(s2, fj2[p]);
-        jj[2 * p] = __float_as_int(r2.x) - 0x4B400000;
-        jj[2 * p + 1] = __float_as_int(r2.y) - 0x4B400000;
-        nearb |= !(fabsf(h2.x) <= hmax);
-        if (2 * p + 1 < N) nearb |= !(fabsf(h2.y) <= hmax);
-    }
-    if (nearb) {  // rare: every tap of the group with the IEEE quotient
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-            const float x = (k & 1) ? x2[k >> 1].y : x2[k >> 1].x;
-            const float fl = floorf(__fdiv_rn(__fsub_rn(x, a.t0), a.dt));
-            jj[k] = (int)fminf(fmaxf(fl, -1.f), (float)a.nt);  // NaN: -1
-            if (k & 1) fj2[k >> 1].y = fl;
-            else fj2[k >> 1].x = fl;
-        }
-    }
+    float2 x2[NP], fj2[NP];
+    unsigned r[2 * NP];
+    knot_pairs<NP>(a, c, tt2, trx, x2, fj2, r);
     float4 pv[N];
 #pragma unroll
     for (int k = 0; k < N; ++k) {
         if (STAGED) {
-            pv[k] = stage[min((unsigned)(sb[k] + jj[k]), cap - 1u)];
+            pv[k] = lds_record(r[k] * (unsigned)sizeof(float4) + sb[k], last,
+                               static_cast<float4 *>(nullptr));
         } else {
-            const int j = min(max(jj[k], 0), a.nt - 1);
+            const int j = min(max((int)(r[k] - kKnotBits), 0), a.nt - 1);
             pv[k] = __ldg(grec + k * chs + j);
         }
     }
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
-        const float2 xlo2 = make_float2(__fadd_rn(a.t0, __fmul_rn(a.dt, fj2[p].x)),
-                                        __fadd_rn(a.t0, __fmul_rn(a.dt, fj2[p].y)));
-        const float2 b2 = mul2_rn(sub2_rn(x2[p], xlo2), inv2);
+        const float2 w2 = mul2_rn(at2[p], make_float2(arx, arx));
+        const float2 b2 = knot_frac2(c, x2[p], fj2[p]);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int k = 2 * p + h;
             if (k < N) {
                 const float b = h ? b2.y : b2.x;
                 const float x = h ? x2[p].y : x2[p].x;
-                const float apod = h ? ap2[p].y : ap2[p].x;
+                const float apod = h ? w2.y : w2.x;
                 const float slope =
                     fmaf(fmaf(3.f * pv[k].w, b, 2.f * pv[k].z), b, pv[k].y) * a.inv_dt;
                 const float d = apod * (gp * slope);
-                const bool ok = (x >= a.t0) && (x <= a.xmax) && (fabsf(apod) >= a.thresh);
+                const bool ok = (x >= c.t0) && (x <= c.xmax) && (fabsf(apod) >= c.thresh);
                 if (ok) {
                     gt[k] += d;
                     gr += d;
@@ -638,13 +569,13 @@ template <int KIND, int SUM, typename T, bool ADJ = false>
 __global__ void __launch_bounds__(kBlock, ADJ ? 4 : 5) das_staged_kernel(const __grid_constant__ DasArgs a,
                                                               int *__restrict__ plan) {
     using E = typename StagedElem<KIND, T>::E;
-    constexpr bool kPolyCubic = KIND == PYCBF_GB_INTERP_CUBIC && CoefRec<T>::kPoly;
+    constexpr bool kCubic = KIND == PYCBF_GB_INTERP_CUBIC;
     constexpr int kWarps = kBlock / 32;
     constexpr unsigned kFull = 0xffffffffu;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long full[kStages];
     __shared__ __align__(8) unsigned long long empty[kStages];
-    __shared__ __align__(16) int sbase[kStages][kTxReg];  // element base of each window - its e0
+    __shared__ __align__(16) unsigned sbase[kStages][kTxReg];  // see `produce`
     __shared__ int sstaged[kStages];
     __shared__ int s_copies[kStages];  // the slot's latest phase has bulk copies in flight
     __shared__ int s_failed;
@@ -667,6 +598,9 @@ __global__ void __launch_bounds__(kBlock, ADJ ? 4 : 5) das_staged_kernel(const _
     int *counters = plan + L.counters;
     float *partials = reinterpret_cast<float *>(plan + L.partials);
     unsigned *queue = reinterpret_cast<unsigned *>(plan + 1);
+    const TapConst tc(a);
+    const unsigned stage0 = smem_u32(smem_raw);  // the stages, and the last record's address
+    const unsigned last_rec = stage0 + kStages * kStageBytes - (unsigned)sizeof(E);
     const long long wait_lim = a.wait_cycles > 0 ? a.wait_cycles : (1LL << 31);
 
     if (tid < kStages) {
@@ -730,7 +664,13 @@ __global__ void __launch_bounds__(kBlock, ADJ ? 4 : 5) das_staged_kernel(const _
                 if (lane >= o) off += v;
             }
             off -= cnt;
-            if (lane < kTxReg) sbase[slot][lane] = (staged && lane < ntx) ? off - e0 : 0;
+            // where the taps find the window.  Cubic: the byte address of its first record
+            // less e0 and kKnotBits records (staged_taps); else its offset in the stage less e0
+            if (lane < kTxReg)
+                sbase[slot][lane] =
+                    kCubic ? stage0 + (unsigned)slot * kStageBytes +
+                                 ((unsigned)(off - e0) - kKnotBits) * (unsigned)sizeof(E)
+                           : (staged && lane < ntx ? (unsigned)(off - e0) : 0u);
             // stall test: the item's first receive announces its bytes (at least 16)
             // and issues no copy, so its phase never completes and nothing is in flight
             const bool stall = a.stall_test && it == 0;
@@ -775,7 +715,7 @@ __global__ void __launch_bounds__(kBlock, ADJ ? 4 : 5) das_staged_kernel(const _
         float amax = 0.f;
 #pragma unroll
         for (int k = 0; k < kTxReg; ++k) {
-            float tv = a.t0, av = 0.f;
+            float tv = kCubic ? __int_as_float(0x7f800000) : a.t0, av = 0.f;
             if (k < ntx && valid) {
                 tv = __ldg(a.tautx + (long long)k * np + i);
                 av = __ldg(a.apodtx + (long long)k * np + i);
@@ -843,13 +783,11 @@ __global__ void __launch_bounds__(kBlock, ADJ ? 4 : 5) das_staged_kernel(const _
                 if (live) {
                     const long long chs = (long long)nrx * a.nt;
                     const float4 *grow = static_cast<const float4 *>(a.data) + (frame_ch + r) * a.nt;
-                    const bool stg = sstaged[slot] != 0;
-                    const float4 *st4 =
-                        reinterpret_cast<const float4 *>(smem_raw + (size_t)slot * kStageBytes);
-                    int sb[kTxReg];
+                    const bool stg = sstaged[slot] != 0 && a.fast_axis;
+                    unsigned sb[kTxReg];
 #pragma unroll
                     for (int g = 0; g < kTxReg; g += 4) {
-                        const int4 b = *reinterpret_cast<const int4 *>(&sbase[slot][g]);
+                        const uint4 b = *reinterpret_cast<const uint4 *>(&sbase[slot][g]);
                         sb[g] = b.x;
                         sb[g + 1] = b.y;
                         sb[g + 2] = b.z;
@@ -860,7 +798,7 @@ __global__ void __launch_bounds__(kBlock, ADJ ? 4 : 5) das_staged_kernel(const _
                         if (g < ntx) {
                             const int rem = ntx - g;
 #define PGB_AGROUP(n, st)                                                                         \
-    adj_cubic_group<n, st>(a, tt2 + g / 2, at2 + g / 2, trx, arx, gp, sb + g, st4,                \
+    adj_cubic_group<n, st>(a, tc, tt2 + g / 2, at2 + g / 2, trx, arx, gp, sb + g, last_rec,           \
                            grow + (long long)g * chs, chs, gt + g, gr)
                             if (stg) {
                                 if (rem >= 4) gr = PGB_AGROUP(4, true);
@@ -879,52 +817,64 @@ __global__ void __launch_bounds__(kBlock, ADJ ? 4 : 5) das_staged_kernel(const _
                 }
                 if (valid && a.grx) a.grx[(long long)r * np + i] = gr;
             } else if (live) {
-                if (sstaged[slot]) {
-                    const E *stage = reinterpret_cast<const E *>(smem_raw + (size_t)slot * kStageBytes);
-                    int sb[kTxReg];
+                const long long ch_first = (frame_ch + r) * a.nt;
+                const long long chs = (long long)nrx * a.nt;
+                unsigned sb[kTxReg];
 #pragma unroll
-                    for (int g = 0; g < kTxReg; g += 4) {
-                        const int4 b = *reinterpret_cast<const int4 *>(&sbase[slot][g]);
-                        sb[g] = b.x;
-                        sb[g + 1] = b.y;
-                        sb[g + 2] = b.z;
-                        sb[g + 3] = b.w;
-                    }
+                for (int g = 0; g < kTxReg; g += 4) {
+                    const uint4 b = *reinterpret_cast<const uint4 *>(&sbase[slot][g]);
+                    sb[g] = b.x;
+                    sb[g + 1] = b.y;
+                    sb[g + 2] = b.z;
+                    sb[g + 3] = b.w;
+                }
+                if constexpr (kCubic) {
+                    auto sum = CubicAcc<T>::zero();
+                    if (sstaged[slot] && a.fast_axis) {
 #pragma unroll
-                    for (int g = 0; g < kTxReg; g += kTapGroup) {
-                        if (g < ntx) {
-                            // the last group holds only the transmits left (no padded tap)
-                            const int rem = ntx - g;
-                            if constexpr (kPolyCubic) {
-                                const float4 *st4 = reinterpret_cast<const float4 *>(stage);
-#define PGB_CGROUP(n) staged_cubic_group<n>(a, tt2 + g / 2, at2 + g / 2, trx, arx, sb + g, st4, accr)
-                                if (rem >= 4) accr = PGB_CGROUP(4);
-                                else if (rem == 3) accr = PGB_CGROUP(3);
-                                else if (rem == 2) accr = PGB_CGROUP(2);
-                                else accr = PGB_CGROUP(1);
+                        for (int g = 0; g < kTxReg; g += kTapGroup) {
+                            if (g < ntx) {
+                                // the last group holds only the transmits left (no padded tap)
+                                const int rem = ntx - g;
+#define PGB_CGROUP(n) staged_taps<T, n>(a, tc, tt2 + g / 2, at2 + g / 2, trx, arx, sb + g, last_rec, sum)
+                                if (rem >= 4) sum = PGB_CGROUP(4);
+                                else if (rem == 3) sum = PGB_CGROUP(3);
+                                else if (rem == 2) sum = PGB_CGROUP(2);
+                                else sum = PGB_CGROUP(1);
 #undef PGB_CGROUP
-                            } else {
-#define PGB_GROUP(n)                                                                              \
-    staged_group<KIND, T, true, n>(a, tt2 + g / 2, at2 + g / 2, trx, arx, sb + g, stage, 0, 0, g, ntx, \
-                                   accr)
-                                if (rem >= 4) accr = PGB_GROUP(4);
-                                else if (rem == 3) accr = PGB_GROUP(3);
-                                else if (rem == 2) accr = PGB_GROUP(2);
-                                else accr = PGB_GROUP(1);
-#undef PGB_GROUP
                             }
                         }
+                    } else {
+                        const E *rec = static_cast<const E *>(a.data) + ch_first;
+#pragma unroll
+                        for (int g = 0; g < kTxReg; g += kTapGroup)
+                            if (g < ntx)
+                                sum = a.fast_axis
+                                          ? cubic_taps<GEOM_TABBED, T, kTapGroup>(
+                                                a, tc, tt2 + g / 2, at2 + g / 2, trx, arx,
+                                                rec + (long long)g * chs, (unsigned)chs, sum)
+                                          : cubic_taps_clamped<GEOM_TABBED, T, kTapGroup>(
+                                                a, tt2 + g / 2, at2 + g / 2, trx, arx,
+                                                rec + (long long)g * chs, chs, sum);
                     }
+                    accr = CubicAcc<T>::total(sum);
                 } else {
-                    const long long ch_first = (frame_ch + r) * a.nt;
-                    const long long chs = (long long)nrx * a.nt;
+                    const E *stage = reinterpret_cast<const E *>(smem_raw + (size_t)slot * kStageBytes);
+                    const bool stg = sstaged[slot] != 0;
 #pragma unroll
                     for (int g = 0; g < kTxReg; g += kTapGroup) {
                         if (g < ntx) {
-                            const int bk[kTapGroup] = {0, 0, 0, 0};
-                            accr = staged_group<KIND, T, false, kTapGroup>(a, tt2 + g / 2, at2 + g / 2, trx,
-                                                                arx, bk, nullptr, ch_first, chs, g,
-                                                                ntx, accr);
+                            const int rem = ntx - g;
+                            const int *sbi = reinterpret_cast<const int *>(sb) + g;
+#define PGB_GROUP(st, n)                                                                          \
+    staged_group<KIND, T, st, n>(a, tt2 + g / 2, at2 + g / 2, trx, arx, sbi, stage, ch_first, chs, g, \
+                                 ntx, accr)
+                            if (!stg) accr = PGB_GROUP(false, kTapGroup);
+                            else if (rem >= 4) accr = PGB_GROUP(true, 4);
+                            else if (rem == 3) accr = PGB_GROUP(true, 3);
+                            else if (rem == 2) accr = PGB_GROUP(true, 2);
+                            else accr = PGB_GROUP(true, 1);
+#undef PGB_GROUP
                         }
                     }
                 }
