@@ -189,6 +189,53 @@ int prepare_data(const pycbf_gb_rfinfo *rf, const void *rfdata, int interp, void
     return PYCBF_GB_OK;
 }
 
+// Cubic images of several frames, in groups that share the decisions of a tap
+// (das_frames.cuh): the largest groups first, each prefiltered and summed in turn,
+// while at least `least` frames are left.  On return rf, rfdata, workspace and a.out
+// stand for the frames left to the single-frame kernels, if any.  The groups'
+// records take the space of the single frames' ones, so the workspace is no larger.
+//
+// Groups of four; of eight for 16-bit records of up to a gigabyte (eight Tabbed
+// float16 frames 0.85 against 0.94 ms; eight 3-D volumes, 3.4 GB, 56 against 54 ms).
+int take_frame_groups(pycbf_gb_rfinfo *rf, const void **rfdata, int geom, DasArgs &a, int sumtype,
+                      int least, void **workspace, size_t *workspace_bytes, cudaStream_t s) {
+    if (rf->nframes < least || !das_frames_ok(a, sumtype) || !spline_pairs_fit(rf->nt))
+        return PYCBF_GB_OK;
+    if (!*workspace || *workspace_bytes < pycbf_gb_workspace_bytes(rf, PYCBF_GB_INTERP_CUBIC))
+        return PYCBF_GB_EWORKSPACE;
+    if (reinterpret_cast<uintptr_t>(*workspace) % 16) return PYCBF_GB_EINVAL;
+    const int gdt = rf->dtype == PYCBF_GB_I16 ? PYCBF_GB_F32 : rf->dtype;
+    const size_t nch = (size_t)rf->ntx * rf->nrx, frame = nch * rf->nt;
+    const size_t rec = gdt == PYCBF_GB_F32 ? 16 : 8;
+    const size_t img = sumtype == PYCBF_GB_SUM_TX_ONLY ? (size_t)rf->nrx * a.np : (size_t)a.np;
+    const int most = gdt != PYCBF_GB_F32 && 8 * frame * rec <= ((size_t)1 << 30) ? 8 : 4;
+    while (rf->nframes >= least) {
+        int fg = most;
+        while (fg > rf->nframes) fg /= 2;
+        const int n = (int)rf->nframes / fg * fg;
+        SplineArgs sa;
+        sa.rf = *rfdata;
+        sa.coef = *workspace;
+        sa.nch = (long long)nch;
+        sa.nt = rf->nt;
+        sa.t0 = rf->t0;
+        sa.dt = rf->dt;
+        sa.nframes = n;
+        int st = cuda_status(launch_spline_pairs(sa, rf->dtype, s));
+        if (st) return st;
+        a.data = sa.coef;
+        a.nframes = n;
+        st = cuda_status(launch_das_frames(a, geom, sumtype, gdt, fg, s));
+        if (st) return st;
+        rf->nframes -= n;
+        *rfdata = static_cast<const char *>(*rfdata) + (size_t)n * frame * dtype_bytes(rf->dtype);
+        *workspace = static_cast<char *>(*workspace) + (size_t)n * frame * rec;
+        *workspace_bytes -= (size_t)n * frame * rec;
+        a.out += (size_t)n * img;
+    }
+    return PYCBF_GB_OK;
+}
+
 // the kernels' interpolation kind of an interp code (akima and makima share
 // their gather: they differ only in the prefilter)
 int gather_kind(int interp) {
@@ -293,13 +340,8 @@ int pycbf_gb_das_tabbed(const pycbf_gb_rfinfo *rf, const void *rfdata, const flo
     if (std::isnan(thresh)) return PYCBF_GB_EINVAL;
     if (!das_shape_ok(GEOM_TABBED, sumtype, rf->ntx)) return PYCBF_GB_ERANGE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const void *data = nullptr;
-    pycbf_gb_rfinfo eff;
-    st = prepare_data(rf, rfdata, interp, workspace, workspace_bytes, s, &data, &eff);
-    if (st) return st;
     DasArgs a = {};
     fill_time_axis(a, rf);
-    a.data = data;
     a.tautx = tautx;
     a.apodtx = apodtx;
     a.taurx = taurx;
@@ -308,6 +350,25 @@ int pycbf_gb_das_tabbed(const pycbf_gb_rfinfo *rf, const void *rfdata, const flo
     a.out = out;
     a.np = np;
     a.thresh = thresh;
+    pycbf_gb_rfinfo one = *rf;  // what the groups of frames leave
+    if (interp == PYCBF_GB_INTERP_CUBIC) {
+        // with a staging plan the staged kernel is as fast for fewer frames (float32: 4
+        // frames 0.59 against 0.61 ms, 8 1.11 against 1.01; float16: 2 0.35 against
+        // 0.49, 4 0.62 against 0.59)
+        pycbf_gb_rfinfo rec = *rf;
+        if (rf->dtype == PYCBF_GB_I16) rec.dtype = PYCBF_GB_F32;
+        const bool staged = plan && staged_ok(&rec, interp, sumtype, workspace);
+        const int least = !staged ? 2 : rec.dtype == PYCBF_GB_F32 ? 8 : 4;
+        st = take_frame_groups(&one, &rfdata, GEOM_TABBED, a, sumtype, least, &workspace,
+                               &workspace_bytes, s);
+        if (st || one.nframes == 0) return st;
+    }
+    const void *data = nullptr;
+    pycbf_gb_rfinfo eff;
+    st = prepare_data(&one, rfdata, interp, workspace, workspace_bytes, s, &data, &eff);
+    if (st) return st;
+    a.data = data;
+    a.nframes = (int)one.nframes;
     return launch_tabbed(&eff, a, interp, sumtype, plan, s);
 }
 
@@ -380,19 +441,26 @@ int pycbf_gb_das_synthetic(const pycbf_gb_rfinfo *rf, const void *rfdata,
     if (interp < 0 || interp > 3 || sumtype < 0 || sumtype > 5) return PYCBF_GB_EINVAL;
     if (!das_shape_ok(GEOM_SYNTH, sumtype, rf->ntx)) return PYCBF_GB_ERANGE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const void *data = nullptr;
-    pycbf_gb_rfinfo eff;
-    st = prepare_data(rf, rfdata, interp, workspace, workspace_bytes, s, &data, &eff);
-    if (st) return st;
     DasArgs a = {};
     fill_time_axis(a, rf);
-    a.data = data;
     a.geo = *geo;
     a.ndim = rf->ndim;
     a.pixel_index = pixel_index;
     a.out = out;
     a.np = geo->np;
     a.thresh = 0.01f;
+    pycbf_gb_rfinfo one = *rf;  // what the groups of frames leave
+    if (interp == PYCBF_GB_INTERP_CUBIC) {
+        st = take_frame_groups(&one, &rfdata, GEOM_SYNTH, a, sumtype, 2, &workspace, &workspace_bytes,
+                               s);
+        if (st || one.nframes == 0) return st;
+    }
+    const void *data = nullptr;
+    pycbf_gb_rfinfo eff;
+    st = prepare_data(&one, rfdata, interp, workspace, workspace_bytes, s, &data, &eff);
+    if (st) return st;
+    a.data = data;
+    a.nframes = (int)one.nframes;
     return cuda_status(launch_das(a, GEOM_SYNTH, interp, sumtype, eff.dtype, false, s));
 }
 

@@ -166,8 +166,13 @@ struct SplineArgs {
     long long nch;
     int nt;
     float t0, dt;            // the time axis (the float32 records depend on the knots)
+    int nframes;             // launch_spline_pairs only
 };
 cudaError_t launch_spline(const SplineArgs &a, int dtype, cudaStream_t s);
+// the records of pairs of frames (das_frames.cuh): a.nch channels of each of
+// a.nframes frames (even); two channels of nt samples have to fit a CTA
+cudaError_t launch_spline_pairs(const SplineArgs &a, int dtype, cudaStream_t s);
+bool spline_pairs_fit(int nt);
 
 // ---------------------------------------------------------------------------
 // delay-and-sum
@@ -200,6 +205,10 @@ struct DasArgs {
     // cubic_taps applies: the fast knot of every x <= xmax is at most nt - 1, and a
     // group's transmits are less than 2^32 records apart
     int fast_axis;
+    // das_frames_kernel: the receives of this launch (TX_AND_RX: the sum of those
+    // before r0, a block boundary, is in out), and whether DMAS sums plain products
+    int r0, r1;
+    int dmas_power;
     const float *slow;  // GEOM_SYNTH_SLOW: slowness per pixel (s/m), kernel pixel order
     float xfma;         // fma(dt, nt-1, t0): the last knot as the reference's CUDA kernels round it
     // staged kernel: SM cycles after which an mbarrier wait gives up (0: 2^31,
@@ -221,6 +230,10 @@ cudaError_t launch_poly_records(const DasArgs &a, const void *rf, int dtype, int
                                 const float *S, float4 *rec, long long nch, cudaStream_t s);
 cudaError_t launch_das(const DasArgs &a, int geom, int interp, int sumtype, int dtype, bool census,
                        cudaStream_t s);
+// cubic sums over transmits of a.nframes frames (a multiple of fg) from grouped records
+bool das_frames_ok(const DasArgs &a, int sumtype);
+cudaError_t launch_das_frames(const DasArgs &a, int geom, int sumtype, int dtype, int fg,
+                              cudaStream_t s);
 cudaError_t launch_synth_rx_mask(const DasArgs &a, unsigned char *mask, cudaStream_t s);
 // TMA-staged Tabbed path (ntx <= 12; sums over transmits per receive)
 long long tabbed_plan_words(long long np, int ntx, int nrx);

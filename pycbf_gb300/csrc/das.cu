@@ -16,6 +16,24 @@ cudaError_t launch_staged_f32(const DasArgs &, int, int, const int *, int *, cud
 cudaError_t launch_staged_f16(const DasArgs &, int, int, const int *, int *, cudaStream_t);
 cudaError_t launch_staged_bf16(const DasArgs &, int, int, const int *, int *, cudaStream_t);
 cudaError_t launch_staged_adj_f32(const DasArgs &, int, const int *, cudaStream_t);
+cudaError_t launch_das_frames_f32(const DasArgs &, int, int, int, cudaStream_t);
+cudaError_t launch_das_frames_f16(const DasArgs &, int, int, int, cudaStream_t);
+cudaError_t launch_das_frames_bf16(const DasArgs &, int, int, int, cudaStream_t);
+
+bool das_frames_ok(const DasArgs &a, int sumtype) {
+    return a.fast_axis && cubic_column_padded(a.ntx) % kCubicGroup == 0 &&
+           sumtype != PYCBF_GB_SUM_NONE && sumtype != PYCBF_GB_SUM_RX_ONLY;
+}
+
+cudaError_t launch_das_frames(const DasArgs &a, int geom, int sumtype, int dtype, int fg,
+                              cudaStream_t s) {
+    switch (dtype) {
+        case PYCBF_GB_F32: return launch_das_frames_f32(a, geom, sumtype, fg, s);
+        case PYCBF_GB_F16: return launch_das_frames_f16(a, geom, sumtype, fg, s);
+        case PYCBF_GB_BF16: return launch_das_frames_bf16(a, geom, sumtype, fg, s);
+        default: return cudaErrorInvalidValue;
+    }
+}
 
 long long tabbed_plan_words(long long np, int ntx, int nrx) {
     return plan_layout(np, ntx, nrx).total;

@@ -49,7 +49,9 @@ __device__ __forceinline__ void lanes_sync(int bar) {
     if (LANES == 32) __syncwarp();
     else asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(LANES) : "memory");
 }
-template <typename T, int LANES = 32>
+// WRITE false: leaves the samples and z in smem, synchronised over the lanes,
+// and writes no records.
+template <typename T, int LANES = 32, bool WRITE = true>
 __device__ __forceinline__ void spline_channel(const T *__restrict__ src,
                                                typename CoefRec<T>::raw *__restrict__ dst, int nt,
                                                float t0, float dt, const SplineTable &tab,
@@ -120,6 +122,7 @@ __device__ __forceinline__ void spline_channel(const T *__restrict__ src,
             yn = y2k;
         }
     lanes_sync<LANES>(bar);
+    if (!WRITE) return;
     for (int k = lane; k < nt; k += LANES)
         dst[k] = CoefRec<T>::make(y[k], y[k + 1], uz[k], uz[k + 1], k, t0, dt);
 }
@@ -138,6 +141,36 @@ spline_coef_kernel(const T *__restrict__ rf, typename CoefRec<T>::raw *__restric
     const int stride = (nt + 4) & ~3;
     spline_channel<T, 64>(rf + ch * (long long)nt, coef + ch * (long long)nt, nt, t0, dt, tab,
                           smem + (size_t)pr * 2 * stride, 1 + pr);
+}
+
+// The records of pairs of frames in planes of 16 bytes a sample (das_frames.cuh):
+// a CTA solves one channel of both frames, a pair of warps each, then writes them
+// together.  blockIdx.y: the pair.
+template <typename T>
+__global__ void __launch_bounds__(128)
+spline_pairs_kernel(const T *__restrict__ rf, uint4 *__restrict__ coef, long long nch, int nt,
+                    float t0, float dt, const __grid_constant__ SplineTable tab) {
+    extern __shared__ float smem[];
+    const int pr = threadIdx.x >> 6;
+    const long long ch = blockIdx.x, pair = blockIdx.y;
+    const int stride = (nt + 4) & ~3;
+    spline_channel<T, 64, false>(rf + ((pair * 2 + pr) * nch + ch) * (long long)nt, nullptr, nt, t0,
+                                 dt, tab, smem + (size_t)pr * 2 * stride, 1 + pr);
+    __syncthreads();
+    const float *ya = smem, *za = ya + stride, *yb = za + stride, *zb = yb + stride;
+    constexpr int planes = CoefRec<T>::kPoly ? 2 : 1;
+    uint4 *dst = coef + (pair * planes * nch + ch) * (long long)nt;
+    for (int k = threadIdx.x; k < nt; k += 128) {
+        const auto u = CoefRec<T>::make(ya[k], ya[k + 1], za[k], za[k + 1], k, t0, dt);
+        const auto v = CoefRec<T>::make(yb[k], yb[k + 1], zb[k], zb[k + 1], k, t0, dt);
+        if constexpr (CoefRec<T>::kPoly) {
+            float4 *d = reinterpret_cast<float4 *>(dst) + k;
+            d[0] = make_float4(u.x, v.x, u.y, v.y);
+            d[nch * nt] = make_float4(u.z, v.z, u.w, v.w);
+        } else {
+            dst[k] = make_uint4(u.x, u.y, v.x, v.y);
+        }
+    }
 }
 
 // Batched: one pair of warps per channel of any job (jobs' channels numbered
@@ -198,6 +231,38 @@ static cudaError_t launch_spline_t(const SplineArgs &a, cudaStream_t s) {
         static_cast<const T *>(a.rf), static_cast<typename CoefRec<T>::raw *>(a.coef), a.nch, a.nt,
         a.t0, a.dt, tab);
     return cudaGetLastError();
+}
+
+bool spline_pairs_fit(int nt) {
+    return sizeof(float) * 4 * (size_t)((nt + 4) & ~3) <= 227 * 1024;
+}
+
+template <typename T>
+static cudaError_t launch_spline_pairs_t(const SplineArgs &a, cudaStream_t s) {
+    const size_t smem = sizeof(float) * 4 * (size_t)((a.nt + 4) & ~3);
+    static SplineTable tab = [] {
+        SplineTable t;
+        make_spline_table(&t);
+        return t;
+    }();
+    auto kern = spline_pairs_kernel<T>;
+    cudaError_t err =
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return err;
+    if (a.nch > 0x7fffffffLL || a.nframes % 2) return cudaErrorInvalidValue;
+    kern<<<dim3((unsigned)a.nch, (unsigned)(a.nframes / 2)), 128, smem, s>>>(
+        static_cast<const T *>(a.rf), static_cast<uint4 *>(a.coef), a.nch, a.nt, a.t0, a.dt, tab);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_spline_pairs(const SplineArgs &a, int dtype, cudaStream_t s) {
+    switch (dtype) {
+        case PYCBF_GB_F32: return launch_spline_pairs_t<float>(a, s);
+        case PYCBF_GB_F16: return launch_spline_pairs_t<__half>(a, s);
+        case PYCBF_GB_BF16: return launch_spline_pairs_t<__nv_bfloat16>(a, s);
+        case PYCBF_GB_I16: return launch_spline_pairs_t<short>(a, s);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 cudaError_t launch_batch_spline(const BatchJob *jobs, int njobs, long long nch_total, int max_nt,
