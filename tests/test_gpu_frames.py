@@ -80,3 +80,34 @@ def test_frames_int16_and_dmas():
 def test_more_than_a_gigabyte_of_records_goes_by_receive_blocks(sumtype):
     bf = _synthetic(40, 200, 140, 2100, 7, sumtype=sumtype)
     _same(bf, _frames(bf, 4, 3))
+
+
+@pytest.mark.parametrize("lags", [[1], [0, 2, 5], list(range(1, 9)), [31, 1, -3, 7, 30],
+                                  list(range(1, 17)), [1, 32], list(range(1, 18)), [40]])
+@pytest.mark.parametrize("nsep,npx", [(1, 5), (7, 300), (33, 128), (70, 131)])
+@pytest.mark.parametrize("power,sumlags", [(0, 1), (1, 1), (0, 0)])
+def test_dmas_lag_lists(lags, nsep, npx, power, sumlags):
+    """Short lags (one walk with a ring) and any others, against float64 sums: at most
+    70 products of at most 16 lags, each rounded a few times: 100 ulp of the sum of
+    their magnitudes."""
+    import ctypes as ct
+
+    from pycbf_gb300 import _lib
+    im = torch.randn((2, nsep, npx), device="cuda")
+    lg = torch.tensor(lags, dtype=torch.int32, device="cuda")
+    out = torch.empty((2, npx) if sumlags else (2, len(lags), npx), device="cuda")
+    p = lambda t: ct.c_void_p(t.data_ptr())  # noqa: E731
+    L = _lib.load()
+    _lib.check(L.pycbf_gb_dmas(p(im), 2, nsep, npx, p(lg), len(lags), power, sumlags, p(out),
+                               ct.c_void_p(torch.cuda.current_stream().cuda_stream)), "dmas")
+    x = im.double()
+    ref = torch.zeros((2, len(lags), npx), dtype=torch.float64, device="cuda")
+    mag = torch.zeros_like(ref)
+    for k, lag in enumerate(lags):
+        if 0 <= lag < nsep:
+            q = x[:, :nsep - lag] * x[:, lag:]
+            q = q if power else q.sign() * q.abs().sqrt()
+            ref[:, k], mag[:, k] = q.sum(1), q.abs().sum(1)
+    if sumlags:
+        ref, mag = ref.sum(1), mag.sum(1)
+    assert bool(((out.double() - ref).abs() <= 100 * 2.0 ** -24 * mag).all())
