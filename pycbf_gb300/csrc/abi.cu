@@ -585,7 +585,7 @@ int check_adjoint_common(const pycbf_gb_rfinfo *rf, const void *coef, int sumtyp
     if (!coef || reinterpret_cast<uintptr_t>(coef) % 16) return PYCBF_GB_EINVAL;
     if (sumtype != PYCBF_GB_SUM_TX_AND_RX && sumtype != PYCBF_GB_SUM_TX_ONLY)
         return PYCBF_GB_EUNSUPPORTED;
-    if (rf->ntx > kMaxAdjTx || rf->nt > kMaxNtSpline || !adjoint_rows_warps(rf->nt))
+    if (rf->ntx > kMaxAdjTx || rf->nt > kMaxNtSpline)
         return PYCBF_GB_ERANGE;
     return PYCBF_GB_OK;
 }
@@ -596,12 +596,8 @@ int run_adjoint(const pycbf_gb_rfinfo *rf, AdjArgs &g, void *workspace, size_t w
         const size_t need = pycbf_gb_adjoint_workspace_bytes(rf, g.d.np);
         if (!workspace || workspace_bytes < need || reinterpret_cast<uintptr_t>(workspace) % 16)
             return PYCBF_GB_EWORKSPACE;
-        g.gk_buf = static_cast<float *>(workspace);
-        char *ws = static_cast<char *>(workspace);
-        const size_t gb = adjoint_grad_bytes(rf->nframes, rf->nrx, g.d.np);
-        g.partial = reinterpret_cast<float *>(ws + gb);
-        g.live = reinterpret_cast<unsigned char *>(
-            ws + gb + adjoint_partial_bytes(rf->nframes, rf->ntx, rf->nrx, g.d.np, rf->nt));
+        adjoint_layout(rf->nframes, rf->ntx, rf->nrx, g.d.np, rf->nt, g.geom != GEOM_TABBED,
+                       static_cast<char *>(workspace), &g);
     }
     return cuda_status(launch_adjoint(g, rf->dtype, s));
 }
@@ -632,7 +628,7 @@ int pycbf_gb_das_synthetic_slowness(const pycbf_gb_rfinfo *rf, const void *coef,
 
 size_t pycbf_gb_adjoint_workspace_bytes(const pycbf_gb_rfinfo *rf, long long np) {
     if (!rf || np <= 0 || rf->ntx <= 0 || rf->nrx <= 0 || rf->nt <= 0 || rf->nframes <= 0) return 0;
-    return adjoint_workspace_bytes(rf->nframes, rf->ntx, rf->nrx, np, rf->nt);
+    return adjoint_layout(rf->nframes, rf->ntx, rf->nrx, np, rf->nt, rf->ndim != 0, nullptr, nullptr);
 }
 
 int pycbf_gb_das_tabbed_adjoint(const pycbf_gb_rfinfo *rf, const void *coef,

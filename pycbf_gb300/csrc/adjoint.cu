@@ -12,15 +12,13 @@
 //                       dL/dtau_tx (ntx, np) and dL/dtau_rx (nrx, np) for
 //                       Tabbed tables, or into dL/ds (np) for the Synthetic
 //                       slowness form (x = (D_tx + D_rx) s + t0).
-//   adj_scatter_kernel  one CTA per (channel, part of the pixel range): the
-//                       transpose of the interpolation into two shared-memory
-//                       rows (dL/dy, dL/dz) of the channel, one pair per CTA.
-//                       The taps of one warp step are grouped by knot with
-//                       match.any and each group's weights are summed in lane
-//                       order by its lowest lane, which alone updates the rows
-//                       (so no two lanes ever touch one word together); the
-//                       warps take turns, in warp order between CTA barriers,
-//                       so no two warps do either.
+//   adj_scatter_kernel  one warp per (channel, part of the tiles): the transpose of
+//                       the interpolation.  A tap adds (v, v b, v b^2, v b^3) to its
+//                       interval's four moments in the warp's own shared-memory rows
+//                       (512 intervals of the part's window at a time), lanes that
+//                       share an interval in lane order; the moments then give dL/dy
+//                       and dL/dz of the window's samples.  Parts are tiles of similar
+//                       depth (adj_rank_kernel), so a part's window is short.
 //   adj_finalize_kernel one warp per channel: adds the parts in order, then
 //                       the adjoint of the prefilter, dL/drf = dL/dy +
 //                       1/2 D^T T^-1 dL/dz (T is symmetric: the same chunked
@@ -37,19 +35,12 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWarmAdj = 32;  // warm-up of the chunked recurrences (0.268^32 ~ 5e-19)
-constexpr size_t kRowSmemMax = 160 * 1024;
 
-// The forward's decisions for one cubic tap; fractions only where it is in range.
-__device__ __forceinline__ bool cubic_tap(float x, const DasArgs &a, int &j, float &am, float &b) {
-    using K = Kind<PYCBF_GB_INTERP_CUBIC, float>;
-    int idx;
-    bool fix;
-    bool inr = K::index(x, a, idx, fix);
-    if (fix) inr = K::index_exact(x, a, idx);
-    j = idx;
-    am = b = 0.f;
-    if (inr) knot_fractions(x, (float)idx, a, am, b);
-    return inr;
+// c_j = (xhi_j - xlo_j) / dt of the float32 knots (CoefRec<float>::make)
+__device__ __forceinline__ float knot_step(const DasArgs &a, int j) {
+    const float xlo = __fadd_rn(a.t0, __fmul_rn(a.dt, (float)j));
+    const float xhi = __fadd_rn(a.t0, __fmul_rn(a.dt, (float)(j + 1)));
+    return __fdiv_rn(__fsub_rn(xhi, xlo), a.dt);
 }
 
 // the upstream gradient of (frame f, receive r) at kernel-order pixel i (g.gk
@@ -69,23 +60,27 @@ __global__ void adj_gather_kernel(const float *__restrict__ gout, const int *__r
 // ---------------------------------------------------------------------------
 // delays / slowness: gather per pixel
 // ---------------------------------------------------------------------------
+// Bound by the issue rate and the latency of the gathers, as the forward: the taps
+// are decided by its operations (knot_pairs), four at a time, in pairs.  Per thread a
+// column of shared memory for pairs of transmits: delay, weight (Tabbed) or path
+// length (Synthetic), and the running dL/dtau_tx.
 template <int GEOM, int SUM, typename T>
-__global__ void __launch_bounds__(kBlock) adj_delay_kernel(const __grid_constant__ AdjArgs g) {
+__global__ void __launch_bounds__(kBlock, 6) adj_delay_kernel(const __grid_constant__ AdjArgs g) {
     using rec = typename CoefRec<T>::raw;
-    constexpr int G = 6;  // taps whose record loads are in flight together
+    constexpr int G = kCubicGroup;
     const DasArgs &a = g.d;
-    extern __shared__ float sm[];
+    extern __shared__ float2 smp[];
     const int tid = threadIdx.x;
-    const long long i = (long long)blockIdx.x * kBlock + tid;
-    if (i >= a.np) return;
     const long long np = a.np;
+    long long i = (long long)blockIdx.x * kBlock + tid;
+    const bool valid = i < np;
+    if (!valid) i = np - 1;
     const int ntx = a.ntx, nrx = a.nrx, nfr = a.nframes, nt = a.nt;
-    const rec *coef = static_cast<const rec *>(a.data);
-    // this thread's columns: transmit delay, apodization (Tabbed) or path
-    // length (Synthetic), and the dL/dtau_tx accumulator
-    float *stau = sm + tid;
-    float *sw = stau + (size_t)ntx * kBlock;
-    float *sg = sw + (size_t)ntx * kBlock;
+    const int ncol = cubic_column_padded(ntx);
+    const float inf = __int_as_float(0x7f800000);
+    const TapConst tc(a);
+    float2 *stau = smp + tid, *sw = stau + (size_t)(ncol / 2) * kBlock,
+           *sg = sw + (size_t)(ncol / 2) * kBlock;
 
     float pnt[3] = {0.f, 0.f, 0.f};
     float slow = 0.f;
@@ -94,282 +89,423 @@ __global__ void __launch_bounds__(kBlock) adj_delay_kernel(const __grid_constant
         slow = __ldg(a.slow + i);
     }
     float amax = 0.f;
-    for (int t = 0; t < ntx; ++t) {
-        if (GEOM == GEOM_TABBED) {
-            stau[(size_t)t * kBlock] = __ldg(a.tautx + (long long)t * np + i);
-            const float at = __ldg(a.apodtx + (long long)t * np + i);
-            sw[(size_t)t * kBlock] = at;
-            sg[(size_t)t * kBlock] = 0.f;
-            amax = fmaxf(amax, fabsf(at));
-        } else {
-            float D, t0add;
-            const bool ok = synth_tx_path(a, t, pnt, D, t0add);
-            stau[(size_t)t * kBlock] = slow_delay(ok, D, slow, t0add);
-            sw[(size_t)t * kBlock] = D;
+    for (int t = 0; t < ncol; t += 2) {
+        float tau[2] = {inf, inf}, w[2] = {0.f, 0.f};  // padding: never counts
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (t + h >= ntx) continue;
+            if (GEOM == GEOM_TABBED) {
+                tau[h] = __ldg(a.tautx + (long long)(t + h) * np + i);
+                w[h] = __ldg(a.apodtx + (long long)(t + h) * np + i);
+                amax = fmaxf(amax, fabsf(w[h]));
+            } else {
+                float t0add;
+                const bool ok = synth_tx_path(a, t + h, pnt, w[h], t0add);
+                tau[h] = slow_delay(ok, w[h], slow, t0add);
+            }
         }
+        stau[(size_t)(t / 2) * kBlock] = make_float2(tau[0], tau[1]);
+        sw[(size_t)(t / 2) * kBlock] = make_float2(w[0], w[1]);
+        sg[(size_t)(t / 2) * kBlock] = make_float2(0.f, 0.f);
     }
+    const long long chs = (long long)nrx * nt;
+    unsigned off[G];
+#pragma unroll
+    for (int k = 0; k < G; ++k) off[k] = (unsigned)k * (unsigned)chs - kKnotBits;
 
     float gs = 0.f;
     for (int r = 0; r < nrx; ++r) {
         float trx, arx = 1.f, Drx = 0.f;
+        bool live;
         if (GEOM == GEOM_TABBED) {
             trx = __ldg(a.taurx + (long long)r * np + i);
             arx = __ldg(a.apodrx + (long long)r * np + i);
-            // the forward's exact reject: no tap of this receive passes the threshold
-            if (__fmul_rn(amax, fabsf(arx)) < a.thresh) {
-                if (g.grad_taurx) g.grad_taurx[(long long)r * np + i] = 0.f;
-                continue;
-            }
+            live = __fmul_rn(amax, fabsf(arx)) >= a.thresh;
         } else {
-            const bool ok = synth_rx_path(a, r, pnt, Drx);
-            if (!ok) continue;
-            trx = slow_delay(true, Drx, slow, 0.f);
+            live = synth_rx_path(a, r, pnt, Drx);
+            trx = slow_delay(live, Drx, slow, 0.f);
         }
         float grx = 0.f;
-        for (int t0 = 0; t0 < ntx; t0 += G) {
-            // the forward's decisions (fast knots, IEEE redo next to a boundary)
-            const int nk = min(G, ntx - t0);
-            float tt[G], ap[G], sum[G], xs[G], fj[G];
-            int jj[G];
+        // the forward's exact reject, by warps: no tap of the others passes its tests
+        if (__any_sync(kFull, live)) {
+            const float gp0 = nfr == 1 ? __ldg(g.gk + grad_row(SUM, 0, r, nrx) * np + i) : 0.f;
+            for (int t0 = 0; t0 < ncol; t0 += G) {
+                float2 tt2[G / 2], w2[G / 2], x2[G / 2], fj2[G / 2];
+                unsigned rk[G];
 #pragma unroll
-            for (int k = 0; k < G; ++k) {
-                tt[k] = (k < nk) ? stau[(size_t)(t0 + k) * kBlock] : 0.f;
-                sum[k] = 0.f;
-            }
-            unsigned inr, near;
-            cubic_knots<G>(a, tt, trx, xs, jj, fj, inr, near);
-            unsigned hitm = inr & ((1u << nk) - 1u);
-#pragma unroll
-            for (int k = 0; k < G; ++k) {
-                ap[k] = 1.f;
-                if (GEOM == GEOM_TABBED && k < nk) {
-                    ap[k] = __fmul_rn(sw[(size_t)(t0 + k) * kBlock], arx);
-                    if (!(fabsf(ap[k]) >= a.thresh)) hitm &= ~(1u << k);
+                for (int p = 0; p < G / 2; ++p) {
+                    tt2[p] = stau[(size_t)(t0 / 2 + p) * kBlock];
+                    w2[p] = sw[(size_t)(t0 / 2 + p) * kBlock];
+                    if (GEOM == GEOM_TABBED) w2[p] = mul2_rn(w2[p], make_float2(arx, arx));
                 }
-            }
-            if (!hitm) continue;
-            if (hitm & near) cubic_knots_exact<G>(a, xs, jj, fj, hitm & near);
-            bool hit[G];
+                knot_pairs<G / 2>(a, tc, tt2, trx, x2, fj2, rk);
+                if (!a.fast_axis) {  // knots past the record are clamped
 #pragma unroll
-            for (int k = 0; k < G; ++k) hit[k] = (hitm >> k) & 1u;
-            for (int f = 0; f < nfr; ++f) {
-                const float gp = __ldg(g.gk + grad_row(SUM, f, r, nrx) * np + i);
-                float4 c[G];
+                    for (int k = 0; k < G; ++k) {
+                        const float fl = fminf(floorf(__fdiv_rn(__fsub_rn(pair_lane(x2, k), a.t0), a.dt)),
+                                               (float)(nt - 1));
+                        if (k & 1) fj2[k >> 1].y = fl;
+                        else fj2[k >> 1].x = fl;
+                        rk[k] = kKnotBits + (unsigned)(int)fl;
+                    }
+                }
+                bool ok[G];
+                float sum[G];
 #pragma unroll
-                for (int k = 0; k < G; ++k)
-                    if (hit[k])
-                        c[k] = CoefRec<T>::load(coef + (((long long)f * ntx + t0 + k) * nrx + r) * nt +
-                                                jj[k]);
+                for (int k = 0; k < G; ++k) {
+                    const float x = pair_lane(x2, k);
+                    ok[k] = (x >= tc.t0) && (x <= tc.xmax);
+                    if (GEOM == GEOM_TABBED) ok[k] = ok[k] && (fabsf(pair_lane(w2, k)) >= tc.thresh);
+                    sum[k] = 0.f;
+                }
+                for (int f = 0; f < nfr; ++f) {
+                    const float gp = nfr == 1 ? gp0 : __ldg(g.gk + grad_row(SUM, f, r, nrx) * np + i);
+                    const rec *row = static_cast<const rec *>(a.data) +
+                                     (((long long)f * ntx + t0) * nrx + r) * nt;
+                    rec c[G];
 #pragma unroll
-                for (int k = 0; k < G; ++k)
-                    if (hit[k])
-                        sum[k] = fmaf(gp, Kind<PYCBF_GB_INTERP_CUBIC, T>::slope(c[k], xs[k], fj[k], a),
-                                      sum[k]);
-            }
+                    for (int k = 0; k < G; ++k) {
+                        if (ok[k])
+                            c[k] = a.fast_axis ? __ldg(row + (rk[k] + off[k]))
+                                               : __ldg(row + k * chs + (long long)(rk[k] - kKnotBits));
+                    }
 #pragma unroll
-            for (int k = 0; k < G; ++k) {
-                if (!hit[k]) continue;
-                const int t = t0 + k;
-                if (GEOM == GEOM_TABBED) {
-                    const float d = ap[k] * sum[k];
-                    sg[(size_t)t * kBlock] += d;
-                    grx += d;
-                } else {
-                    gs = fmaf(sum[k], sw[(size_t)t * kBlock] + Drx, gs);  // dx/ds = D_tx + D_rx
+                    for (int k = 0; k < G; ++k) {
+                        float slope;
+                        if constexpr (CoefRec<T>::kPoly) {
+                            const float2 b2 = knot_frac2(tc, x2[k >> 1], fj2[k >> 1]);
+                            const float b = (k & 1) ? b2.y : b2.x;
+                            slope = fmaf(fmaf(3.f * c[k].w, b, 2.f * c[k].z), b, c[k].y) * a.inv_dt;
+                        } else {
+                            slope = Kind<PYCBF_GB_INTERP_CUBIC, T>::slope(
+                                CoefRec<T>::unpack(c[k]), pair_lane(x2, k), pair_lane(fj2, k), a);
+                        }
+                        if (ok[k]) sum[k] = fmaf(gp, slope, sum[k]);
+                    }
+                }
+#pragma unroll
+                for (int p = 0; p < G / 2; ++p) {
+                    if (GEOM == GEOM_TABBED) {
+                        float2 d = sg[(size_t)(t0 / 2 + p) * kBlock];
+                        if (ok[2 * p]) {
+                            d.x = fmaf(w2[p].x, sum[2 * p], d.x);
+                            grx = fmaf(w2[p].x, sum[2 * p], grx);
+                        }
+                        if (ok[2 * p + 1]) {
+                            d.y = fmaf(w2[p].y, sum[2 * p + 1], d.y);
+                            grx = fmaf(w2[p].y, sum[2 * p + 1], grx);
+                        }
+                        sg[(size_t)(t0 / 2 + p) * kBlock] = d;
+                    } else {  // dx/ds = D_tx + D_rx
+                        if (ok[2 * p]) gs = fmaf(sum[2 * p], w2[p].x + Drx, gs);
+                        if (ok[2 * p + 1]) gs = fmaf(sum[2 * p + 1], w2[p].y + Drx, gs);
+                    }
                 }
             }
         }
-        if (GEOM == GEOM_TABBED && g.grad_taurx) g.grad_taurx[(long long)r * np + i] = grx;
+        if (GEOM == GEOM_TABBED && g.grad_taurx && valid) g.grad_taurx[(long long)r * np + i] = grx;
     }
-    if (GEOM == GEOM_TABBED && g.grad_tautx)
-        for (int t = 0; t < ntx; ++t) g.grad_tautx[(long long)t * np + i] = sg[(size_t)t * kBlock];
+    if (!valid) return;
+    if (GEOM == GEOM_TABBED && g.grad_tautx) {
+        for (int t = 0; t < ntx; ++t) {
+            const float2 d = sg[(size_t)(t / 2) * kBlock];
+            g.grad_tautx[(long long)t * np + i] = (t & 1) ? d.y : d.x;
+        }
+    }
     if (GEOM == GEOM_SYNTH_SLOW && g.grad_slow) g.grad_slow[i] = gs;
 }
 
 // ---------------------------------------------------------------------------
-// which receives can contribute to which tiles of kBlock pixels: Tabbed, some
-// pixel has fl(max_t |apodtx| * |apodrx|) >= thresh (by monotonic rounding
-// every tap of a dead pair fails the threshold); Synthetic, the receive's mask
-// accepts some pixel.  One CTA per tile.
+// what the scatter needs to know of each tile of kBlock pixels: which receives can
+// contribute to it (Tabbed: some pixel has fl(max_t |apodtx| * |apodrx|) >= thresh,
+// so every tap of a dead pair fails the threshold; Synthetic: the receive's mask
+// accepts some pixel), and the range of every transmit's and receive's delays (over
+// the pixels that the receive reaches; empty: inf, -inf).  TABLES: also writes the
+// Synthetic delays, NaN where masked.  One CTA per tile (blockIdx.x) and share of the
+// receives (blockIdx.y).
 // ---------------------------------------------------------------------------
-template <int GEOM>
-__global__ void __launch_bounds__(kBlock) adj_live_kernel(const __grid_constant__ AdjArgs g) {
+// floats as integers of the same order (no NaN), for the warp's integer reductions
+__device__ __forceinline__ int to_key(float v) {
+    const int b = __float_as_int(v);
+    return b < 0 ? b ^ 0x7fffffff : b;
+}
+__device__ __forceinline__ float from_key(int k) { return __int_as_float(k < 0 ? k ^ 0x7fffffff : k); }
+
+template <int GEOM, bool TABLES>
+__global__ void __launch_bounds__(kBlock) adj_range_kernel(const __grid_constant__ AdjArgs g) {
+    constexpr int kWarps = kBlock / 32, M = kBlock / 32;  // a warp per element, M pixels a lane
     const DasArgs &a = g.d;
-    const long long tile = blockIdx.x;
-    const long long tiles = gridDim.x;
-    const long long i = tile * kBlock + threadIdx.x;
-    const bool valid = i < a.np;
-    float amax = 0.f;
-    float pnt[3] = {0.f, 0.f, 0.f};
-    if (valid) {
-        if (GEOM == GEOM_TABBED)
-            for (int t = 0; t < a.ntx; ++t)
-                amax = fmaxf(amax, fabsf(__ldg(a.apodtx + (long long)t * a.np + i)));
-        else
-            for (int k = 0; k < 3; ++k) if (k < a.ndim) pnt[k] = __ldg(a.geo.pnts + i * a.ndim + k);
+    const float inf = __int_as_float(0x7f800000), nan = __int_as_float(0x7fc00000);
+    __shared__ float s_amax[kWarps][kBlock];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long long tile = blockIdx.x, tiles = gridDim.x;
+    const long long i0 = tile * kBlock + lane;
+    float2 *ranges = g.ranges + tile * (a.ntx + a.nrx);
+    float pnt[M][3], slow[M], amax[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        const long long i = i0 + 32 * m;
+        amax[m] = slow[m] = 0.f;
+        for (int k = 0; k < 3; ++k)
+            pnt[m][k] = (GEOM != GEOM_TABBED && i < a.np && k < a.ndim)
+                            ? __ldg(a.geo.pnts + i * a.ndim + k) : 0.f;
+        if (GEOM != GEOM_TABBED && i < a.np) slow[m] = __ldg(a.slow + i);
     }
-    for (int r = 0; r < a.nrx; ++r) {
-        bool v = false;
-        if (valid) {
+    auto element = [&](int e) {
+        const bool tx = e < a.ntx;
+        const int r = e - a.ntx;
+        float lo = inf, hi = -inf;
+        bool any = false;
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            const long long i = i0 + 32 * m;
+            if (i >= a.np) continue;
+            float tau;
+            bool live = true;
             if (GEOM == GEOM_TABBED) {
-                v = __fmul_rn(amax, fabsf(__ldg(a.apodrx + (long long)r * a.np + i))) >= a.thresh;
+                tau = __ldg((tx ? a.tautx + (long long)e * a.np : a.taurx + (long long)r * a.np) + i);
+                if (tx) amax[m] = fmaxf(amax[m], fabsf(__ldg(a.apodtx + (long long)e * a.np + i)));
+                else live = __fmul_rn(amax[m], fabsf(__ldg(a.apodrx + (long long)r * a.np + i))) >= a.thresh;
             } else {
-                float D;
-                v = synth_rx_path(a, r, pnt, D);
+                float D, t0add = 0.f;
+                live = tx ? synth_tx_path(a, e, pnt[m], D, t0add) : synth_rx_path(a, r, pnt[m], D);
+                tau = slow_delay(live, D, slow[m], t0add);
+                if (TABLES)
+                    (tx ? g.tau_tx + (long long)e * a.np : g.tau_rx + (long long)r * a.np)[i] =
+                        live ? tau : nan;
+            }
+            any |= live;
+            if (live && fabsf(tau) < inf) {
+                lo = fminf(lo, tau);
+                hi = fmaxf(hi, tau);
             }
         }
-        v = __syncthreads_or(v);
-        if (threadIdx.x == 0) g.live[(long long)r * tiles + tile] = v ? 1 : 0;
+        lo = from_key(__reduce_min_sync(kFull, to_key(lo)));
+        hi = from_key(__reduce_max_sync(kFull, to_key(hi)));
+        any = __any_sync(kFull, any);
+        if (lane == 0 && !(tx && blockIdx.y > 0)) {
+            ranges[e] = make_float2(lo, hi);
+            if (tx && e == a.ntx / 2) g.depth[tile] = lo;
+            if (!tx) g.live[(long long)r * tiles + tile] = any ? 1 : 0;
+        }
+    };
+    for (int t = w; t < a.ntx; t += kWarps) element(t);
+    if (GEOM == GEOM_TABBED) {  // the largest weight over every warp's transmits
+#pragma unroll
+        for (int m = 0; m < M; ++m) s_amax[w][lane + 32 * m] = amax[m];
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+            for (int k = 0; k < kWarps; ++k) amax[m] = fmaxf(amax[m], s_amax[k][lane + 32 * m]);
     }
+    for (int r = blockIdx.y * kWarps + w; r < a.nrx; r += gridDim.y * kWarps) element(a.ntx + r);
+}
+
+// The tiles by depth -- the earliest delay of the middle transmit -- so that the
+// consecutive tiles of a part share a short window of samples, in any pixel order:
+// each tile's place is the number of tiles before it (ties by tile number, so the
+// order is always the same).
+constexpr long long kRankTiles = 1 << 16;  // above: the pixels' own order
+
+__global__ void __launch_bounds__(256) adj_rank_kernel(const float *__restrict__ depth, int tiles,
+                                                       int *__restrict__ order) {
+    const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;  // a warp per tile
+    if (t >= tiles) return;
+    const float key = __ldg(depth + t);
+    int rank = 0;
+    for (int k = lane; k < tiles; k += 32) {
+        const float v = __ldg(depth + k);
+        rank += (v < key || (v == key && k < t)) ? 1 : 0;
+    }
+    rank = __reduce_add_sync(kFull, rank);
+    if (lane == 0) order[rank] = t;
 }
 
 // ---------------------------------------------------------------------------
-// channel data: transpose of the interpolation, per (channel, part)
-// ---------------------------------------------------------------------------
-template <int GEOM, int SUM>
-__global__ void __launch_bounds__(128) adj_scatter_kernel(const __grid_constant__ AdjArgs g,
-                                                          long long part_len, int Lp) {
-    const DasArgs &a = g.d;
-    extern __shared__ float rows[];  // [2][Lp]: dL/dy, dL/dz
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const long long np = a.np;
-    const int ntx = a.ntx, nrx = a.nrx;
-    const long long nch = (long long)a.nframes * ntx * nrx;
-    const long long c = blockIdx.x;  // channel ((f * ntx + t) * nrx + r)
-    const int q = blockIdx.y;        // part
-    const int r = (int)(c % nrx);
-    const int t = (int)((c / nrx) % ntx);
-    const int f = (int)(c / ((long long)nrx * ntx));
-    float *ry = rows;
-    float *rz = ry + Lp;
-    for (int n = threadIdx.x; n < 2 * Lp; n += blockDim.x) ry[n] = 0.f;
-    __syncthreads();
+// channel data: transpose of the interpolation, one warp per (channel, part).  The
+// four warps of a CTA take four transmits of one receive (they share its delays,
+// weights and gradient in L1) and never wait for one another.
+//
+// TABLES: delays from tau_tx / tau_rx (NaN: masked), weights Tabbed only.
+//
+// What the walk waits for is its loads, so a warp has the next live tile's inputs (20
+// a lane) in flight, and which lanes share an interval: along image lines (neighbouring
+// pixels some samples apart) none do, and a compare with the next lane shows it.  11 x
+// 128 x 2048 samples, 256 x 512 pixels: 321 us along lines, 478 in Morton order with
+// masks (59 and 52 % of the issue slots), against 920 and 1271 for one CTA a channel
+// part whose warps took turns on full-length rows between barriers.
+constexpr int kSeg = 512;  // intervals of a warp's rows: 8 KB, seven CTAs an SM
 
-    const long long i0 = (long long)q * part_len;
-    const long long i1 = min(np, i0 + part_len);
-    const float *grow = g.gk + grad_row(SUM, f, r, nrx) * np;
-    // this pixel's inputs, fetched one step ahead: Tabbed apodtx, apodrx,
-    // tautx, taurx; Synthetic the point and its slowness; the upstream gradient
-    struct In {
-        float v[4];
-        float gp;
-    };
-    auto fetch = [&](long long i, In &in) {
-        if (i >= i1) return;
-        if (GEOM == GEOM_TABBED) {
-            in.v[0] = __ldg(a.apodtx + (long long)t * np + i);
-            in.v[1] = __ldg(a.apodrx + (long long)r * np + i);
-            in.v[2] = __ldg(a.tautx + (long long)t * np + i);
-            in.v[3] = __ldg(a.taurx + (long long)r * np + i);
-        } else {
-            for (int k = 0; k < 3; ++k) if (k < a.ndim) in.v[k] = __ldg(a.geo.pnts + i * a.ndim + k);
-            in.v[3] = __ldg(a.slow + i);
-        }
-        in.gp = __ldg(grow + i);
-    };
-    // steps of blockDim pixels whose tile receive r can contribute to; the
-    // others are skipped (the same for every thread of the CTA)
-    const unsigned char *rx_live = g.live + (long long)r * ((np + kBlock - 1) / kBlock);
-    auto next_live = [&](long long b) {
-        while (b < i1 && !rx_live[b / kBlock]) b += blockDim.x;
-        return b;
-    };
-    // one live step's tap of this lane: knot, fractions and the weighted gradient
-    struct Tap {
-        bool hit;
-        int j;
-        float am, b, v;
-    };
-    auto tap_of = [&](long long base, const In &in) {
-        Tap tp = {false, 0, 0.f, 0.f, 0.f};
-        const long long i = base + threadIdx.x;
-        if (base >= i1 || i >= i1) return tp;
-        float x = 0.f, apod = 1.f;
-        bool live;
-        if (GEOM == GEOM_TABBED) {
-            apod = __fmul_rn(in.v[0], in.v[1]);
-            live = fabsf(apod) >= a.thresh;
-            x = __fadd_rn(in.v[2], in.v[3]);
-        } else {
-            const float pnt[3] = {in.v[0], in.v[1], in.v[2]};
-            float Dt, t0add, Dr;
-            const bool okt = synth_tx_path(a, t, pnt, Dt, t0add);
-            const bool okr = synth_rx_path(a, r, pnt, Dr);
-            live = okt && okr;
-            x = __fadd_rn(slow_delay(true, Dt, in.v[3], t0add), slow_delay(true, Dr, in.v[3], 0.f));
-        }
-        if (live && cubic_tap(x, a, tp.j, tp.am, tp.b)) {
-            tp.hit = true;
-            tp.v = (GEOM == GEOM_TABBED) ? in.gp * apod : in.gp;
-        }
-        return tp;
-    };
-    // the warp's taps of one step into its rows: grouped by knot, the lowest
-    // lane of a group sums the group's weights in lane order
-    auto scatter = [&](const Tap &tp) {
-        if (!__any_sync(kFull, tp.hit)) return;
-        const unsigned grp = __match_any_sync(kFull, tp.hit ? tp.j : -1);
-        const int n = __popc(grp);
-        const int nmax = (int)__reduce_max_sync(kFull, tp.hit ? (unsigned)n : 0u);
-        const float wa = tp.v * tp.am, wb = tp.v * tp.b;
-        const float wc = tp.v * fmaf(tp.am * tp.am, tp.am, -tp.am);
-        const float wd = tp.v * fmaf(tp.b * tp.b, tp.b, -tp.b);
-        float A = wa, B = wb, C = wc, D = wd;
-        unsigned rest = grp & (grp - 1u);
-        for (int k = 1; k < nmax; ++k) {
-            const int src = rest ? __ffs(rest) - 1 : lane;
-            rest &= rest - 1u;
-            const float xa = __shfl_sync(kFull, wa, src), xb = __shfl_sync(kFull, wb, src);
-            const float xc = __shfl_sync(kFull, wc, src), xd = __shfl_sync(kFull, wd, src);
-            if (k < n) {
-                A += xa;
-                B += xb;
-                C += xc;
-                D += xd;
+template <int GEOM, int SUM, bool TABLES>
+__global__ void __launch_bounds__(128, 5) adj_scatter_kernel(const __grid_constant__ AdjArgs g,
+                                                             int per, int Lp) {
+    const DasArgs &a = g.d;
+    extern __shared__ float4 rows[];
+    int *list = reinterpret_cast<int *>(rows + 4 * kSeg);  // [per] the part's live tiles
+    __shared__ int s_count[4];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long long np = a.np;
+    const int ntx = a.ntx, nrx = a.nrx, nt = a.nt, nel = ntx + nrx;
+    const int r = blockIdx.x % nrx;
+    const int tq = blockIdx.x / nrx, nq = (ntx + 3) / 4;  // group of four transmits, over frames
+    const int f = tq / nq, t = tq % nq * 4 + w;
+    const int q = blockIdx.y;
+    const long long nch = (long long)a.nframes * ntx * nrx;
+    const long long ch = ((long long)f * ntx + t) * nrx + r;
+    const int tiles = (int)((np + kBlock - 1) / kBlock);
+    // the part's tiles that receive r can reach, in order
+    int nlist = 0;
+    {
+        const unsigned char *live = g.live + (long long)r * tiles;
+        const int k1 = min(tiles, (q + 1) * per);
+        for (int b = q * per; b < k1; b += 128) {
+            const int k = b + threadIdx.x;
+            const int tile = k < k1 ? (g.order ? __ldg(g.order + k) : k) : 0;
+            const bool on = k < k1 && live[tile];
+            const unsigned m = __ballot_sync(kFull, on);
+            if (lane == 0) s_count[w] = __popc(m);
+            __syncthreads();
+            int at = nlist + __popc(m & ((1u << lane) - 1u));
+            for (int v = 0; v < 4; ++v) {
+                at += v < w ? s_count[v] : 0;
+                nlist += s_count[v];
             }
-        }
-        const bool leader = tp.hit && (lane == __ffs(grp) - 1);
-        if (leader) {
-            ry[tp.j] += A;
-            rz[tp.j] += C;
-        }
-        __syncwarp();
-        if (leader) {
-            ry[tp.j + 1] += B;
-            rz[tp.j + 1] += D;
-        }
-        __syncwarp();
-    };
-    // live steps two at a time (their taps computed together; each warp adds
-    // its two steps' taps in its turn, warps in order), the next two fetched
-    // meanwhile
-    In c0 = {{0.f, 0.f, 0.f, 0.f}, 0.f}, c1 = c0, n0 = c0, n1 = c0;
-    long long b0 = next_live(i0);
-    long long b1 = b0 < i1 ? next_live(b0 + blockDim.x) : i1;
-    if (b0 < i1) fetch(b0 + threadIdx.x, c0);
-    if (b1 < i1) fetch(b1 + threadIdx.x, c1);
-    while (b0 < i1) {
-        const long long nb0 = b1 < i1 ? next_live(b1 + blockDim.x) : i1;
-        const long long nb1 = nb0 < i1 ? next_live(nb0 + blockDim.x) : i1;
-        if (nb0 < i1) fetch(nb0 + threadIdx.x, n0);
-        if (nb1 < i1) fetch(nb1 + threadIdx.x, n1);
-        const Tap t0 = tap_of(b0, c0);
-        const Tap t1 = tap_of(b1, c1);
-        for (int turn = 0; turn < nw; ++turn) {  // b0 is the same in every thread
-            if (w == turn) {
-                scatter(t0);
-                scatter(t1);
-            }
+            if (on) list[at] = tile;
             __syncthreads();
         }
-        b0 = nb0;
-        b1 = nb1;
-        c0 = n0;
-        c1 = n1;
     }
-    __syncthreads();
-    float *dst = g.partial + ((size_t)q * nch + c) * 2 * Lp;
-    for (int m = threadIdx.x; m < 2 * Lp; m += blockDim.x) dst[m] = rows[m];
+    if (t >= ntx) return;  // a whole warp; no barrier below
+    float4 *row = rows + w * kSeg;
+    float *py = g.partial + ((size_t)q * nch + ch) * 2 * Lp, *pz = py + Lp;
+
+    // samples that those tiles' taps of this channel can touch: intervals [w0, w1)
+    float4 rng = make_float4(__int_as_float(0x7f800000), -__int_as_float(0x7f800000),
+                             __int_as_float(0x7f800000), -__int_as_float(0x7f800000));
+    for (int k = lane; k < nlist; k += 32) {
+        const float2 u = __ldg(g.ranges + (long long)list[k] * nel + t);
+        const float2 v = __ldg(g.ranges + (long long)list[k] * nel + ntx + r);
+        rng = make_float4(fminf(rng.x, u.x), fmaxf(rng.y, u.y), fminf(rng.z, v.x), fmaxf(rng.w, v.y));
+    }
+    const float lo = __fadd_rn(from_key(__reduce_min_sync(kFull, to_key(rng.x))),
+                               from_key(__reduce_min_sync(kFull, to_key(rng.z))));
+    const float hi = __fadd_rn(from_key(__reduce_max_sync(kFull, to_key(rng.y))),
+                               from_key(__reduce_max_sync(kFull, to_key(rng.w))));
+    int w0 = 0, w1 = 0;
+    if (lo <= hi && hi >= a.t0 && lo <= a.xmax) {
+        w0 = lo <= a.t0 ? 0 : (int)floorf(__fdiv_rn(__fsub_rn(lo, a.t0), a.dt));
+        w1 = hi >= a.xmax ? nt : min(nt, (int)floorf(__fdiv_rn(__fsub_rn(hi, a.t0), a.dt)) + 1);
+        w0 = min(w0, nt - 1);
+    }
+    if (lane == 0) g.windows[(size_t)q * nch + ch] = make_int2(w0, w1);  // samples w0 .. w1 of the rows
+
+    const float *ptx = (GEOM == GEOM_TABBED ? a.tautx : g.tau_tx) + (long long)t * np;
+    const float *prx = (GEOM == GEOM_TABBED ? a.taurx : g.tau_rx) + (long long)r * np;
+    const float *pat = a.apodtx + (long long)t * np, *par = a.apodrx + (long long)r * np;
+    const float *grow = g.gk + grad_row(SUM, f, r, nrx) * np;
+    constexpr int M = kBlock / 32;  // steps of 32 pixels in a tile
+    struct In {
+        float tx[M], rx[M], wt[M], wr[M], gp[M];
+    };
+    // the inputs of a lane's pixels of one tile: delays, weights and gradient
+    auto fetch = [&](int tile, In &in) {
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const long long i = (long long)tile * kBlock + 32 * m + lane;
+        in.tx[m] = __int_as_float(0x7fc00000);  // NaN delay: no tap
+        in.rx[m] = in.wt[m] = in.wr[m] = in.gp[m] = 0.f;
+        if (i >= np) continue;
+        if (GEOM == GEOM_TABBED || TABLES) {
+            in.tx[m] = __ldg(ptx + i);
+            in.rx[m] = __ldg(prx + i);
+        } else {
+            float pnt[3] = {0.f, 0.f, 0.f}, Dt, t0add, Dr;
+            for (int k = 0; k < 3; ++k) if (k < a.ndim) pnt[k] = __ldg(a.geo.pnts + i * a.ndim + k);
+            const float s = __ldg(a.slow + i);
+            const bool okt = synth_tx_path(a, t, pnt, Dt, t0add);
+            const bool okr = synth_rx_path(a, r, pnt, Dr);
+            if (okt && okr) in.tx[m] = slow_delay(true, Dt, s, t0add);
+            in.rx[m] = slow_delay(true, Dr, s, 0.f);
+        }
+        in.gp[m] = __ldg(grow + i);
+        if (GEOM == GEOM_TABBED) {
+            in.wt[m] = __ldg(pat + i);
+            in.wr[m] = __ldg(par + i);
+        }
+      }
+    };
+
+    float4 carry = make_float4(0.f, 0.f, 0.f, 0.f);  // the interval before the segment
+    for (int s0 = w0; s0 < w1; s0 += kSeg) {
+        const int n = min(kSeg, w1 - s0);
+        for (int m = lane; m < n; m += 32) row[m] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncwarp();
+        // the live tiles in turn, the next one's inputs fetched meanwhile
+        In cur, nxt;
+        if (nlist > 0) fetch(list[0], cur);
+        for (int k = 0; k < nlist; ++k, cur = nxt) {
+          if (k + 1 < nlist) fetch(list[k + 1], nxt);
+#pragma unroll
+          for (int m = 0; m < M; ++m) {
+            const float x = __fadd_rn(cur.tx[m], cur.rx[m]);
+            int j;
+            bool fix;
+            using K = Kind<PYCBF_GB_INTERP_CUBIC, float>;
+            bool hit = K::index(x, a, j, fix);
+            if (fix) hit = K::index_exact(x, a, j);
+            float v = cur.gp[m];
+            if (GEOM == GEOM_TABBED) {
+                const float wt = __fmul_rn(cur.wt[m], cur.wr[m]);
+                hit = hit && fabsf(wt) >= a.thresh;
+                v *= wt;
+            }
+            j -= s0;
+            hit = hit && (unsigned)j < (unsigned)n;
+            if (__any_sync(kFull, hit)) {
+                const float xlo = __fadd_rn(a.t0, __fmul_rn(a.dt, (float)(j + s0)));
+                const float b = __fmul_rn(__fsub_rn(x, xlo), a.inv_dt);
+                const float m1 = v * b, m2 = m1 * b, m3 = m2 * b;
+                // lanes of one interval add in lane order.  Along a line of pixels the
+                // intervals mostly increase from lane to lane: then no two are alike.
+                const int key = hit ? j : -1 - lane;
+                const int up = __shfl_up_sync(kFull, j, 1);
+                if (__all_sync(kFull, hit && (lane == 0 || j > up))) {
+                    float4 c = row[j];
+                    row[j] = make_float4(c.x + v, c.y + m1, c.z + m2, c.w + m3);
+                } else {
+                    const unsigned grp = __match_any_sync(kFull, key);
+                    const int mine = __popc(grp & ((1u << lane) - 1u));
+                    const int most = (int)__reduce_max_sync(kFull, hit ? (unsigned)mine : 0u);
+                    for (int turn = 0; turn <= most; ++turn) {
+                        if (hit && mine == turn) {
+                            float4 c = row[j];
+                            row[j] = make_float4(c.x + v, c.y + m1, c.z + m2, c.w + m3);
+                        }
+                        __syncwarp();
+                    }
+                }
+                __syncwarp();
+            }
+          }
+        }
+        __syncwarp();
+        // samples s0 .. s0 + n - 1 (and, past the last segment, s0 + n) from the moments of
+        // the intervals on either side, with a = c_j - b as in the records
+        const bool last = s0 + n >= w1;
+        for (int m0 = 0; m0 < n + (last ? 1 : 0); m0 += 32) {
+            const int m = m0 + lane;
+            const float4 here = m < n ? row[m] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 before = m == 0 ? carry : (m <= n ? row[m - 1] : here);
+            if (m < n || (last && m == n)) {
+                const float c = knot_step(a, s0 + m), c2 = c * c;
+                py[s0 + m] = fmaf(c, here.x, -here.y) + before.y;
+                pz[s0 + m] = fmaf(c2 * c - c, here.x,
+                                  fmaf(1.f - 3.f * c2, here.y, fmaf(3.f * c, here.z, -here.w))) +
+                             (before.w - before.y);
+            }
+        }
+        carry = row[n - 1];
+        __syncwarp();
+    }
 }
 
 // v = T^-1 dL/dz in place of zv (one warp; u: scratch of nt floats), with v_0 =
@@ -417,8 +553,9 @@ __device__ __forceinline__ void prefilter_adjoint_warp(float *zv, float *u, int 
 // adjoint of the prefilter, one warp per channel
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-adj_finalize_kernel(const float *__restrict__ partial, int nparts, long long nch, int nt, int Lp,
-                    float *__restrict__ grad_rf, const __grid_constant__ SplineTable tab) {
+adj_finalize_kernel(const float *__restrict__ partial, const int2 *__restrict__ windows, int nparts,
+                    long long nch, int nt, int Lp, float *__restrict__ grad_rf,
+                    const __grid_constant__ SplineTable tab) {
     extern __shared__ float smem[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     const long long ch = (long long)blockIdx.x * wpb + w;
@@ -428,24 +565,34 @@ adj_finalize_kernel(const float *__restrict__ partial, int nparts, long long nch
     float *u = zv + stride;
     const float *p0 = partial + (size_t)ch * 2 * Lp;
     const size_t pstride = (size_t)nch * 2 * Lp;  // between parts
-    for (int n = lane; n < nt; n += 32) {
-        float sz = 0.f;
-        for (int q = 0; q < nparts; ++q) sz += p0[q * pstride + Lp + n];
-        zv[n] = sz;
-    }
+    // the parts' samples into dst, parts in order, each from its window only
+    auto sum_parts = [&](float *dst, int off) {
+        for (int n = lane; n < nt; n += 32) dst[n] = 0.f;
+        for (int q = 0; q < nparts; ++q) {
+            const int2 win = __ldg(windows + q * nch + ch);
+            if (win.x >= win.y) continue;
+            const float *src = p0 + q * pstride + off;
+#pragma unroll 4
+            for (int n = win.x + lane; n <= min(win.y, nt - 1); n += 32) dst[n] += src[n];
+        }
+    };
+    sum_parts(zv, Lp);
+    __syncwarp();
     prefilter_adjoint_warp(zv, u, nt, tab, lane);
+    sum_parts(u, 0);
+    __syncwarp();
     float *dst = grad_rf + ch * (long long)nt;
     for (int n = lane; n < nt; n += 32) {
-        float sy = 0.f;
-        for (int q = 0; q < nparts; ++q) sy += p0[q * pstride + n];
         const float vm = n >= 1 ? zv[n - 1] : 0.f;
         const float vp = n + 1 < nt ? zv[n + 1] : 0.f;
-        dst[n] = fmaf(0.5f, vm - 2.f * zv[n] + vp, sy);
+        dst[n] = fmaf(0.5f, vm - 2.f * zv[n] + vp, u[n]);
     }
 }
 
 
-size_t delay_smem_bytes(int ntx) { return 3 * (size_t)ntx * kBlock * sizeof(float); }
+size_t delay_smem_bytes(int ntx) {
+    return 3 * (size_t)cubic_column_padded(ntx) * kBlock * sizeof(float);
+}
 
 template <int GEOM, int SUM, typename T>
 cudaError_t launch_delay_one(const AdjArgs &g, cudaStream_t s) {
@@ -462,25 +609,43 @@ cudaError_t launch_delay_one(const AdjArgs &g, cudaStream_t s) {
 }
 
 template <int GEOM, int SUM>
-cudaError_t launch_scatter_one(const AdjArgs &g, cudaStream_t s) {
+cudaError_t launch_scatter_one(const AdjArgs &g0, cudaStream_t s) {
+    AdjArgs g = g0;
     const DasArgs &a = g.d;
     const long long nch = (long long)a.nframes * a.ntx * a.nrx;
-    const int nparts = adjoint_parts(nch, a.np);
-    const int nw = adjoint_rows_warps(a.nt);
-    if (nw == 0) return cudaErrorInvalidValue;
-    const int Lp = (a.nt + 1 + 3) & ~3;
-    const long long per = (a.np + nparts - 1) / nparts;
-    const long long part_len = (per + 127) / 128 * 128;
     const long long tiles = (a.np + kBlock - 1) / kBlock;
-    adj_live_kernel<GEOM><<<(unsigned)tiles, kBlock, 0, s>>>(g);
-    cudaError_t lerr = cudaGetLastError();
-    if (lerr != cudaSuccess) return lerr;
-    const size_t smem = (size_t)2 * Lp * sizeof(float);
-    auto kern = adj_scatter_kernel<GEOM, SUM>;
-    cudaError_t err =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int nparts = adjoint_parts(nch, a.np);
+    const int per = (int)((tiles + nparts - 1) / nparts);
+    const int Lp = (a.nt + 1 + 3) & ~3;
+    // Synthetic delays once into tables where they fit (the scatter would take a root
+    // and a quotient per tap again)
+    const bool tables = GEOM == GEOM_TABBED || g.tau_tx;
+    constexpr bool kSynth = GEOM != GEOM_TABBED;
+    const dim3 rgrid((unsigned)tiles, 4);
+    if (tables) adj_range_kernel<GEOM, kSynth><<<rgrid, kBlock, 0, s>>>(g);
+    else adj_range_kernel<GEOM, false><<<rgrid, kBlock, 0, s>>>(g);
+    cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
-    kern<<<dim3((unsigned)nch, (unsigned)nparts), 32 * nw, smem, s>>>(g, part_len, Lp);
+    if (tiles <= kRankTiles) {
+        adj_rank_kernel<<<(unsigned)((tiles + 7) / 8), 256, 0, s>>>(g.depth, (int)tiles, g.order);
+        if ((err = cudaGetLastError()) != cudaSuccess) return err;
+    } else {
+        g.order = nullptr;
+    }
+    const size_t smem = 4 * kSeg * sizeof(float4) + per * sizeof(int);
+    if (smem > 48 * 1024) {
+        const int lim = (int)smem;
+        const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        err = cudaFuncSetAttribute(adj_scatter_kernel<GEOM, SUM, true>, attr, lim);
+        if (err == cudaSuccess && kSynth)
+            err = cudaFuncSetAttribute(adj_scatter_kernel<GEOM, SUM, !kSynth>, attr, lim);
+        if (err != cudaSuccess) return err;
+    }
+    const long long groups = (long long)a.nframes * ((a.ntx + 3) / 4) * a.nrx;
+    if (groups > 0x7fffffffLL) return cudaErrorInvalidValue;
+    const dim3 grid((unsigned)groups, (unsigned)nparts);
+    if (tables) adj_scatter_kernel<GEOM, SUM, true><<<grid, 128, smem, s>>>(g, per, Lp);
+    else adj_scatter_kernel<GEOM, SUM, !kSynth><<<grid, 128, smem, s>>>(g, per, Lp);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
 
@@ -496,8 +661,8 @@ cudaError_t launch_scatter_one(const AdjArgs &g, cudaStream_t s) {
                                (int)fsmem);
     if (err != cudaSuccess) return err;
     const long long blocks = (nch + wpb - 1) / wpb;
-    adj_finalize_kernel<<<(unsigned)blocks, 32 * wpb, fsmem, s>>>(g.partial, nparts, nch, a.nt, Lp,
-                                                                  g.grad_rf, tab);
+    adj_finalize_kernel<<<(unsigned)blocks, 32 * wpb, fsmem, s>>>(
+        g.partial, g.windows, nparts, nch, a.nt, Lp, g.grad_rf, tab);
     return cudaGetLastError();
 }
 
@@ -550,12 +715,9 @@ int adjoint_parts(long long nch, long long np) {
     // 2.22 at 2), parts of >= 2048 pixels
     long long p = (11264 + nch - 1) / nch;
     p = std::min<long long>(p, std::max<long long>(1, np / 2048));
-    return (int)std::max<long long>(1, std::min<long long>(p, 64));
-}
-
-int adjoint_rows_warps(int nt) {
-    const size_t row = 2 * (size_t)((nt + 1 + 3) & ~3) * sizeof(float);
-    return row <= kRowSmemMax ? 4 : 0;
+    p = std::max<long long>(1, std::min<long long>(p, 64));
+    // a part's tile list has to fit shared memory: 16,384 tiles
+    return (int)std::max<long long>(p, ((np + kBlock - 1) / kBlock + 16383) / 16384);
 }
 
 size_t adjoint_grad_bytes(long long nframes, long long nrx, long long np) {
@@ -569,11 +731,46 @@ size_t adjoint_partial_bytes(long long nframes, long long ntx, long long nrx, lo
     return (size_t)adjoint_parts(nch, np) * (size_t)nch * 2 * Lp * sizeof(float);
 }
 
-size_t adjoint_workspace_bytes(long long nframes, long long ntx, long long nrx, long long np,
-                               int nt) {
-    const size_t tiles = (size_t)((np + kBlock - 1) / kBlock);
-    return adjoint_grad_bytes(nframes, nrx, np) + adjoint_partial_bytes(nframes, ntx, nrx, np, nt) +
-           (((size_t)nrx * tiles + 255) & ~(size_t)255);
+// [gathered gradient][partial sums][live][tile ranges][depths][windows][order]
+// [Synthetic delay tables], each 256-byte aligned
+constexpr size_t kAdjTableMax = (size_t)1 << 30;  // above: the scatter recomputes the delays
+
+size_t adjoint_layout(long long nframes, long long ntx, long long nrx, long long np, int nt,
+                      bool synthetic, char *ws, AdjArgs *g) {
+    const size_t tiles = (size_t)((np + kBlock - 1) / kBlock), nel = (size_t)(ntx + nrx);
+    const long long nch = nframes * ntx * nrx;
+    const size_t parts = (size_t)adjoint_parts(nch, np);
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        char *p = ws ? ws + at : nullptr;
+        at += (bytes + 255) & ~(size_t)255;
+        return p;
+    };
+    AdjArgs d = {};
+    d.gk_buf = reinterpret_cast<float *>(take(adjoint_grad_bytes(nframes, nrx, np)));
+    d.partial = reinterpret_cast<float *>(take(adjoint_partial_bytes(nframes, ntx, nrx, np, nt)));
+    d.live = reinterpret_cast<unsigned char *>(take((size_t)nrx * tiles));
+    d.ranges = reinterpret_cast<float2 *>(take(tiles * nel * sizeof(float2)));
+    d.depth = reinterpret_cast<float *>(take(tiles * sizeof(float)));
+    d.windows = reinterpret_cast<int2 *>(take(parts * (size_t)nch * sizeof(int2)));
+    d.order = reinterpret_cast<int *>(take(tiles * sizeof(int)));
+    const size_t table = nel * (size_t)np * sizeof(float);
+    if (synthetic && table <= kAdjTableMax) {
+        d.tau_tx = reinterpret_cast<float *>(take((size_t)ntx * np * sizeof(float)));
+        d.tau_rx = reinterpret_cast<float *>(take((size_t)nrx * np * sizeof(float)));
+    }
+    if (g) {
+        g->gk_buf = d.gk_buf;
+        g->partial = d.partial;
+        g->live = d.live;
+        g->ranges = d.ranges;
+        g->depth = d.depth;
+        g->windows = d.windows;
+        g->order = d.order;
+        g->tau_tx = d.tau_tx;
+        g->tau_rx = d.tau_rx;
+    }
+    return at;
 }
 
 cudaError_t launch_adjoint(const AdjArgs &g, int dtype, cudaStream_t s) {

@@ -301,19 +301,19 @@ struct AdjArgs {
     float *gk_buf;        // workspace: grad_out gathered into kernel pixel order
     float *partial;       // workspace: per-part sums of the spline-record adjoints
     unsigned char *live;  // workspace: live[r * tiles + tile] = receive r can contribute to the tile
+    float2 *ranges;       // workspace: per tile the delay ranges of ntx transmits, nrx receives
+    float *depth;         // workspace: per tile the earliest delay of the middle transmit
+    int2 *windows;        // workspace: per part and channel the intervals written in partial
+    int *order;           // workspace: the tiles by depth
+    float *tau_tx, *tau_rx;  // workspace: Synthetic delays (ntx, np), (nrx, np), or null
     const float *gk;      // set by launch_adjoint: gk_buf, or grad_out without pixel_index
     const int *plan;      // Tabbed: the forward's staging plan when its staged path applies, or NULL
 };
-// parts of the pixel range whose channel adjoints are summed separately, and
-// the workspace: [gathered gradient (nframes * nrx * np floats, 256-byte
-// rounded)][partial sums (parts * nch * 2 * Lp floats)][receive-tile liveness
-// (nrx * tiles bytes, 256-byte rounded)]
+// parts of the tiles whose channel adjoints are summed separately
 int adjoint_parts(long long nch, long long np);
-size_t adjoint_grad_bytes(long long nframes, long long nrx, long long np);
-size_t adjoint_partial_bytes(long long nframes, long long ntx, long long nrx, long long np, int nt);
-size_t adjoint_workspace_bytes(long long nframes, long long ntx, long long nrx, long long np,
-                               int nt);
-int adjoint_rows_warps(int nt);  // warps per scatter CTA (they share its rows), 0 = nt too large
+// the workspace: its size, and its pieces set in g (both may be null)
+size_t adjoint_layout(long long nframes, long long ntx, long long nrx, long long np, int nt,
+                      bool synthetic, char *ws, AdjArgs *g);
 cudaError_t launch_adjoint(const AdjArgs &a, int dtype, cudaStream_t s);
 cudaError_t launch_das_synth_slow(const DasArgs &a, int sumtype, int dtype, cudaStream_t s);
 

@@ -379,64 +379,6 @@ __host__ __device__ inline int cubic_column_padded(int ntx) {
     return (size_t)full * kBlock * sizeof(float) <= kColumnSmemMax ? full : (ntx + 1) / 2 * 2;
 }
 
-// Fast knots of N cubic taps x_k = fl(tt_k + trx), decided as the staged
-// kernel decides them: delay sums and quotients q = fl(fl(x - t0) * fl(1/dt))
-// two taps per instruction; s = q - 1/2 plus 1.5 * 2^23 rounds to the knot j
-// in the sum's low bits, and where |s - j| <= 1/2 - eps_fast the fast
-// quotient and the reference's correctly rounded one floor to the same j.
-// Bit k of inr: t0 <= x_k <= xmax; of near: the quotient is closer to an
-// integer (or NaN), so the caller redoes the taps it keeps with
-// cubic_knots_exact.  For a tap in range and not near, jj[k] <= nt - 1.
-template <int N>
-__device__ __forceinline__ void cubic_knots(const DasArgs &a, const float *tt, float trx,
-                                            float *xs, int *jj, float *fj, unsigned &inr,
-                                            unsigned &near) {
-    constexpr int NP = (N + 1) / 2;
-    const float2 trx2 = make_float2(trx, trx);
-    const float2 t02 = make_float2(a.t0, a.t0), inv2 = make_float2(a.inv_dt, a.inv_dt);
-    const float2 half2 = make_float2(0.5f, 0.5f), mag2 = make_float2(12582912.f, 12582912.f);
-    const float hmax = 0.5f - a.eps_fast;
-    inr = near = 0u;
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        const int k1 = (2 * p + 1 < N) ? 2 * p + 1 : 2 * p;
-        const float2 x2 = add2_rn(make_float2(tt[2 * p], tt[k1]), trx2);
-        const float2 q2 = mul2_rn(sub2_rn(x2, t02), inv2);
-        const float2 s2 = sub2_rn(q2, half2);
-        const float2 r2 = add2_rn(s2, mag2);
-        const float2 f2 = sub2_rn(r2, mag2);
-        const float2 h2 = sub2_rn(s2, f2);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int k = 2 * p + h;
-            if (k < N) {
-                const float x = h ? x2.y : x2.x;
-                xs[k] = x;
-                fj[k] = h ? f2.y : f2.x;
-                jj[k] = __float_as_int(h ? r2.y : r2.x) - 0x4B400000;
-                inr |= (unsigned)((x >= a.t0) && (x <= a.xmax)) << k;
-                near |= (unsigned)!(fabsf(h ? h2.y : h2.x) <= hmax) << k;
-            }
-        }
-    }
-}
-
-// the knots of the taps in `redo` from the IEEE quotient (the reference's rule)
-template <int N>
-__device__ __forceinline__ void cubic_knots_exact(const DasArgs &a, const float *xs, int *jj,
-                                                  float *fj, unsigned redo) {
-    using K = Kind<PYCBF_GB_INTERP_CUBIC, float>;
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-        if ((redo >> k) & 1u) {
-            int idx;
-            K::index_exact(xs[k], a, idx);
-            jj[k] = idx;
-            fj[k] = (float)idx;
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Cubic taps summed over the transmits of one receive, for every kernel
 // (generic, batched, staged): the same operations, so the same bits.

@@ -532,11 +532,11 @@ __device__ __forceinline__ float adj_cubic_group(const DasArgs &a, const TapCons
                 const float apod = h ? w2.y : w2.x;
                 const float slope =
                     fmaf(fmaf(3.f * pv[k].w, b, 2.f * pv[k].z), b, pv[k].y) * a.inv_dt;
-                const float d = apod * (gp * slope);
+                const float d = gp * slope;
                 const bool ok = (x >= c.t0) && (x <= c.xmax) && (fabsf(apod) >= c.thresh);
                 if (ok) {
-                    gt[k] += d;
-                    gr += d;
+                    gt[k] = fmaf(apod, d, gt[k]);
+                    gr = fmaf(apod, d, gr);
                 }
             }
         }

@@ -111,3 +111,28 @@ def test_dmas_lag_lists(lags, nsep, npx, power, sumlags):
     if sumlags:
         ref, mag = ref.sum(1), mag.sum(1)
     assert bool(((out.double() - ref).abs() <= 100 * 2.0 ** -24 * mag).all())
+
+
+@pytest.mark.parametrize("ntx,frames", [(2, 1), (13, 2)])
+def test_channel_gradient_in_any_pixel_order(ntx, frames):
+    """Parts whose taps span a long record (several segments of rows, pixels in random
+    order) and parts of similar depth give the same channel gradient, up to the
+    rounding of sums of some hundred terms in another order (float32: 1e-5)."""
+    from pycbf_gb300 import adjoint
+    r = np.random.default_rng(9)
+    nrx, npx, nt, dt = 6, 5000, 2100, 4e-8
+    depth = np.linspace(0.02, 0.7, npx) * nt * dt
+    tabs = [depth[None] + r.uniform(0, 40, (ntx, 1)) * dt, 0.4 * depth[None] + r.uniform(0, 90, (nrx, 1)) * dt,
+            np.ones((ntx, npx)), r.choice([0.0, 0.3, 1.0], (nrx, npx))]
+    tabs = [torch.as_tensor(t, dtype=torch.float32, device="cuda") for t in tabs]
+    rf = torch.randn((frames, ntx, nrx, nt), device="cuda")
+    gout = torch.randn((frames, npx), device="cuda")
+    perm = torch.as_tensor(r.permutation(npx), device="cuda")
+    got = []
+    for order in (torch.arange(npx, device="cuda"), perm):
+        x = rf.clone().requires_grad_(True)
+        out = adjoint.das_tabbed(x, *[t[:, order].contiguous() for t in tabs], t0=0.0, dt=dt)
+        out.backward(gout[:, order].contiguous())
+        got.append(x.grad.double())
+    assert float(got[0].abs().max()) > 0
+    assert float((got[0] - got[1]).norm() / got[0].norm()) < 1e-5
