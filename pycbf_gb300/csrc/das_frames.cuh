@@ -157,8 +157,7 @@ __global__ void __launch_bounds__(kBlock, 4) das_frames_kernel(const __grid_cons
                     tau = __ldg(a.tautx + (long long)(k + h) * np + i);
                     const float w = __ldg(a.apodtx + (long long)(k + h) * np + i);
                     amax = fmaxf(amax, fabsf(w));
-                    amin = fminf(amin, w);
-                    atop = fmaxf(atop, w);
+                    weight_range(w, amin, atop);
                 } else {
                     tau = synth_tx_delay(a, k + h, pnt);
                 }

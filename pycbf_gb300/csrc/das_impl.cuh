@@ -369,6 +369,14 @@ constexpr int kGroup = 6;  // taps whose gathers a thread keeps in flight togeth
 // 25 in float16 (registers); at eight slower throughout
 constexpr int kCubicGroup = 4;
 
+// Smallest and largest transmit weight of a pixel: where they are equal the weights are
+// all alike.  A NaN weight (its taps never count) is like no other.
+__device__ __forceinline__ void weight_range(float w, float &lo, float &hi) {
+    const bool nan = w != w;
+    lo = nan ? -__int_as_float(0x7f800000) : fminf(lo, w);
+    hi = nan ? __int_as_float(0x7f800000) : fmaxf(hi, w);
+}
+
 // The transmit delays of a pixel beyond kTxReg: a column of shared memory per
 // thread.  Cubic sums keep them as pairs, padded with infinite delays to whole
 // groups of kCubicGroup where that still fits; the padding of the last few
@@ -793,15 +801,13 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
     // the column form and so raises the CTAs per SM (two -> five at 75 transmits)
     float *sacc = stau + (size_t)ntx * kBlock;
     float amax = 0.f;  // max |apodtx| of this pixel, for the exact receive-level reject
-    float amin = __int_as_float(0x7f800000);  // min apodtx: the weights are all alike where it is
-    float atop = -amin;                       // also the max
+    float amin = __int_as_float(0x7f800000), atop = -amin;  // weight_range
     auto tx_side = [&](int t, float &tau, float &apod) {
         if (GEOM == GEOM_TABBED) {
             tau = __ldg(a.tautx + (long long)t * np + i);
             apod = __ldg(a.apodtx + (long long)t * np + i);
             amax = fmaxf(amax, fabsf(apod));
-            amin = fminf(amin, apod);
-            atop = fmaxf(atop, apod);
+            weight_range(apod, amin, atop);
         } else if (GEOM == GEOM_SYNTH) {
             tau = synth_tx_delay(a, t, pnt);
             apod = 1.f;

@@ -40,3 +40,21 @@ def test_sums_equal_their_single_taps(kind, storage, ntx, t0, dt):
     assert float(mag.max()) > 0 or (dt == 2.561e-8 and kind != "nearest")
     assert bool(((got - taps.sum((0, 1))).abs() <= 1e-5 * mag + 1e-30).all())
     assert bool(((each - taps.sum(0)).abs() <= 1e-5 * taps.abs().sum(0) + 1e-30).all())
+
+
+@pytest.mark.parametrize("kind", ["cubic", "linear"])
+@pytest.mark.parametrize("ntx", [3, 13, 40])
+def test_nan_weights_drop_their_taps(kind, ntx):
+    """A NaN weight among equal ones drops its tap, as a weight below the threshold does."""
+    case = _case(ntx, 70, 133, 64, 1.3e-6, 4e-8, ntx)
+    r = np.random.default_rng(ntx)
+    bad = r.uniform(size=(ntx, 133)) < 0.2
+    rf = r.standard_normal((3, ntx, 70, 64)).astype(np.float32)
+    images = []
+    for value in (np.nan, 0.0):
+        case["apodtx"] = np.where(bad, value, 1.0)
+        bf = pg.TabbedBeamformer(interp={"kind": kind}, stage_channels=False, **case)
+        images.append([bf(rf), np.stack([bf(f) for f in rf])])
+    assert np.abs(images[1][0]).max() > 0
+    for a, b in zip(*images):
+        np.testing.assert_array_equal(a, b)
