@@ -11,8 +11,7 @@ returns the images (cubic interpolation, summed over transmits and receives,
 the 'tx_and_rx' image of each beamformer).  The graph holds either two
 launches -- the batched prefilter and the persistent delay-and-sum of
 pycbf_gb_batch_run, every frame's tiles taken from one queue -- or every
-frame's own single-frame launches (the staged kernel for Tabbed frames with a
-plan) on a few concurrent branches.
+frame's own single-frame launches on a few concurrent branches.
 
 The form and its launch shape -- branches, pixel tiles per work item, work
 order, transmits held in registers per chunk, CTAs per SM -- are chosen by
@@ -140,8 +139,8 @@ class BatchBeamformer:
         return self._plans[key]
 
     def _launch_frame(self, k: int):
-        """Frame k with the single-frame launches of its beamformer (the staged
-        kernel for Tabbed frames with a plan), on the current stream."""
+        """Frame k with the single-frame launches of its beamformer, on the
+        current stream."""
         bf = self.beamformers[k]
         rf, coef, out = self.inputs[k], self._coef[k], self.outputs[k]
         L, stream = self._lib, _stream()

@@ -136,7 +136,8 @@ bool staged_ok(const pycbf_gb_rfinfo *rf, int interp, int sumtype, const void *d
 
 int launch_tabbed(const pycbf_gb_rfinfo *rf, DasArgs &a, int interp, int sumtype, const void *plan,
                   cudaStream_t s) {
-    if (plan && staged_ok(rf, interp, sumtype, a.data)) {
+    if (plan && staged_ok(rf, interp, sumtype, a.data) &&
+        (a.stall_test || !das_rx_ok(a, interp, sumtype))) {
         if (sumtype == PYCBF_GB_SUM_TX_ONLY) {  // rows of receives no pixel of a tile uses stay 0
             const size_t bytes = sizeof(float) * (size_t)rf->nframes * rf->nrx * (size_t)a.np;
             int st = cuda_status(cudaMemsetAsync(a.out, 0, bytes, s));
@@ -191,15 +192,17 @@ int prepare_data(const pycbf_gb_rfinfo *rf, const void *rfdata, int interp, void
 
 // Cubic images of several frames, in groups that share the decisions of a tap
 // (das_frames.cuh): the largest groups first, each prefiltered and summed in turn,
-// while at least `least` frames are left.  On return rf, rfdata, workspace and a.out
-// stand for the frames left to the single-frame kernels, if any.  The groups'
+// while at least two frames are left.  On return rf, rfdata, workspace and a.out
+// stand for the frame left to the single-frame kernels, if any.  The groups'
 // records take the space of the single frames' ones, so the workspace is no larger.
 //
-// Groups of four; of eight for 16-bit records of up to a gigabyte (eight Tabbed
-// float16 frames 0.85 against 0.94 ms; eight 3-D volumes, 3.4 GB, 56 against 54 ms).
+// Two frames gain already (tables, 11 transmits, 256 x 512 pixels: float32 285 -> 228 us,
+// float16 329 -> 247; 64 x 128 pixels 68 -> 72); the other side is das_rx_kernel once per
+// frame.  Groups of four; of eight for 16-bit records of up to a gigabyte (eight float16
+// frames of that table 0.54 against 0.70 ms; eight 3-D volumes, 3.4 GB, 65 against 57 ms).
 int take_frame_groups(pycbf_gb_rfinfo *rf, const void **rfdata, int geom, DasArgs &a, int sumtype,
-                      int least, void **workspace, size_t *workspace_bytes, cudaStream_t s) {
-    if (rf->nframes < least || !das_frames_ok(a, sumtype) || !spline_pairs_fit(rf->nt))
+                      void **workspace, size_t *workspace_bytes, cudaStream_t s) {
+    if (rf->nframes < 2 || !das_frames_ok(a, sumtype) || !spline_pairs_fit(rf->nt))
         return PYCBF_GB_OK;
     if (!*workspace || *workspace_bytes < pycbf_gb_workspace_bytes(rf, PYCBF_GB_INTERP_CUBIC))
         return PYCBF_GB_EWORKSPACE;
@@ -209,7 +212,7 @@ int take_frame_groups(pycbf_gb_rfinfo *rf, const void **rfdata, int geom, DasArg
     const size_t rec = gdt == PYCBF_GB_F32 ? 16 : 8;
     const size_t img = sumtype == PYCBF_GB_SUM_TX_ONLY ? (size_t)rf->nrx * a.np : (size_t)a.np;
     const int most = gdt != PYCBF_GB_F32 && 8 * frame * rec <= ((size_t)1 << 30) ? 8 : 4;
-    while (rf->nframes >= least) {
+    while (rf->nframes >= 2) {
         int fg = most;
         while (fg > rf->nframes) fg /= 2;
         const int n = (int)rf->nframes / fg * fg;
@@ -352,15 +355,8 @@ int pycbf_gb_das_tabbed(const pycbf_gb_rfinfo *rf, const void *rfdata, const flo
     a.thresh = thresh;
     pycbf_gb_rfinfo one = *rf;  // what the groups of frames leave
     if (interp == PYCBF_GB_INTERP_CUBIC) {
-        // with a staging plan the staged kernel is as fast for fewer frames (float32: 4
-        // frames 0.59 against 0.61 ms, 8 1.11 against 1.01; float16: 2 0.35 against
-        // 0.49, 4 0.62 against 0.59)
-        pycbf_gb_rfinfo rec = *rf;
-        if (rf->dtype == PYCBF_GB_I16) rec.dtype = PYCBF_GB_F32;
-        const bool staged = plan && staged_ok(&rec, interp, sumtype, workspace);
-        const int least = !staged ? 2 : rec.dtype == PYCBF_GB_F32 ? 8 : 4;
-        st = take_frame_groups(&one, &rfdata, GEOM_TABBED, a, sumtype, least, &workspace,
-                               &workspace_bytes, s);
+        st = take_frame_groups(&one, &rfdata, GEOM_TABBED, a, sumtype, &workspace, &workspace_bytes,
+                               s);
         if (st || one.nframes == 0) return st;
     }
     const void *data = nullptr;
@@ -451,8 +447,7 @@ int pycbf_gb_das_synthetic(const pycbf_gb_rfinfo *rf, const void *rfdata,
     a.thresh = 0.01f;
     pycbf_gb_rfinfo one = *rf;  // what the groups of frames leave
     if (interp == PYCBF_GB_INTERP_CUBIC) {
-        st = take_frame_groups(&one, &rfdata, GEOM_SYNTH, a, sumtype, 2, &workspace, &workspace_bytes,
-                               s);
+        st = take_frame_groups(&one, &rfdata, GEOM_SYNTH, a, sumtype, &workspace, &workspace_bytes, s);
         if (st || one.nframes == 0) return st;
     }
     const void *data = nullptr;

@@ -1,4 +1,5 @@
 // Dispatch of the delay-and-sum kernels by geometry and channel-data type.
+#include "das_frames.cuh"
 #include "das_staged.cuh"
 
 namespace pgb {
@@ -21,8 +22,8 @@ cudaError_t launch_das_frames_f16(const DasArgs &, int, int, int, cudaStream_t);
 cudaError_t launch_das_frames_bf16(const DasArgs &, int, int, int, cudaStream_t);
 
 bool das_frames_ok(const DasArgs &a, int sumtype) {
-    return a.fast_axis && cubic_column_padded(a.ntx) % kCubicGroup == 0 &&
-           sumtype != PYCBF_GB_SUM_NONE && sumtype != PYCBF_GB_SUM_RX_ONLY;
+    return a.fast_axis && sumtype != PYCBF_GB_SUM_NONE && sumtype != PYCBF_GB_SUM_RX_ONLY &&
+           das_frames_smem(GEOM_TABBED, sumtype, 8, a.ntx) <= 200 * 1024;
 }
 
 cudaError_t launch_das_frames(const DasArgs &a, int geom, int sumtype, int dtype, int fg,
@@ -58,8 +59,36 @@ cudaError_t launch_das_staged(const DasArgs &a, int interp, int sumtype, int dty
     }
 }
 
+cudaError_t launch_rx_f32(const DasArgs &, int, int, int, cudaStream_t);
+cudaError_t launch_rx_f16(const DasArgs &, int, int, int, cudaStream_t);
+cudaError_t launch_rx_bf16(const DasArgs &, int, int, int, cudaStream_t);
+
+// Sums over transmits of the kinds with packed decisions, on time axes that allow them
+// (fast_axis), at every size: das_rx_kernel is the faster one throughout (its figures are
+// beside it).  On other axes every tap takes the exact decisions, which
+// das_staged_kernel and das_kernel make.
+bool das_rx_ok(const DasArgs &a, int interp, int sumtype) {
+    if (interp != PYCBF_GB_INTERP_CUBIC && interp != PYCBF_GB_INTERP_LINEAR &&
+        interp != PYCBF_GB_INTERP_NEAREST)
+        return false;
+    return a.fast_axis && sumtype != PYCBF_GB_SUM_NONE && sumtype != PYCBF_GB_SUM_RX_ONLY &&
+           das_rx_smem(GEOM_TABBED, a.ntx, a.nrx) <= kRxSmemMax;
+}
+
+static cudaError_t launch_das_rx(const DasArgs &a, int geom, int interp, int sumtype, int dtype,
+                                 cudaStream_t s) {
+    switch (dtype) {
+        case PYCBF_GB_F32: return launch_rx_f32(a, geom, interp, sumtype, s);
+        case PYCBF_GB_F16: return launch_rx_f16(a, geom, interp, sumtype, s);
+        case PYCBF_GB_BF16: return launch_rx_bf16(a, geom, interp, sumtype, s);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
 cudaError_t launch_das(const DasArgs &a, int geom, int interp, int sumtype, int dtype, bool census,
                        cudaStream_t s) {
+    if (!census && geom != GEOM_SYNTH_SLOW && das_rx_ok(a, interp, sumtype))
+        return launch_das_rx(a, geom, interp, sumtype, dtype, s);
     if (geom == GEOM_TABBED) {
         switch (dtype) {
             case PYCBF_GB_F32: return launch_das_tabbed_f32(a, interp, sumtype, census, s);

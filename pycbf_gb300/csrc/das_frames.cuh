@@ -12,11 +12,18 @@
 //     frames per instruction in packed float32 pairs;
 //   16-bit:  one plane, (y y z z) of a and of b; each frame's y and z terms are
 //     summed side by side as in cubic_taps.
+//
+// The gathers and their latency bound it, so the receives are spread over the warps as
+// in das_rx_kernel.  Against a thread per pixel and all its receives (128 pixels, 16
+// warps an SM), with 11 transmits, 128 receives and 256 x 512 pixels from tables: four
+// float32 frames 591 -> 364 us, eight float16 857 -> 541; 64 x 256 pixels, eight frames
+// 567 -> 240 us; two 75-transmit synthetic frames 5.3 -> 4.7 ms; eight 3-D float16
+// volumes 53.8 -> 56.8 ms (the smaller tiles share fewer gathers in L1).
 // The operations on one frame and their order are those of cubic_taps and
 // das_pixel, so the images are the single-frame ones bit for bit.
 #pragma once
 
-#include "das_impl.cuh"
+#include "das_rx.cuh"
 
 namespace pgb {
 
@@ -121,151 +128,185 @@ __device__ __forceinline__ void frames_taps(const DasArgs &a, const TapConst &c,
     }
 }
 
-// One thread per pixel and group of FG frames (blockIdx.y); the transmit delays in
-// the thread's column of shared memory, as das_pixel keeps them.
+// receives whose sums (and table rows) are in shared memory together
+__host__ __device__ constexpr int frames_run(int geom, int fg) {
+    return geom == GEOM_SYNTH && fg == 2 ? 2 * kRxBlockSum : kRxBlockSum;
+}
+
+inline size_t das_frames_smem(int geom, int sum, int fg, int ntx) {
+    const size_t sums = sum == PYCBF_GB_SUM_TX_ONLY ? 0 : fg;
+    const size_t rows = (sums + (geom == GEOM_TABBED ? 4 : 0)) * frames_run(geom, fg);
+    return 32 * sizeof(float) * ((size_t)(ntx + 3) / 4 * 4 + rows);
+}
+
+// CTAs an SM.  Three (80 registers) hide more of the gathers: two 75-transmit float32
+// frames 4.7 against 5.7 ms, four 8.5 against 10.9; Tabbed groups of four and eight hold
+// the tables as well and gain nothing or spill (eight float16 frames 0.75 against 0.54 ms).
+constexpr int frames_ctas(int geom, int fg) { return fg <= (geom == GEOM_TABBED ? 2 : 4) ? 3 : 2; }
+
+// das_rx_kernel's division of the work for a group of FG frames (blockIdx.y): 32 pixels
+// a CTA, the receives of a block of kRxBlockSum spread over the warps, each receive's FG
+// sums in shared memory; warp f then adds frame f's, in order.
 template <int GEOM, int SUM, typename T, int FG>
-__global__ void __launch_bounds__(kBlock, 4) das_frames_kernel(const __grid_constant__ DasArgs a) {
+__global__ void __launch_bounds__(32 * kRxWarps, frames_ctas(GEOM, FG))
+    das_frames_kernel(const __grid_constant__ DasArgs a) {
     constexpr unsigned kFull = 0xffffffffu;
     constexpr bool W = GEOM == GEOM_TABBED;
-    constexpr bool kDmas = SUM == PYCBF_GB_SUM_DMAS_SSR;  // or POWER, by a.dmas_power
+    constexpr bool kEach = SUM == PYCBF_GB_SUM_TX_ONLY;  // written per receive, nothing to add
+    constexpr int kRun = frames_run(GEOM, FG);
+    static_assert(FG <= kRxWarps, "a warp adds a frame");
     extern __shared__ float sm[];
+    __shared__ float s_w[3][kRxWarps][32];  // Tabbed weights: largest magnitude, min, max
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long np = a.np;
-    long long i = (long long)blockIdx.x * kBlock + threadIdx.x;
+    long long i = (long long)blockIdx.x * 32 + lane;
     const bool valid = i < np;
     if (!valid) i = np - 1;
-    const int ntx = a.ntx, nrx = a.nrx;
+    const int ntx = a.ntx, nrx = a.nrx, ncol = (ntx + 3) / 4 * 4;
     const int f0 = (int)blockIdx.y * FG;
-    const int ncol = cubic_column_padded(ntx);
     const long long op = a.pixel_index ? (long long)__ldg(a.pixel_index + i) : i;
     const float inf = __int_as_float(0x7f800000);
+    float2 *col = reinterpret_cast<float2 *>(sm) + lane;  // [ncol / 2][32] transmit delays
+    float *sums = sm + (size_t)ncol * 32 + lane;          // [kRun][FG][32]
+    float *tabs = sums + (kEach ? 0 : kRun * FG * 32);    // as in das_rx_kernel
+    auto fetch_run = [&](int r0, int buf) {
+        rx_fetch_run<kRun, kRxWarps>(a, tabs + (size_t)buf * 2 * kRun * 32, r0, min(kRun, a.r1 - r0), w, i);
+    };
+    if (W) fetch_run(a.r0, 0);
+
+    float pnt[3] = {0.f, 0.f, 0.f};
+    if (!W)
+        for (int k = 0; k < 3; ++k) if (k < a.ndim) pnt[k] = __ldg(a.geo.pnts + i * a.ndim + k);
+    float amax = 0.f, amin = inf, atop = -inf;
+    rx_column<GEOM, kRxWarps>(a, pnt, i, w, col, amax, amin, atop);
+    if (W) {
+        s_w[0][w][lane] = amax;
+        s_w[1][w][lane] = amin;
+        s_w[2][w][lane] = atop;
+    }
     const TapConst tc(a);
     unsigned off[kCubicGroup];
 #pragma unroll
     for (int k = 0; k < kCubicGroup; ++k) off[k] = (unsigned)k * (unsigned)nrx * (unsigned)a.nt - kKnotBits;
-    float2 *col = reinterpret_cast<float2 *>(sm) + threadIdx.x;
-    float pnt[3] = {0.f, 0.f, 0.f};
-    if (GEOM == GEOM_SYNTH)
-        for (int k = 0; k < 3; ++k) if (k < a.ndim) pnt[k] = __ldg(a.geo.pnts + i * a.ndim + k);
-    float amax = 0.f, amin = inf, atop = -inf;
-    for (int k = 0; k < ncol; k += 2) {
-        float2 t = make_float2(inf, inf);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (k + h < ntx) {
-                float tau;
-                if (W) {
-                    tau = __ldg(a.tautx + (long long)(k + h) * np + i);
-                    const float w = __ldg(a.apodtx + (long long)(k + h) * np + i);
-                    amax = fmaxf(amax, fabsf(w));
-                    weight_range(w, amin, atop);
-                } else {
-                    tau = synth_tx_delay(a, k + h, pnt);
-                }
-                if (h) t.y = tau;
-                else t.x = tau;
-            }
+    __syncthreads();
+    if (W) {
+#pragma unroll 4
+        for (int k = 0; k < kRxWarps; ++k) {
+            amax = fmaxf(amax, s_w[0][k][lane]);
+            amin = fminf(amin, s_w[1][k][lane]);
+            atop = fmaxf(atop, s_w[2][k][lane]);
         }
-        col[(size_t)(k >> 1) * kBlock] = t;
     }
     const bool one_weight = W && __all_sync(kFull, amin == atop);
-
-    float acc[FG], s1[FG];  // s1: the current receive block's sum, or DMAS's running sum
-#pragma unroll
-    for (int f = 0; f < FG; ++f) acc[f] = s1[f] = 0.f;
     const unsigned long long plane = 16ULL * ntx * nrx * a.nt;  // bytes
     const char *base = static_cast<const char *>(a.data) +
                        (unsigned long long)blockIdx.y * FramesRec<T, FG>::kPlanes * plane;
     const long long rstep = 16LL * a.nt;
     const long long gstep = (long long)kCubicGroup * nrx * rstep;
-    if (SUM == PYCBF_GB_SUM_TX_AND_RX && a.r0 > 0) {
+    // warp f < FG: frame f's image so far and DMAS's running sum
+    float acc = 0.f, s1 = 0.f;
+    if (SUM == PYCBF_GB_SUM_TX_AND_RX && a.r0 > 0 && w < FG)
+        acc = a.out[(long long)(f0 + w) * np + op];
+    int buf = 0;
+    for (int r0 = a.r0; r0 < a.r1; r0 += kRun, buf ^= 1) {
+        const int n = min(kRun, a.r1 - r0);
+        if (W) {
+            fetch_run(min(r0 + kRun, a.r1), buf ^ 1);  // none past the last: an empty group
+            copy_wait_but_one();
+        }
+        const float *tab = tabs + (size_t)buf * 2 * kRun * 32;
+        for (int e = w; e < n; e += kRxWarps) {
+            const int r = r0 + e;
+            float trx, arx = 1.f;
+            bool live;
+            if (W) {
+                trx = tab[e * 32];
+                arx = tab[(kRun + e) * 32];
+                live = __fmul_rn(amax, fabsf(arx)) >= a.thresh;
+            } else {
+                trx = synth_rx_delay_warp(a, r, pnt);
+                live = trx != inf;
+            }
+            FramesAcc<T, FG> sum;
 #pragma unroll
-        for (int f = 0; f < FG; ++f) acc[f] = a.out[(long long)(f0 + f) * np + op];
-    }
-    base += a.r0 * rstep;
-    for (int r = a.r0; r < a.r1; ++r, base += rstep) {
-        if (SUM == PYCBF_GB_SUM_TX_AND_RX && r > a.r0 && r % kRxBlockSum == 0) {
+            for (int k = 0; k < FramesAcc<T, FG>::n; ++k) sum.v[k] = make_float2(0.f, 0.f);
+            if (__any_sync(kFull, live)) {
+                const char *rec = base + r * rstep;
+                for (int g = 0; g < ncol; g += kCubicGroup, rec += gstep) {
+                    float2 t2[kCubicGroup / 2], w2[kCubicGroup / 2];
+#pragma unroll
+                    for (int p = 0; p < kCubicGroup / 2; ++p) {
+                        t2[p] = col[(g / 2 + p) * 32];
+                        w2[p] = make_float2(amin, amin);
+                    }
+                    if (W && !one_weight) {
+                        float *v = reinterpret_cast<float *>(w2);
+#pragma unroll
+                        for (int k = 0; k < kCubicGroup; ++k)
+                            v[k] = __ldg(a.apodtx + (long long)min(g + k, ntx - 1) * np + i);
+                    }
+                    frames_taps<GEOM, T, FG>(a, tc, t2, w2, trx, arx, rec, plane, off, sum);
+                }
+            }
 #pragma unroll
             for (int f = 0; f < FG; ++f) {
-                acc[f] += s1[f];
-                s1[f] = 0.f;
-            }
-        }
-        float trx, arx = 1.f;
-        bool live;
-        if (W) {
-            trx = __ldg(a.taurx + (long long)r * np + i);
-            arx = __ldg(a.apodrx + (long long)r * np + i);
-            live = __fmul_rn(amax, fabsf(arx)) >= a.thresh;
-        } else {
-            trx = synth_rx_delay_warp(a, r, pnt);
-            live = trx != inf;
-        }
-        FramesAcc<T, FG> sum;
-#pragma unroll
-        for (int k = 0; k < FramesAcc<T, FG>::n; ++k) sum.v[k] = make_float2(0.f, 0.f);
-        if (__any_sync(kFull, live)) {
-            const char *rec = base;
-            for (int g = 0; g < ncol; g += kCubicGroup, rec += gstep) {
-                float2 t2[kCubicGroup / 2], w2[kCubicGroup / 2];
-#pragma unroll
-                for (int p = 0; p < kCubicGroup / 2; ++p) {
-                    t2[p] = col[(size_t)(g / 2 + p) * kBlock];
-                    w2[p] = make_float2(amin, amin);
+                float v = sum.total(f);
+                if (kEach) {
+                    if (valid) a.out[((long long)(f0 + f) * nrx + r) * np + op] = v;
+                } else {
+                    if (SUM == PYCBF_GB_SUM_DMAS_SSR && !a.dmas_power)
+                        v = copysignf(sqrtf(fabsf(v)), v);
+                    sums[(e * FG + f) * 32] = v;
                 }
-                if (W && !one_weight) {
-                    float *w = reinterpret_cast<float *>(w2);
-#pragma unroll
-                    for (int k = 0; k < kCubicGroup; ++k)
-                        w[k] = __ldg(a.apodtx + (long long)min(g + k, ntx - 1) * np + i);
+            }
+        }
+        if (kEach) continue;
+        __syncthreads();
+        if (w < FG) {
+            for (int e0 = 0; e0 < n; e0 += kRxBlockSum) {
+                const int e1 = min(n, e0 + kRxBlockSum);
+                float b = 0.f;
+#pragma unroll 8
+                for (int e = e0; e < e1; ++e) {
+                    const float v = sums[(e * FG + w) * 32];
+                    if (SUM == PYCBF_GB_SUM_TX_AND_RX) {
+                        b += v;
+                    } else {
+                        acc = fmaf(v, s1, acc);
+                        s1 += v;
+                    }
                 }
-                frames_taps<GEOM, T, FG>(a, tc, t2, w2, trx, arx, rec, plane, off, sum);
-            }
-        } else if (SUM != PYCBF_GB_SUM_TX_ONLY) {
-            continue;
-        }
-#pragma unroll
-        for (int f = 0; f < FG; ++f) {
-            const float v = sum.total(f);
-            if (SUM == PYCBF_GB_SUM_TX_AND_RX) s1[f] += v;
-            if (SUM == PYCBF_GB_SUM_TX_ONLY && valid)
-                a.out[((long long)(f0 + f) * nrx + r) * np + op] = v;
-            if (kDmas) {
-                const float s = a.dmas_power ? v : copysignf(sqrtf(fabsf(v)), v);
-                acc[f] = fmaf(s, s1[f], acc[f]);
-                s1[f] += s;
+                acc += b;
             }
         }
+        __syncthreads();
     }
-    if (!valid || SUM == PYCBF_GB_SUM_TX_ONLY) return;
-#pragma unroll
-    for (int f = 0; f < FG; ++f)
-        a.out[(long long)(f0 + f) * np + op] =
-            SUM == PYCBF_GB_SUM_TX_AND_RX ? acc[f] + s1[f] : acc[f];
+    if (!kEach && w < FG && valid) a.out[(long long)(f0 + w) * np + op] = acc;
 }
 
 // Records of more than a gigabyte pass through L2 while the tiles run at every
-// receive at once, so such launches go block of receives by block of receives
-// (kRxBlockSum: the sums so far carry over in the image).  Two 192-element float32
-// frames of 75 transmits (1.9 GB): 6.06 -> 5.33 ms; eight 3-D float16 volumes (3.4
-// GB): 75 -> 56 ms; 0.18 GB of Tabbed frames: 0.85 -> 0.89 ms, so they go in one.
+// receive at once, so such launches go by kFramesStep receives at a time (whole blocks
+// of kRxBlockSum: the sums so far carry over in the image).  Eight 3-D float16 volumes
+// (3.4 GB of records): 59.4 ms in one launch, 56.8 by 256 or 128 receives, 57.7 by 64.
 constexpr long long kFramesSplitBytes = 1LL << 30;
+constexpr int kFramesStep = 256;
 
 template <int GEOM, int SUM, typename T, int FG>
 cudaError_t launch_das_frames_one(DasArgs a, cudaStream_t s) {
     auto kern = das_frames_kernel<GEOM, SUM, T, FG>;
-    const size_t smem = (size_t)kBlock * cubic_column_padded(a.ntx) * sizeof(float);
-    if (smem > 48 * 1024) {
+    const size_t smem = das_frames_smem(GEOM, SUM, FG, a.ntx);
+    if (smem > 40 * 1024) {  // with the static part
         cudaError_t err =
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (err != cudaSuccess) return err;
     }
-    const dim3 grid((unsigned)((a.np + kBlock - 1) / kBlock), (unsigned)(a.nframes / FG));
+    const dim3 grid((unsigned)((a.np + 31) / 32), (unsigned)(a.nframes / FG));
     const long long bytes = 16LL * FramesRec<T, FG>::kPlanes * a.ntx * a.nrx * a.nt;
     const bool split = SUM != PYCBF_GB_SUM_DMAS_SSR && bytes > kFramesSplitBytes;
-    const int step = split ? kRxBlockSum : a.nrx;
+    const int step = split ? kFramesStep : a.nrx;
     for (a.r0 = 0; a.r0 < a.nrx; a.r0 += step) {
         a.r1 = std::min(a.nrx, a.r0 + step);
-        kern<<<grid, kBlock, smem, s>>>(a);
+        kern<<<grid, 32 * kRxWarps, smem, s>>>(a);
         cudaError_t err = cudaGetLastError();
         if (err != cudaSuccess) return err;
     }
