@@ -164,6 +164,7 @@ int pycbf_gb_spline_coefficients(const pycbf_gb_rfinfo *rf, const void *rfdata, 
 /* locality-friendly order).  plan: NULL, or a staging plan built by       */
 /* pycbf_gb_tabbed_plan for these tables, this thresh and this interp;     */
 /* with it, ntx <= 12 and sumtype tx_only / tx_and_rx / dmas, the kernel   */
+/* for time axes coarser than float32 delays (every tap decided exactly)   */
 /* stages channel windows in shared memory by TMA (same results).  out is  */
 /* written, not accumulated.                                               */
 /* ---------------------------------------------------------------------- */
@@ -428,11 +429,9 @@ int pycbf_gb_das_tabbed_adjoint(const pycbf_gb_rfinfo *rf, const void *coef,
                                 float *grad_rf, float *grad_tautx, float *grad_taurx,
                                 void *workspace, size_t workspace_bytes, void *stream);
 /* The same with the forward's staging plan (pycbf_gb_tabbed_plan of these   */
-/* tables, or NULL): where the plan's staged path applies (cubic, float32   */
-/* channel data, one frame, ntx <= 12), the delay gradients gather the      */
-/* records from its staged windows.  The plan's queue head is reused, so it */
-/* must not be in use by another call at the same time.  No counterpart in  */
-/* the reference, whose beamformers are forward-only.                       */
+/* tables, or NULL), which is checked for alignment only: the gradients do  */
+/* not need it.  No counterpart in the reference, whose beamformers are     */
+/* forward-only.                                                            */
 int pycbf_gb_das_tabbed_adjoint_planned(const pycbf_gb_rfinfo *rf, const void *coef,
                                         const float *tautx, const float *apodtx,
                                         const float *taurx, const float *apodrx, long long np,

@@ -208,8 +208,8 @@ def das_tabbed(rf: torch.Tensor, tautx: torch.Tensor, taurx: torch.Tensor, apodt
     (np,) / (nframes, np) for 'tx_and_rx', (nrx, np) / (nframes, nrx, np) for
     'tx_only'.  Values equal TabbedBeamformer(interp cubic) on the same inputs.
     plan: a staging plan built for exactly these tables and thresh
-    (pycbf_gb_tabbed_plan): the forward then runs the staged kernel, and so
-    do the delay gradients for one frame of float32 channel data.
+    (pycbf_gb_tabbed_plan), which the forward uses where its staged kernel
+    runs; the values and gradients are the same with or without it.
     """
     _check_rf(rf)
     rf4, squeeze = _as4(rf)

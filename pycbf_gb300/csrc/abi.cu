@@ -685,11 +685,6 @@ int pycbf_gb_das_tabbed_adjoint_planned(const pycbf_gb_rfinfo *rf, const void *c
     g.grad_rf = grad_rf;
     g.grad_tautx = grad_tautx;
     g.grad_taurx = grad_taurx;
-    // the staged delay gradients need the plan's staged path for cubic
-    // float32 records and one frame; otherwise the plan is not used
-    if (plan && rf->nframes == 1 && rf->dtype == PYCBF_GB_F32 &&
-        staged_ok(rf, PYCBF_GB_INTERP_CUBIC, sumtype, coef))
-        g.plan = static_cast<const int *>(plan);
     return run_adjoint(rf, g, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
 }
 

@@ -8,8 +8,8 @@
 // samples, D the second difference; natural ends z_0 = z_nt-1 = 0).
 //
 // Three kernels, all deterministic (no atomics; every sum has a fixed order):
-//   adj_delay_kernel    one thread per pixel: dL/dx = g w S'(x) summed into
-//                       dL/dtau_tx (ntx, np) and dL/dtau_rx (nrx, np) for
+//   adj_delay_kernel    a warp per 32 pixels and share of the receives:
+//                       dL/dx = g w S'(x) summed into dL/dtau_tx (ntx, np) and dL/dtau_rx (nrx, np) for
 //                       Tabbed tables, or into dL/ds (np) for the Synthetic
 //                       slowness form (x = (D_tx + D_rx) s + t0).
 //   adj_scatter_kernel  one warp per (channel, part of the tiles): the transpose of
@@ -27,7 +27,7 @@
 // the tap decisions (range, threshold, correctly rounded knot) are the forward's.
 #include <algorithm>
 
-#include "das_impl.cuh"
+#include "das_rx.cuh"
 
 namespace pgb {
 
@@ -61,65 +61,100 @@ __global__ void adj_gather_kernel(const float *__restrict__ gout, const int *__r
 // delays / slowness: gather per pixel
 // ---------------------------------------------------------------------------
 // Bound by the issue rate and the latency of the gathers, as the forward: the taps
-// are decided by its operations (knot_pairs), four at a time, in pairs.  Per thread a
-// column of shared memory for pairs of transmits: delay, weight (Tabbed) or path
-// length (Synthetic), and the running dL/dtau_tx.
-template <int GEOM, int SUM, typename T>
-__global__ void __launch_bounds__(kBlock, 6) adj_delay_kernel(const __grid_constant__ AdjArgs g) {
+// are decided by its operations (knot_pairs), four at a time, in pairs, and the
+// receives of 32 pixels are spread over the warps as in das_rx_kernel.  The warps share
+// a column of delays and of weights (Tabbed) or path lengths (Synthetic); each has its
+// own running dL/dtau_tx, added in warp order at the end.  11 transmits, 128 receives,
+// 256 x 512 pixels: with a thread per pixel and all its receives 339 us from tables and
+// 302 for the slowness (the whole call 955 and 1344 us); so 780 and 1113 (gathers from
+// staged windows, as the TMA kernel of the forward makes them, measured 20 % slower).
+//
+// ONE: one frame on a time axis with packed decisions.  The gradient then goes into the
+// weights, so a tap is its decisions, a gather, the slope of its cubic and two
+// multiply-adds; otherwise the frames' products are summed per tap, and the knots of
+// other axes are quotients.
+template <int GEOM, int SUM, typename T, bool ONE>
+__global__ void __launch_bounds__(32 * kRxWarps, 4) adj_delay_kernel(const __grid_constant__ AdjArgs g) {
     using rec = typename CoefRec<T>::raw;
-    constexpr int G = kCubicGroup;
+    constexpr int G = kCubicGroup, kRun = kRxRun<GEOM_TABBED>;
+    constexpr bool W = GEOM == GEOM_TABBED;
     const DasArgs &a = g.d;
     extern __shared__ float2 smp[];
-    const int tid = threadIdx.x;
+    __shared__ float s_part[kRxWarps][32];  // largest weights; then dL/dslowness
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long np = a.np;
-    long long i = (long long)blockIdx.x * kBlock + tid;
+    long long i = (long long)blockIdx.x * 32 + lane;
     const bool valid = i < np;
     if (!valid) i = np - 1;
     const int ntx = a.ntx, nrx = a.nrx, nfr = a.nframes, nt = a.nt;
-    const int ncol = cubic_column_padded(ntx);
+    const int npair = (ntx + 3) / 4 * 2, ncol = 2 * npair;
     const float inf = __int_as_float(0x7f800000);
     const TapConst tc(a);
-    float2 *stau = smp + tid, *sw = stau + (size_t)(ncol / 2) * kBlock,
-           *sg = sw + (size_t)(ncol / 2) * kBlock;
+    float2 *stau = smp + lane, *sw = stau + (size_t)npair * 32,
+           *sg = sw + (size_t)npair * 32 * (1 + w);  // Tabbed: [kRxWarps][npair][32]
+    float *tabs = reinterpret_cast<float *>(smp + (size_t)npair * 32 * (2 + kRxWarps)) + lane;
+    auto fetch_run = [&](int r0, int buf) {
+        rx_fetch_run<kRun, kRxWarps>(a, tabs + (size_t)buf * 2 * kRun * 32, r0, min(kRun, nrx - r0), w, i);
+    };
+    if (W) fetch_run(0, 0);
 
     float pnt[3] = {0.f, 0.f, 0.f};
     float slow = 0.f;
-    if (GEOM == GEOM_SYNTH_SLOW) {
+    if (!W) {
         for (int k = 0; k < 3; ++k) if (k < a.ndim) pnt[k] = __ldg(a.geo.pnts + i * a.ndim + k);
         slow = __ldg(a.slow + i);
     }
     float amax = 0.f;
-    for (int t = 0; t < ncol; t += 2) {
-        float tau[2] = {inf, inf}, w[2] = {0.f, 0.f};  // padding: never counts
+    for (int p = w; p < npair; p += kRxWarps) {
+        float tau[2] = {inf, inf}, wt[2] = {0.f, 0.f};  // padding: never counts
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            if (t + h >= ntx) continue;
-            if (GEOM == GEOM_TABBED) {
-                tau[h] = __ldg(a.tautx + (long long)(t + h) * np + i);
-                w[h] = __ldg(a.apodtx + (long long)(t + h) * np + i);
-                amax = fmaxf(amax, fabsf(w[h]));
+            const int t = 2 * p + h;
+            if (t >= ntx) continue;
+            if (W) {
+                tau[h] = __ldg(a.tautx + (long long)t * np + i);
+                wt[h] = __ldg(a.apodtx + (long long)t * np + i);
+                amax = fmaxf(amax, fabsf(wt[h]));
             } else {
                 float t0add;
-                const bool ok = synth_tx_path(a, t + h, pnt, w[h], t0add);
-                tau[h] = slow_delay(ok, w[h], slow, t0add);
+                const bool ok = synth_tx_path(a, t, pnt, wt[h], t0add);
+                tau[h] = slow_delay(ok, wt[h], slow, t0add);
             }
         }
-        stau[(size_t)(t / 2) * kBlock] = make_float2(tau[0], tau[1]);
-        sw[(size_t)(t / 2) * kBlock] = make_float2(w[0], w[1]);
-        sg[(size_t)(t / 2) * kBlock] = make_float2(0.f, 0.f);
+        stau[(size_t)p * 32] = make_float2(tau[0], tau[1]);
+        sw[(size_t)p * 32] = make_float2(wt[0], wt[1]);
+    }
+    if (W) {
+        for (int p = 0; p < npair; ++p) sg[(size_t)p * 32] = make_float2(0.f, 0.f);
+        s_part[w][lane] = amax;
+    }
+    __syncthreads();
+    if (W) {
+#pragma unroll
+        for (int k = 0; k < kRxWarps; ++k) amax = fmaxf(amax, s_part[k][lane]);
     }
     const long long chs = (long long)nrx * nt;
     unsigned off[G];
 #pragma unroll
     for (int k = 0; k < G; ++k) off[k] = (unsigned)k * (unsigned)chs - kKnotBits;
 
+    const float gpix = nfr == 1 && SUM == PYCBF_GB_SUM_TX_AND_RX ? __ldg(g.gk + i) : 0.f;
     float gs = 0.f;
-    for (int r = 0; r < nrx; ++r) {
+    // receive r by warp r % kRxWarps (a run is a multiple of kRxWarps)
+    int buf = 1;
+    for (int r = w; r < nrx; r += kRxWarps) {
         float trx, arx = 1.f, Drx = 0.f;
         bool live;
-        if (GEOM == GEOM_TABBED) {
-            trx = __ldg(a.taurx + (long long)r * np + i);
-            arx = __ldg(a.apodrx + (long long)r * np + i);
+        if (W) {
+            const int e = r % kRun;
+            if (e == w) {  // the warp's first receive of a run
+                buf ^= 1;
+                fetch_run(min(r - w + kRun, nrx), buf ^ 1);  // none past the last: an empty group
+                copy_wait_but_one();
+            }
+            const float *tab = tabs + (size_t)buf * 2 * kRun * 32;
+            trx = tab[e * 32];
+            arx = tab[(kRun + e) * 32];
             live = __fmul_rn(amax, fabsf(arx)) >= a.thresh;
         } else {
             live = synth_rx_path(a, r, pnt, Drx);
@@ -128,18 +163,21 @@ __global__ void __launch_bounds__(kBlock, 6) adj_delay_kernel(const __grid_const
         float grx = 0.f;
         // the forward's exact reject, by warps: no tap of the others passes its tests
         if (__any_sync(kFull, live)) {
-            const float gp0 = nfr == 1 ? __ldg(g.gk + grad_row(SUM, 0, r, nrx) * np + i) : 0.f;
+            const float gp0 = nfr == 1 && SUM == PYCBF_GB_SUM_TX_ONLY
+                                  ? __ldg(g.gk + (long long)r * np + i) : gpix;
+            const float gq = CoefRec<T>::kPoly ? gp0 * a.inv_dt : gp0;
+            const rec *row = static_cast<const rec *>(a.data) + (long long)r * nt;
             for (int t0 = 0; t0 < ncol; t0 += G) {
                 float2 tt2[G / 2], w2[G / 2], x2[G / 2], fj2[G / 2];
                 unsigned rk[G];
 #pragma unroll
                 for (int p = 0; p < G / 2; ++p) {
-                    tt2[p] = stau[(size_t)(t0 / 2 + p) * kBlock];
-                    w2[p] = sw[(size_t)(t0 / 2 + p) * kBlock];
+                    tt2[p] = stau[(size_t)(t0 / 2 + p) * 32];
+                    w2[p] = sw[(size_t)(t0 / 2 + p) * 32];
                     if (GEOM == GEOM_TABBED) w2[p] = mul2_rn(w2[p], make_float2(arx, arx));
                 }
                 knot_pairs<G / 2>(a, tc, tt2, trx, x2, fj2, rk);
-                if (!a.fast_axis) {  // knots past the record are clamped
+                if (!ONE && !a.fast_axis) {  // knots past the record are clamped
 #pragma unroll
                     for (int k = 0; k < G; ++k) {
                         const float fl = fminf(floorf(__fdiv_rn(__fsub_rn(pair_lane(x2, k), a.t0), a.dt)),
@@ -157,6 +195,47 @@ __global__ void __launch_bounds__(kBlock, 6) adj_delay_kernel(const __grid_const
                     ok[k] = (x >= tc.t0) && (x <= tc.xmax);
                     if (GEOM == GEOM_TABBED) ok[k] = ok[k] && (fabsf(pair_lane(w2, k)) >= tc.thresh);
                     sum[k] = 0.f;
+                }
+                if constexpr (ONE) {
+                    rec c[G];
+#pragma unroll
+                    for (int k = 0; k < G; ++k)
+                        if (ok[k]) c[k] = __ldg(row + (rk[k] + off[k]));
+                    row += G * chs;
+#pragma unroll
+                    for (int p = 0; p < G / 2; ++p) {
+                        float2 slope;
+                        if constexpr (CoefRec<T>::kPoly) {  // c1 + 2 b (c2 + 1.5 b c3), times 1/dt (gq)
+                            const float2 b2 = knot_frac2(tc, x2[p], fj2[p]);
+                            const float2 u2 = add2_rn(b2, b2), v2 = mul2_rn(b2, make_float2(1.5f, 1.5f));
+                            const rec &cx = c[2 * p], &cy = c[2 * p + 1];
+                            slope.x = fmaf(fmaf(cx.w, v2.x, cx.z), u2.x, cx.y);
+                            slope.y = fmaf(fmaf(cy.w, v2.y, cy.z), u2.y, cy.y);
+                        } else {
+                            slope.x = Kind<PYCBF_GB_INTERP_CUBIC, T>::slope(
+                                CoefRec<T>::unpack(c[2 * p]), x2[p].x, fj2[p].x, a);
+                            slope.y = Kind<PYCBF_GB_INTERP_CUBIC, T>::slope(
+                                CoefRec<T>::unpack(c[2 * p + 1]), x2[p].y, fj2[p].y, a);
+                        }
+                        if (W) {
+                            const float2 h = mul2_rn(w2[p], make_float2(gq, gq));
+                            float2 d = sg[(size_t)(t0 / 2 + p) * 32];
+                            if (ok[2 * p]) {
+                                d.x = fmaf(h.x, slope.x, d.x);
+                                grx = fmaf(h.x, slope.x, grx);
+                            }
+                            if (ok[2 * p + 1]) {
+                                d.y = fmaf(h.y, slope.y, d.y);
+                                grx = fmaf(h.y, slope.y, grx);
+                            }
+                            sg[(size_t)(t0 / 2 + p) * 32] = d;
+                        } else {  // dx/ds = D_tx + D_rx; times gq at the end of the receive
+                            const float2 D = add2_rn(w2[p], make_float2(Drx, Drx));
+                            if (ok[2 * p]) grx = fmaf(slope.x, D.x, grx);
+                            if (ok[2 * p + 1]) grx = fmaf(slope.y, D.y, grx);
+                        }
+                    }
+                    continue;
                 }
                 for (int f = 0; f < nfr; ++f) {
                     const float gp = nfr == 1 ? gp0 : __ldg(g.gk + grad_row(SUM, f, r, nrx) * np + i);
@@ -186,7 +265,7 @@ __global__ void __launch_bounds__(kBlock, 6) adj_delay_kernel(const __grid_const
 #pragma unroll
                 for (int p = 0; p < G / 2; ++p) {
                     if (GEOM == GEOM_TABBED) {
-                        float2 d = sg[(size_t)(t0 / 2 + p) * kBlock];
+                        float2 d = sg[(size_t)(t0 / 2 + p) * 32];
                         if (ok[2 * p]) {
                             d.x = fmaf(w2[p].x, sum[2 * p], d.x);
                             grx = fmaf(w2[p].x, sum[2 * p], grx);
@@ -195,24 +274,35 @@ __global__ void __launch_bounds__(kBlock, 6) adj_delay_kernel(const __grid_const
                             d.y = fmaf(w2[p].y, sum[2 * p + 1], d.y);
                             grx = fmaf(w2[p].y, sum[2 * p + 1], grx);
                         }
-                        sg[(size_t)(t0 / 2 + p) * kBlock] = d;
+                        sg[(size_t)(t0 / 2 + p) * 32] = d;
                     } else {  // dx/ds = D_tx + D_rx
                         if (ok[2 * p]) gs = fmaf(sum[2 * p], w2[p].x + Drx, gs);
                         if (ok[2 * p + 1]) gs = fmaf(sum[2 * p + 1], w2[p].y + Drx, gs);
                     }
                 }
             }
+            if (ONE && !W) gs = fmaf(gq, grx, gs);
         }
-        if (GEOM == GEOM_TABBED && g.grad_taurx && valid) g.grad_taurx[(long long)r * np + i] = grx;
+        if (W && g.grad_taurx && valid) g.grad_taurx[(long long)r * np + i] = grx;
     }
+    if (!W) s_part[w][lane] = gs;
+    __syncthreads();
     if (!valid) return;
-    if (GEOM == GEOM_TABBED && g.grad_tautx) {
-        for (int t = 0; t < ntx; ++t) {
-            const float2 d = sg[(size_t)(t / 2) * kBlock];
-            g.grad_tautx[(long long)t * np + i] = (t & 1) ? d.y : d.x;
+    if (W && g.grad_tautx) {
+        const float2 *part = sw + (size_t)npair * 32;
+        for (int p = w; p < npair; p += kRxWarps) {
+            float2 d = part[(size_t)p * 32];
+#pragma unroll
+            for (int k = 1; k < kRxWarps; ++k) d = add2_rn(d, part[((size_t)k * npair + p) * 32]);
+            if (2 * p < ntx) g.grad_tautx[(long long)(2 * p) * np + i] = d.x;
+            if (2 * p + 1 < ntx) g.grad_tautx[(long long)(2 * p + 1) * np + i] = d.y;
         }
     }
-    if (GEOM == GEOM_SYNTH_SLOW && g.grad_slow) g.grad_slow[i] = gs;
+    if (!W && w == 0 && g.grad_slow) {
+#pragma unroll
+        for (int k = 1; k < kRxWarps; ++k) gs += s_part[k][lane];
+        g.grad_slow[i] = gs;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -590,21 +680,23 @@ adj_finalize_kernel(const float *__restrict__ partial, const int2 *__restrict__ 
 }
 
 
-size_t delay_smem_bytes(int ntx) {
-    return 3 * (size_t)cubic_column_padded(ntx) * kBlock * sizeof(float);
+size_t delay_smem_bytes(int geom, int ntx) {
+    const size_t column = (size_t)((ntx + 3) / 4 * 4) * 32 * sizeof(float);
+    return geom == GEOM_TABBED ? (2 + kRxWarps) * column + 4 * kRxRun<GEOM_TABBED> * 32 * sizeof(float)
+                               : 2 * column;
 }
 
 template <int GEOM, int SUM, typename T>
 cudaError_t launch_delay_one(const AdjArgs &g, cudaStream_t s) {
-    auto kern = adj_delay_kernel<GEOM, SUM, T>;
-    const size_t smem = delay_smem_bytes(g.d.ntx);
-    if (smem > 48 * 1024) {
+    auto kern = g.d.fast_axis && g.d.nframes == 1 ? adj_delay_kernel<GEOM, SUM, T, true>
+                                                  : adj_delay_kernel<GEOM, SUM, T, false>;
+    const size_t smem = delay_smem_bytes(GEOM, g.d.ntx);
+    if (smem > 40 * 1024) {  // with the static part
         cudaError_t err =
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (err != cudaSuccess) return err;
     }
-    const long long bx = (g.d.np + kBlock - 1) / kBlock;
-    kern<<<(unsigned)bx, kBlock, smem, s>>>(g);
+    kern<<<(unsigned)((g.d.np + 31) / 32), 32 * kRxWarps, smem, s>>>(g);
     return cudaGetLastError();
 }
 
@@ -669,17 +761,7 @@ cudaError_t launch_scatter_one(const AdjArgs &g0, cudaStream_t s) {
 template <int GEOM, int SUM, typename T>
 cudaError_t launch_adjoint_gs(const AdjArgs &g, cudaStream_t s) {
     if (g.grad_tautx || g.grad_taurx || g.grad_slow) {
-        cudaError_t err;
-        if (GEOM == GEOM_TABBED && g.plan && CoefRec<T>::kPoly) {
-            // the forward's staging plan: the delay gradients gather from staged windows
-            DasArgs d = g.d;
-            d.gk = g.gk;
-            d.gtx = g.grad_tautx;
-            d.grx = g.grad_taurx;
-            err = launch_das_staged_adj(d, SUM, PYCBF_GB_F32, g.plan, s);
-        } else {
-            err = launch_delay_one<GEOM, SUM, T>(g, s);
-        }
+        cudaError_t err = launch_delay_one<GEOM, SUM, T>(g, s);
         if (err != cudaSuccess) return err;
     }
     if (g.grad_rf) return launch_scatter_one<GEOM, SUM>(g, s);
@@ -782,19 +864,21 @@ cudaError_t launch_adjoint(const AdjArgs &g, int dtype, cudaStream_t s) {
     }
 }
 
+template <typename T>
+static cudaError_t launch_synth_slow_t(const DasArgs &a, int sumtype, cudaStream_t s) {
+    constexpr int CU = PYCBF_GB_INTERP_CUBIC, GE = GEOM_SYNTH_SLOW;
+    constexpr int BOTH = PYCBF_GB_SUM_TX_AND_RX, EACH = PYCBF_GB_SUM_TX_ONLY;
+    if (das_rx_ok(a, CU, sumtype))
+        return sumtype == BOTH ? launch_rx_one<GE, CU, BOTH, T>(a, s) : launch_rx_one<GE, CU, EACH, T>(a, s);
+    return sumtype == BOTH ? launch_das_one<GE, CU, BOTH, T, false>(a, s)
+                           : launch_das_one<GE, CU, EACH, T, false>(a, s);
+}
+
 cudaError_t launch_das_synth_slow(const DasArgs &a, int sumtype, int dtype, cudaStream_t s) {
-    constexpr int CU = PYCBF_GB_INTERP_CUBIC;
-    const bool both = sumtype == PYCBF_GB_SUM_TX_AND_RX;
     switch (dtype) {
-        case PYCBF_GB_F32:
-            return both ? launch_das_one<GEOM_SYNTH_SLOW, CU, PYCBF_GB_SUM_TX_AND_RX, float, false>(a, s)
-                        : launch_das_one<GEOM_SYNTH_SLOW, CU, PYCBF_GB_SUM_TX_ONLY, float, false>(a, s);
-        case PYCBF_GB_F16:
-            return both ? launch_das_one<GEOM_SYNTH_SLOW, CU, PYCBF_GB_SUM_TX_AND_RX, __half, false>(a, s)
-                        : launch_das_one<GEOM_SYNTH_SLOW, CU, PYCBF_GB_SUM_TX_ONLY, __half, false>(a, s);
-        case PYCBF_GB_BF16:
-            return both ? launch_das_one<GEOM_SYNTH_SLOW, CU, PYCBF_GB_SUM_TX_AND_RX, __nv_bfloat16, false>(a, s)
-                        : launch_das_one<GEOM_SYNTH_SLOW, CU, PYCBF_GB_SUM_TX_ONLY, __nv_bfloat16, false>(a, s);
+        case PYCBF_GB_F32: return launch_synth_slow_t<float>(a, sumtype, s);
+        case PYCBF_GB_F16: return launch_synth_slow_t<__half>(a, sumtype, s);
+        case PYCBF_GB_BF16: return launch_synth_slow_t<__nv_bfloat16>(a, sumtype, s);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -217,10 +217,6 @@ struct DasArgs {
     // exercised without a fault)
     long long wait_cycles;
     int stall_test;
-    // staged delay gradients: the upstream gradient (kernel pixel order) and
-    // dL/dtautx (ntx, np), dL/dtaurx (nrx, np), either may be null
-    const float *gk;
-    float *gtx, *grx;
 };
 
 // gather kinds of the polynomial-record interpolators (records from poly.cu)
@@ -242,9 +238,6 @@ long long tabbed_plan_words(long long np, int ntx, int nrx);
 cudaError_t launch_tabbed_plan(const DasArgs &a, int interp, int dtype, int *plan, cudaStream_t s);
 cudaError_t launch_das_staged(const DasArgs &a, int interp, int sumtype, int dtype, const int *plan,
                               int *status, cudaStream_t s);
-// the delay gradients on the staging plan (cubic, float32 records, one frame)
-cudaError_t launch_das_staged_adj(const DasArgs &a, int sumtype, int dtype, const int *plan,
-                                  cudaStream_t s);
 
 // cubic upsampling for nearest with usf > 1: out (nch, ntu) float32 from the
 // spline records in a.data (time axis of the original channel data in a)
@@ -309,7 +302,6 @@ struct AdjArgs {
     int *order;           // workspace: the tiles by depth
     float *tau_tx, *tau_rx;  // workspace: Synthetic delays (ntx, np), (nrx, np), or null
     const float *gk;      // set by launch_adjoint: gk_buf, or grad_out without pixel_index
-    const int *plan;      // Tabbed: the forward's staging plan when its staged path applies, or NULL
 };
 // parts of the tiles whose channel adjoints are summed separately
 int adjoint_parts(long long nch, long long np);

@@ -16,7 +16,6 @@ cudaError_t launch_plan_bf16(const DasArgs &, int, int *, cudaStream_t);
 cudaError_t launch_staged_f32(const DasArgs &, int, int, const int *, int *, cudaStream_t);
 cudaError_t launch_staged_f16(const DasArgs &, int, int, const int *, int *, cudaStream_t);
 cudaError_t launch_staged_bf16(const DasArgs &, int, int, const int *, int *, cudaStream_t);
-cudaError_t launch_staged_adj_f32(const DasArgs &, int, const int *, cudaStream_t);
 cudaError_t launch_das_frames_f32(const DasArgs &, int, int, int, cudaStream_t);
 cudaError_t launch_das_frames_f16(const DasArgs &, int, int, int, cudaStream_t);
 cudaError_t launch_das_frames_bf16(const DasArgs &, int, int, int, cudaStream_t);
@@ -65,8 +64,9 @@ cudaError_t launch_rx_bf16(const DasArgs &, int, int, int, cudaStream_t);
 
 // Sums over transmits of the kinds with packed decisions, on time axes that allow them
 // (fast_axis), at every size: das_rx_kernel is the faster one throughout (its figures are
-// beside it).  On other axes every tap takes the exact decisions, which
-// das_staged_kernel and das_kernel make.
+// beside it).  On other axes every tap takes the exact decisions, which das_kernel makes
+// and, with a staging plan, das_staged_kernel (nearest, 11 transmits, 128 receives, 256 x
+// 512 pixels from 1 s at 55 ns: 142 us staged, 877 not).
 bool das_rx_ok(const DasArgs &a, int interp, int sumtype) {
     if (interp != PYCBF_GB_INTERP_CUBIC && interp != PYCBF_GB_INTERP_LINEAR &&
         interp != PYCBF_GB_INTERP_NEAREST)
@@ -119,12 +119,6 @@ cudaError_t launch_synth_rx_mask(const DasArgs &a, unsigned char *mask, cudaStre
     const long long bx = (a.np + 255) / 256;
     synth_rx_mask_kernel<<<(unsigned)bx, 256, 0, s>>>(a, mask);
     return cudaGetLastError();
-}
-
-cudaError_t launch_das_staged_adj(const DasArgs &a, int sumtype, int dtype, const int *plan,
-                                  cudaStream_t s) {
-    if (dtype != PYCBF_GB_F32) return cudaErrorInvalidValue;  // float32 records (F32, I16 data)
-    return launch_staged_adj_f32(a, sumtype, plan, s);
 }
 
 }  // namespace pgb

@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(32 * kRxWarps, frames_ctas(GEOM, FG))
     if (!W)
         for (int k = 0; k < 3; ++k) if (k < a.ndim) pnt[k] = __ldg(a.geo.pnts + i * a.ndim + k);
     float amax = 0.f, amin = inf, atop = -inf;
-    rx_column<GEOM, kRxWarps>(a, pnt, i, w, col, amax, amin, atop);
+    rx_column<GEOM, kRxWarps>(a, pnt, 0.f, i, w, col, amax, amin, atop);
     if (W) {
         s_w[0][w][lane] = amax;
         s_w[1][w][lane] = amin;

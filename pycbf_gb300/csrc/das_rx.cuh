@@ -69,8 +69,8 @@ __device__ __forceinline__ void rx_fetch_run(const DasArgs &a, float *t, int r0,
 // Warp w's part of the transmit delays of pixel i, in pairs padded with infinite delays
 // (never count) to whole groups, and of the range of its weights.
 template <int GEOM, int WARPS>
-__device__ __forceinline__ void rx_column(const DasArgs &a, const float *pnt, long long i, int w,
-                                          float2 *col, float &amax, float &amin, float &atop) {
+__device__ __forceinline__ void rx_column(const DasArgs &a, const float *pnt, float slow,
+                                          long long i, int w, float2 *col, float &amax, float &amin, float &atop) {
     const int npair = (a.ntx + 3) / 4 * 2;
     for (int p = w; p < npair; p += WARPS) {
         float tau[2] = {__int_as_float(0x7f800000), __int_as_float(0x7f800000)};
@@ -83,8 +83,12 @@ __device__ __forceinline__ void rx_column(const DasArgs &a, const float *pnt, lo
                 const float v = __ldg(a.apodtx + (long long)k * a.np + i);
                 amax = fmaxf(amax, fabsf(v));
                 weight_range(v, amin, atop);
-            } else {
+            } else if (GEOM == GEOM_SYNTH) {
                 tau[h] = synth_tx_delay(a, k, pnt);
+            } else {
+                float D, t0add;
+                const bool ok = synth_tx_path(a, k, pnt, D, t0add);
+                tau[h] = slow_delay(ok, D, slow, t0add);
             }
         }
         col[p * 32] = make_float2(tau[0], tau[1]);
@@ -121,10 +125,11 @@ __global__ void __launch_bounds__(32 * kRxWarps, GEOM == GEOM_TABBED ? 4 : 3)
     if (W) fetch_run(0, 0);
 
     float pnt[3] = {0.f, 0.f, 0.f};
+    const float slow = GEOM == GEOM_SYNTH_SLOW ? __ldg(a.slow + i) : 0.f;
     if (!W)
         for (int k = 0; k < 3; ++k) if (k < a.ndim) pnt[k] = __ldg(a.geo.pnts + i * a.ndim + k);
     float amax = 0.f, amin = inf, atop = -inf;
-    rx_column<GEOM, kRxWarps>(a, pnt, i, w, col, amax, amin, atop);
+    rx_column<GEOM, kRxWarps>(a, pnt, slow, i, w, col, amax, amin, atop);
     if (W) {
         s_w[0][w][lane] = amax;
         s_w[1][w][lane] = amin;
@@ -161,8 +166,13 @@ __global__ void __launch_bounds__(32 * kRxWarps, GEOM == GEOM_TABBED ? 4 : 3)
                 trx = tab[e * 32];
                 arx = tab[(kRun + e) * 32];
                 live = __fmul_rn(amax, fabsf(arx)) >= a.thresh;
-            } else {
+            } else if (GEOM == GEOM_SYNTH) {
                 trx = synth_rx_delay_warp(a, r, pnt);
+                live = trx != inf;
+            } else {
+                float D;
+                const bool ok = synth_rx_path(a, r, pnt, D);
+                trx = slow_delay(ok, D, slow, 0.f);
                 live = trx != inf;
             }
             if (!__any_sync(kFull, live)) {

@@ -488,62 +488,6 @@ __device__ __forceinline__ typename CubicAcc<T>::type staged_taps(
     return acc;
 }
 
-// Delay gradients of N <= kTapGroup cubic taps of receive (trx, arx), the
-// adjoint of the delay-and-sum with respect to tautx and taurx: for every tap
-// the forward counts (the same decisions: range, threshold, knot), d = apod *
-// (gp * dS/dx) with dS/dx = (p1 + 2 p2 b + 3 p3 b^2) / dt from the interval's
-// polynomial record; d is added into gt[k] (this pixel's dL/dtautx of the
-// group's transmit k, over receives in order) and into the returned gr
-// (dL/dtaurx, over transmits in order).  Records come from the stage
-// (STAGED; sb as in staged_taps) or from global memory
-// (grec: the record row of the group's first transmit, chs between
-// transmits).
-template <int N, bool STAGED>
-__device__ __forceinline__ float adj_cubic_group(const DasArgs &a, const TapConst &c,
-                                                 const float2 *tt2, const float2 *at2, float trx, float arx, float gp,
-                                                 const unsigned *sb, unsigned last,
-                                                 const float4 *grec, long long chs, float *gt,
-                                                 float gr) {
-    constexpr int NP = (N + 1) / 2;
-    float2 x2[NP], fj2[NP];
-    unsigned r[2 * NP];
-    knot_pairs<NP>(a, c, tt2, trx, x2, fj2, r);
-    float4 pv[N];
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-        if (STAGED) {
-            pv[k] = lds_record(r[k] * (unsigned)sizeof(float4) + sb[k], last,
-                               static_cast<float4 *>(nullptr));
-        } else {
-            const int j = min(max((int)(r[k] - kKnotBits), 0), a.nt - 1);
-            pv[k] = __ldg(grec + k * chs + j);
-        }
-    }
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        const float2 w2 = mul2_rn(at2[p], make_float2(arx, arx));
-        const float2 b2 = knot_frac2(c, x2[p], fj2[p]);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int k = 2 * p + h;
-            if (k < N) {
-                const float b = h ? b2.y : b2.x;
-                const float x = h ? x2[p].y : x2[p].x;
-                const float apod = h ? w2.y : w2.x;
-                const float slope =
-                    fmaf(fmaf(3.f * pv[k].w, b, 2.f * pv[k].z), b, pv[k].y) * a.inv_dt;
-                const float d = gp * slope;
-                const bool ok = (x >= c.t0) && (x <= c.xmax) && (fabsf(apod) >= c.thresh);
-                if (ok) {
-                    gt[k] = fmaf(apod, d, gt[k]);
-                    gr = fmaf(apod, d, gr);
-                }
-            }
-        }
-    }
-    return gr;
-}
-
 // Persistent: a grid sized to the GPU takes work items from the plan's queue
 // head (plan[1], zeroed before the launch) in the plan's order, largest first,
 // so the slowest items start first and the last wave is short: (tile, block
@@ -559,14 +503,8 @@ __device__ __forceinline__ float adj_cubic_group(const DasArgs &a, const TapCons
 // it - 1 with receive it + 3 once every warp has left that slot.  Each warp
 // keeps the plan words of the next receive it will stage in registers,
 // loaded one turn ahead.
-//
-// ADJ: the delay gradients instead of the image (cubic, float32 records, one
-// frame): whole tiles as items, the upstream gradient a.gk (kernel pixel
-// order; per pixel for TX_AND_RX, per receive and pixel for TX_ONLY), dL/dtaurx
-// written per live receive into a.grx and dL/dtautx per item into a.gtx (the
-// rows of receives a tile cannot use stay as the caller zeroed them).
-template <int KIND, int SUM, typename T, bool ADJ = false>
-__global__ void __launch_bounds__(kBlock, ADJ ? 4 : 5) das_staged_kernel(const __grid_constant__ DasArgs a,
+template <int KIND, int SUM, typename T>
+__global__ void __launch_bounds__(kBlock, 5) das_staged_kernel(const __grid_constant__ DasArgs a,
                                                               int *__restrict__ plan) {
     using E = typename StagedElem<KIND, T>::E;
     constexpr bool kCubic = KIND == PYCBF_GB_INTERP_CUBIC;
@@ -591,7 +529,7 @@ __global__ void __launch_bounds__(kBlock, ADJ ? 4 : 5) das_staged_kernel(const _
     const long long tiles = L.tiles;
     const long long tile_words = L.tile_words;
     constexpr bool kBlockSum = SUM == PYCBF_GB_SUM_TX_AND_RX || SUM == PYCBF_GB_SUM_TX_ONLY;
-    const bool by_block = !ADJ && kBlockSum && a.nframes == 1;
+    const bool by_block = kBlockSum && a.nframes == 1;
     const long long nitems = by_block ? (long long)__ldg(plan + 2) : tiles * a.nframes;
     const int *order = plan + L.order;
     const int4 *bitems = reinterpret_cast<const int4 *>(plan + L.items);
@@ -734,32 +672,25 @@ __global__ void __launch_bounds__(kBlock, ADJ ? 4 : 5) das_staged_kernel(const _
         float bacc = 0.f;  // the current receive block's sequential sum (TX_AND_RX)
         int cur_block = -1;
         bool failed = false;
-        // ADJ: this pixel's dL/dtautx per transmit, and its upstream gradient
-        float gt[kTxReg];
-#pragma unroll
-        for (int k = 0; k < kTxReg; ++k) gt[k] = 0.f;
-        const float gpix = (ADJ && SUM == PYCBF_GB_SUM_TX_AND_RX && valid) ? __ldg(a.gk + i) : 0.f;
         // receive-side values, fetched two receives ahead
         const float *trp = a.taurx + i, *arp = a.apodrx + i;
-        auto rx_load = [&](int it, float &trx, float &arx, float &gpr) {
+        auto rx_load = [&](int it, float &trx, float &arx) {
             const long long ro = (long long)(s_rx[it] & ~kCodeFlags) * np;
             trx = valid ? __ldg(trp + ro) : 0.f;
             arx = valid ? __ldg(arp + ro) : 0.f;
-            gpr = (ADJ && SUM == PYCBF_GB_SUM_TX_ONLY && valid) ? __ldg(a.gk + ro + i) : gpix;
         };
-        float trx1 = 0.f, arx1 = 0.f, trx2 = 0.f, arx2 = 0.f, gp1 = 0.f, gp2 = 0.f;
-        if (nlive > 0) rx_load(0, trx1, arx1, gp1);
-        if (nlive > 1) rx_load(1, trx2, arx2, gp2);
+        float trx1 = 0.f, arx1 = 0.f, trx2 = 0.f, arx2 = 0.f;
+        if (nlive > 0) rx_load(0, trx1, arx1);
+        if (nlive > 1) rx_load(1, trx2, arx2);
 
         for (int it = 0; it < nlive; ++it) {
             const int gi = g0 + it;
             const int slot = gi & (kStages - 1);
             const int r = s_rx[it] & ~kCodeFlags;
-            const float trx = trx1, arx = arx1, gp = gp1;
+            const float trx = trx1, arx = arx1;
             trx1 = trx2;
             arx1 = arx2;
-            gp1 = gp2;
-            if (it + 2 < nlive) rx_load(it + 2, trx2, arx2, gp2);
+            if (it + 2 < nlive) rx_load(it + 2, trx2, arx2);
             if (!mbar_try_wait(&full[slot], (unsigned)(gi >> 2) & 1u)) {
                 if (*(volatile int *)&s_failed ||
                     !mbar_wait_bounded(&full[slot], (unsigned)(gi >> 2) & 1u, wait_lim)) {
@@ -776,47 +707,7 @@ __global__ void __launch_bounds__(kBlock, ADJ ? 4 : 5) das_staged_kernel(const _
             }
             const bool live = valid && (__fmul_rn(amax, fabsf(arx)) >= a.thresh);
             float accr = 0.f;
-            if constexpr (ADJ) {
-                // delay gradients of this receive's taps (dL/dtaurx of a
-                // non-live pixel is 0: every tap of it fails the threshold)
-                float gr = 0.f;
-                if (live) {
-                    const long long chs = (long long)nrx * a.nt;
-                    const float4 *grow = static_cast<const float4 *>(a.data) + (frame_ch + r) * a.nt;
-                    const bool stg = sstaged[slot] != 0 && a.fast_axis;
-                    unsigned sb[kTxReg];
-#pragma unroll
-                    for (int g = 0; g < kTxReg; g += 4) {
-                        const uint4 b = *reinterpret_cast<const uint4 *>(&sbase[slot][g]);
-                        sb[g] = b.x;
-                        sb[g + 1] = b.y;
-                        sb[g + 2] = b.z;
-                        sb[g + 3] = b.w;
-                    }
-#pragma unroll
-                    for (int g = 0; g < kTxReg; g += kTapGroup) {
-                        if (g < ntx) {
-                            const int rem = ntx - g;
-#define PGB_AGROUP(n, st)                                                                         \
-    adj_cubic_group<n, st>(a, tc, tt2 + g / 2, at2 + g / 2, trx, arx, gp, sb + g, last_rec,           \
-                           grow + (long long)g * chs, chs, gt + g, gr)
-                            if (stg) {
-                                if (rem >= 4) gr = PGB_AGROUP(4, true);
-                                else if (rem == 3) gr = PGB_AGROUP(3, true);
-                                else if (rem == 2) gr = PGB_AGROUP(2, true);
-                                else gr = PGB_AGROUP(1, true);
-                            } else {
-                                if (rem >= 4) gr = PGB_AGROUP(4, false);
-                                else if (rem == 3) gr = PGB_AGROUP(3, false);
-                                else if (rem == 2) gr = PGB_AGROUP(2, false);
-                                else gr = PGB_AGROUP(1, false);
-                            }
-#undef PGB_AGROUP
-                        }
-                    }
-                }
-                if (valid && a.grx) a.grx[(long long)r * np + i] = gr;
-            } else if (live) {
+            if (live) {
                 const long long ch_first = (frame_ch + r) * a.nt;
                 const long long chs = (long long)nrx * a.nt;
                 unsigned sb[kTxReg];
@@ -880,7 +771,7 @@ __global__ void __launch_bounds__(kBlock, ADJ ? 4 : 5) das_staged_kernel(const _
                 }
             }
             if (SUM == PYCBF_GB_SUM_TX_AND_RX) bacc += accr;
-            if (!ADJ && SUM == PYCBF_GB_SUM_TX_ONLY && valid)
+            if (SUM == PYCBF_GB_SUM_TX_ONLY && valid)
                 a.out[((long long)f * nrx + r) * np + op] = accr;
             if (SUM == PYCBF_GB_SUM_DMAS_SSR || SUM == PYCBF_GB_SUM_DMAS_POWER) {
                 const float sv = (SUM == PYCBF_GB_SUM_DMAS_SSR) ? copysignf(sqrtf(fabsf(accr)), accr) : accr;
@@ -904,17 +795,6 @@ __global__ void __launch_bounds__(kBlock, ADJ ? 4 : 5) das_staged_kernel(const _
             }
         }
         __syncthreads();
-        if constexpr (ADJ) {
-            if (valid && a.gtx) {
-                const float nan = __int_as_float(0x7fc00000);
-#pragma unroll
-                for (int k = 0; k < kTxReg; ++k)
-                    if (k < ntx) a.gtx[(long long)k * np + i] = s_failed ? nan : gt[k];
-            }
-            if (s_failed) break;
-            g0 += nlive;
-            continue;
-        }
         if (s_failed) {
             if (valid) {
                 const float nan = __int_as_float(0x7fc00000);
@@ -1087,36 +967,6 @@ cudaError_t launch_staged_one(const DasArgs &a, const int *plan, int *status, cu
         if (err != cudaSuccess) return err;
     }
     kern<<<(unsigned)grid, kBlock, smem, s>>>(a, const_cast<int *>(plan));
-    return cudaGetLastError();
-}
-
-// The delay gradients on the staging plan (ADJ mode; cubic, float32 records,
-// one frame, sumtype TX_AND_RX or TX_ONLY).  dL/dtaurx rows of receives a tile
-// cannot use are zeroed first.
-template <typename T>
-cudaError_t launch_staged_adj(const DasArgs &a, int sum, const int *plan, cudaStream_t s) {
-    if (!CoefRec<T>::kPoly || a.nframes != 1) return cudaErrorInvalidValue;
-    auto kern = sum == PYCBF_GB_SUM_TX_AND_RX
-                    ? das_staged_kernel<PYCBF_GB_INTERP_CUBIC, PYCBF_GB_SUM_TX_AND_RX, T, true>
-                    : das_staged_kernel<PYCBF_GB_INTERP_CUBIC, PYCBF_GB_SUM_TX_ONLY, T, true>;
-    const int smem = (int)staged_smem_bytes(a.nrx);
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (err != cudaSuccess) return err;
-    int dev = 0, nsm = 0, per_sm = 0;
-    if ((err = cudaGetDevice(&dev)) != cudaSuccess) return err;
-    if ((err = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
-        return err;
-    if ((err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, smem)) !=
-        cudaSuccess)
-        return err;
-    const PlanLayout L = plan_layout(a.np, a.ntx, a.nrx);
-    const long long grid = std::min<long long>(L.tiles, (long long)std::max(1, per_sm) * nsm);
-    int *pl = const_cast<int *>(plan);
-    if ((err = cudaMemsetAsync(pl + 1, 0, sizeof(int), s)) != cudaSuccess) return err;
-    if (a.grx && (err = cudaMemsetAsync(a.grx, 0, sizeof(float) * (size_t)a.nrx * a.np, s)) !=
-                     cudaSuccess)
-        return err;
-    kern<<<(unsigned)grid, kBlock, smem, s>>>(a, pl);
     return cudaGetLastError();
 }
 
