@@ -86,6 +86,16 @@ def _out_shape(rf4, np_, sumtype):
     return (nf, np_) if sumtype == _lib.SUMTYPE["tx_and_rx"] else (nf, nrx, np_)
 
 
+def _workspace(L, info, np_: int, synthetic: bool, device):
+    """The adjoint's workspace, with room for the tiles' delay ranges and the Synthetic
+    delay tables."""
+    nel = info.ntx + info.nrx
+    nws = L.pycbf_gb_adjoint_workspace_bytes(ct.byref(info), np_) + 8 * (nel + 1) * ((np_ + 127) // 128) + 64
+    if synthetic:
+        nws += 4 * nel * np_
+    return torch.empty(nws, dtype=torch.uint8, device=device), nws
+
+
 class _TabbedDAS(torch.autograd.Function):
     @staticmethod
     def forward(ctx, rf4, tautx, taurx, apodtx, apodrx, pixel_index, spec, plan=None):
@@ -124,8 +134,7 @@ class _TabbedDAS(torch.autograd.Function):
         g_trx = torch.empty_like(taurx) if need_trx else None
         ws, nws = None, 0
         if need_rf or ctx.pixel_index is not None:
-            nws = L.pycbf_gb_adjoint_workspace_bytes(ct.byref(info), np_)
-            ws = torch.empty(nws, dtype=torch.uint8, device=dev)
+            ws, nws = _workspace(L, info, np_, False, dev)
         if need_rf or need_ttx or need_trx:
             st = L.pycbf_gb_das_tabbed_adjoint_planned(
                 ct.byref(info), _ptr(coef), _ptr(tautx), _ptr(apodtx), _ptr(taurx), _ptr(apodrx),
@@ -174,8 +183,7 @@ class _SyntheticDAS(torch.autograd.Function):
         g_s = torch.empty_like(slowness) if need_s else None
         ws, nws = None, 0
         if need_rf or ctx.pixel_index is not None:
-            nws = L.pycbf_gb_adjoint_workspace_bytes(ct.byref(info), slowness.shape[0])
-            ws = torch.empty(nws, dtype=torch.uint8, device=dev)
+            ws, nws = _workspace(L, info, slowness.shape[0], True, dev)
         if need_rf or need_s:
             st = L.pycbf_gb_das_synthetic_adjoint(
                 ct.byref(info), _ptr(coef), ct.byref(geom_struct), _ptr(slowness),

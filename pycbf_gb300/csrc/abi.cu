@@ -591,8 +591,7 @@ int run_adjoint(const pycbf_gb_rfinfo *rf, AdjArgs &g, void *workspace, size_t w
         const size_t need = pycbf_gb_adjoint_workspace_bytes(rf, g.d.np);
         if (!workspace || workspace_bytes < need || reinterpret_cast<uintptr_t>(workspace) % 16)
             return PYCBF_GB_EWORKSPACE;
-        adjoint_layout(rf->nframes, rf->ntx, rf->nrx, g.d.np, rf->nt, g.geom != GEOM_TABBED,
-                       static_cast<char *>(workspace), &g);
+        adjoint_layout(static_cast<char *>(workspace), workspace_bytes, &g);
     }
     return cuda_status(launch_adjoint(g, rf->dtype, s));
 }
@@ -623,7 +622,7 @@ int pycbf_gb_das_synthetic_slowness(const pycbf_gb_rfinfo *rf, const void *coef,
 
 size_t pycbf_gb_adjoint_workspace_bytes(const pycbf_gb_rfinfo *rf, long long np) {
     if (!rf || np <= 0 || rf->ntx <= 0 || rf->nrx <= 0 || rf->nt <= 0 || rf->nframes <= 0) return 0;
-    return adjoint_layout(rf->nframes, rf->ntx, rf->nrx, np, rf->nt, rf->ndim != 0, nullptr, nullptr);
+    return adjoint_workspace_bytes(rf->nframes, rf->ntx, rf->nrx, np, rf->nt);
 }
 
 int pycbf_gb_das_tabbed_adjoint(const pycbf_gb_rfinfo *rf, const void *coef,

@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kBlock) adj_range_kernel(const __grid_constant
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long tile = blockIdx.x, tiles = gridDim.x;
     const long long i0 = tile * kBlock + lane;
-    float2 *ranges = g.ranges + tile * (a.ntx + a.nrx);
+    float2 *ranges = g.ranges ? g.ranges + tile * (a.ntx + a.nrx) : nullptr;
     float pnt[M][3], slow[M], amax[M];
 #pragma unroll
     for (int m = 0; m < M; ++m) {
@@ -374,8 +374,8 @@ __global__ void __launch_bounds__(kBlock) adj_range_kernel(const __grid_constant
         hi = from_key(__reduce_max_sync(kFull, to_key(hi)));
         any = __any_sync(kFull, any);
         if (lane == 0 && !(tx && blockIdx.y > 0)) {
-            ranges[e] = make_float2(lo, hi);
-            if (tx && e == a.ntx / 2) g.depth[tile] = lo;
+            if (ranges) ranges[e] = make_float2(lo, hi);
+            if (ranges && tx && e == a.ntx / 2) g.depth[tile] = lo;
             if (!tx) g.live[(long long)r * tiles + tile] = any ? 1 : 0;
         }
     };
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(128, 5) adj_scatter_kernel(const __grid_consta
     // samples that those tiles' taps of this channel can touch: intervals [w0, w1)
     float4 rng = make_float4(__int_as_float(0x7f800000), -__int_as_float(0x7f800000),
                              __int_as_float(0x7f800000), -__int_as_float(0x7f800000));
-    for (int k = lane; k < nlist; k += 32) {
+    for (int k = lane; k < (g.ranges ? nlist : 0); k += 32) {
         const float2 u = __ldg(g.ranges + (long long)list[k] * nel + t);
         const float2 v = __ldg(g.ranges + (long long)list[k] * nel + ntx + r);
         rng = make_float4(fminf(rng.x, u.x), fmaxf(rng.y, u.y), fminf(rng.z, v.x), fmaxf(rng.w, v.y));
@@ -480,13 +480,16 @@ __global__ void __launch_bounds__(128, 5) adj_scatter_kernel(const __grid_consta
                                from_key(__reduce_min_sync(kFull, to_key(rng.z))));
     const float hi = __fadd_rn(from_key(__reduce_max_sync(kFull, to_key(rng.y))),
                                from_key(__reduce_max_sync(kFull, to_key(rng.w))));
-    int w0 = 0, w1 = 0;
-    if (lo <= hi && hi >= a.t0 && lo <= a.xmax) {
+    int w0 = 0, w1 = g.ranges ? 0 : nt;  // without the ranges: every interval
+    if (g.ranges && lo <= hi && hi >= a.t0 && lo <= a.xmax) {
         w0 = lo <= a.t0 ? 0 : (int)floorf(__fdiv_rn(__fsub_rn(lo, a.t0), a.dt));
         w1 = hi >= a.xmax ? nt : min(nt, (int)floorf(__fdiv_rn(__fsub_rn(hi, a.t0), a.dt)) + 1);
         w0 = min(w0, nt - 1);
     }
-    if (lane == 0) g.windows[(size_t)q * nch + ch] = make_int2(w0, w1);  // samples w0 .. w1 of the rows
+    if (lane == 0) {  // samples w0 .. w1 of the rows: kept in the place past their last sample
+        py[nt] = __int_as_float(w0);
+        pz[nt] = __int_as_float(w1);
+    }
 
     const float *ptx = (GEOM == GEOM_TABBED ? a.tautx : g.tau_tx) + (long long)t * np;
     const float *prx = (GEOM == GEOM_TABBED ? a.taurx : g.tau_rx) + (long long)r * np;
@@ -585,7 +588,7 @@ __global__ void __launch_bounds__(128, 5) adj_scatter_kernel(const __grid_consta
             const int m = m0 + lane;
             const float4 here = m < n ? row[m] : make_float4(0.f, 0.f, 0.f, 0.f);
             const float4 before = m == 0 ? carry : (m <= n ? row[m - 1] : here);
-            if (m < n || (last && m == n)) {
+            if (s0 + m < nt && (m < n || (last && m == n))) {
                 const float c = knot_step(a, s0 + m), c2 = c * c;
                 py[s0 + m] = fmaf(c, here.x, -here.y) + before.y;
                 pz[s0 + m] = fmaf(c2 * c - c, here.x,
@@ -643,9 +646,8 @@ __device__ __forceinline__ void prefilter_adjoint_warp(float *zv, float *u, int 
 // adjoint of the prefilter, one warp per channel
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-adj_finalize_kernel(const float *__restrict__ partial, const int2 *__restrict__ windows, int nparts,
-                    long long nch, int nt, int Lp, float *__restrict__ grad_rf,
-                    const __grid_constant__ SplineTable tab) {
+adj_finalize_kernel(const float *__restrict__ partial, int nparts, long long nch, int nt, int Lp,
+                    float *__restrict__ grad_rf, const __grid_constant__ SplineTable tab) {
     extern __shared__ float smem[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     const long long ch = (long long)blockIdx.x * wpb + w;
@@ -658,10 +660,15 @@ adj_finalize_kernel(const float *__restrict__ partial, const int2 *__restrict__ 
     // the parts' samples into dst, parts in order, each from its window only
     auto sum_parts = [&](float *dst, int off) {
         for (int n = lane; n < nt; n += 32) dst[n] = 0.f;
+        int2 wins = make_int2(0, 0);  // of part q0 + lane
         for (int q = 0; q < nparts; ++q) {
-            const int2 win = __ldg(windows + q * nch + ch);
-            if (win.x >= win.y) continue;
+            if (q % 32 == 0 && q + lane < nparts) {
+                const float *row = p0 + (q + lane) * pstride;
+                wins = make_int2(__float_as_int(row[nt]), __float_as_int(row[Lp + nt]));
+            }
+            const int2 win = make_int2(__shfl_sync(kFull, wins.x, q % 32), __shfl_sync(kFull, wins.y, q % 32));
             const float *src = p0 + q * pstride + off;
+            if (win.x >= win.y) continue;
 #pragma unroll 4
             for (int n = win.x + lane; n <= min(win.y, nt - 1); n += 32) dst[n] += src[n];
         }
@@ -711,14 +718,14 @@ cudaError_t launch_scatter_one(const AdjArgs &g0, cudaStream_t s) {
     const int Lp = (a.nt + 1 + 3) & ~3;
     // Synthetic delays once into tables where they fit (the scatter would take a root
     // and a quotient per tap again)
-    const bool tables = GEOM == GEOM_TABBED || g.tau_tx;
+    const bool tables = GEOM == GEOM_TABBED || (g.tau_tx && g.tau_rx);
     constexpr bool kSynth = GEOM != GEOM_TABBED;
     const dim3 rgrid((unsigned)tiles, 4);
     if (tables) adj_range_kernel<GEOM, kSynth><<<rgrid, kBlock, 0, s>>>(g);
     else adj_range_kernel<GEOM, false><<<rgrid, kBlock, 0, s>>>(g);
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
-    if (tiles <= kRankTiles) {
+    if (tiles <= kRankTiles && g.ranges) {
         adj_rank_kernel<<<(unsigned)((tiles + 7) / 8), 256, 0, s>>>(g.depth, (int)tiles, g.order);
         if ((err = cudaGetLastError()) != cudaSuccess) return err;
     } else {
@@ -754,7 +761,7 @@ cudaError_t launch_scatter_one(const AdjArgs &g0, cudaStream_t s) {
     if (err != cudaSuccess) return err;
     const long long blocks = (nch + wpb - 1) / wpb;
     adj_finalize_kernel<<<(unsigned)blocks, 32 * wpb, fsmem, s>>>(
-        g.partial, g.windows, nparts, nch, a.nt, Lp, g.grad_rf, tab);
+        g.partial, nparts, nch, a.nt, Lp, g.grad_rf, tab);
     return cudaGetLastError();
 }
 
@@ -802,57 +809,70 @@ int adjoint_parts(long long nch, long long np) {
     return (int)std::max<long long>(p, ((np + kBlock - 1) / kBlock + 16383) / 16384);
 }
 
-size_t adjoint_grad_bytes(long long nframes, long long nrx, long long np) {
-    return ((size_t)nframes * (size_t)nrx * (size_t)np * sizeof(float) + 255) & ~(size_t)255;
+static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
+static size_t adjoint_grad_bytes(long long nframes, long long nrx, long long np) {
+    return up256((size_t)nframes * nrx * np * sizeof(float));
 }
-
-size_t adjoint_partial_bytes(long long nframes, long long ntx, long long nrx, long long np,
-                             int nt) {
+static size_t adjoint_partial_bytes(long long nframes, long long ntx, long long nrx, long long np,
+                                    int nt) {
     const long long nch = nframes * ntx * nrx;
     const size_t Lp = (size_t)((nt + 1 + 3) & ~3);
     return (size_t)adjoint_parts(nch, np) * (size_t)nch * 2 * Lp * sizeof(float);
 }
 
-// [gathered gradient][partial sums][live][tile ranges][depths][windows][order]
-// [Synthetic delay tables], each 256-byte aligned
+// [gathered gradient][partial sums][live]
+size_t adjoint_workspace_bytes(long long nframes, long long ntx, long long nrx, long long np, int nt) {
+    const size_t tiles = (size_t)((np + kBlock - 1) / kBlock);
+    return adjoint_grad_bytes(nframes, nrx, np) + adjoint_partial_bytes(nframes, ntx, nrx, np, nt) +
+           up256((size_t)nrx * tiles);
+}
+
+// The rest takes space that is free: above the gathered gradient (one row a frame of the
+// sum over receives; none without pixel_index), above the workspace's size, and, for the
+// ranges, depths and order, which the last kernel no longer reads, in grad_rf before it is
+// written.  Without room for them the scatter walks every tile for every interval (1717
+// against 780 us for 11 x 128 x 2048 samples and 256 x 512 pixels; only channel data much
+// smaller than the pixels' tables comes to that), and the Synthetic scatter computes its
+// delays per tap (slowness gradients of the same size 1.71 against 1.13 ms).
 constexpr size_t kAdjTableMax = (size_t)1 << 30;  // above: the scatter recomputes the delays
 
-size_t adjoint_layout(long long nframes, long long ntx, long long nrx, long long np, int nt,
-                      bool synthetic, char *ws, AdjArgs *g) {
-    const size_t tiles = (size_t)((np + kBlock - 1) / kBlock), nel = (size_t)(ntx + nrx);
-    const long long nch = nframes * ntx * nrx;
-    const size_t parts = (size_t)adjoint_parts(nch, np);
-    size_t at = 0;
-    auto take = [&](size_t bytes) {
-        char *p = ws ? ws + at : nullptr;
-        at += (bytes + 255) & ~(size_t)255;
-        return p;
+void adjoint_layout(char *ws, size_t bytes, AdjArgs *g) {
+    const DasArgs &a = g->d;
+    const size_t tiles = (size_t)((a.np + kBlock - 1) / kBlock), nel = (size_t)(a.ntx + a.nrx);
+    const size_t np = (size_t)a.np;
+    char *const partial = ws + adjoint_grad_bytes(a.nframes, a.nrx, np);
+    g->gk_buf = reinterpret_cast<float *>(ws);
+    g->partial = reinterpret_cast<float *>(partial);
+    g->live = reinterpret_cast<unsigned char *>(
+        partial + adjoint_partial_bytes(a.nframes, a.ntx, a.nrx, np, a.nt));
+    const size_t need = adjoint_workspace_bytes(a.nframes, a.ntx, a.nrx, np, a.nt);
+    const int rows = a.nframes * (g->sumtype == PYCBF_GB_SUM_TX_AND_RX ? 1 : a.nrx);
+    struct Room { char *at, *end; } room[3] = {
+        {ws + (a.pixel_index ? up256(rows * np * sizeof(float)) : 0), partial},
+        {ws + need, ws + bytes},
+        {reinterpret_cast<char *>(g->grad_rf),
+         reinterpret_cast<char *>(g->grad_rf) + (size_t)a.nframes * a.ntx * a.nrx * a.nt * sizeof(float)}};
+    auto take = [&](size_t n, int rooms) -> char * {
+        for (int k = 0; k < rooms; ++k) {
+            char *p = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(room[k].at) + 15) & ~(uintptr_t)15);
+            if (p && p <= room[k].end && n <= (size_t)(room[k].end - p)) {
+                room[k].at = p + n;
+                return p;
+            }
+        }
+        return nullptr;
     };
-    AdjArgs d = {};
-    d.gk_buf = reinterpret_cast<float *>(take(adjoint_grad_bytes(nframes, nrx, np)));
-    d.partial = reinterpret_cast<float *>(take(adjoint_partial_bytes(nframes, ntx, nrx, np, nt)));
-    d.live = reinterpret_cast<unsigned char *>(take((size_t)nrx * tiles));
-    d.ranges = reinterpret_cast<float2 *>(take(tiles * nel * sizeof(float2)));
-    d.depth = reinterpret_cast<float *>(take(tiles * sizeof(float)));
-    d.windows = reinterpret_cast<int2 *>(take(parts * (size_t)nch * sizeof(int2)));
-    d.order = reinterpret_cast<int *>(take(tiles * sizeof(int)));
-    const size_t table = nel * (size_t)np * sizeof(float);
-    if (synthetic && table <= kAdjTableMax) {
-        d.tau_tx = reinterpret_cast<float *>(take((size_t)ntx * np * sizeof(float)));
-        d.tau_rx = reinterpret_cast<float *>(take((size_t)nrx * np * sizeof(float)));
+    if (!g->grad_rf) return;
+    char *const small = take(tiles * (nel * sizeof(float2) + sizeof(float) + sizeof(int)), 3);
+    if (small) {
+        g->ranges = reinterpret_cast<float2 *>(small);
+        g->depth = reinterpret_cast<float *>(g->ranges + tiles * nel);
+        g->order = reinterpret_cast<int *>(g->depth + tiles);
     }
-    if (g) {
-        g->gk_buf = d.gk_buf;
-        g->partial = d.partial;
-        g->live = d.live;
-        g->ranges = d.ranges;
-        g->depth = d.depth;
-        g->windows = d.windows;
-        g->order = d.order;
-        g->tau_tx = d.tau_tx;
-        g->tau_rx = d.tau_rx;
+    if (g->geom != GEOM_TABBED && nel * np * sizeof(float) <= kAdjTableMax) {
+        g->tau_rx = reinterpret_cast<float *>(take((size_t)a.nrx * np * sizeof(float), 2));
+        if (g->tau_rx) g->tau_tx = reinterpret_cast<float *>(take((size_t)a.ntx * np * sizeof(float), 2));
     }
-    return at;
 }
 
 cudaError_t launch_adjoint(const AdjArgs &g, int dtype, cudaStream_t s) {

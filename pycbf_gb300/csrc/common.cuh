@@ -296,18 +296,18 @@ struct AdjArgs {
     float *gk_buf;        // workspace: grad_out gathered into kernel pixel order
     float *partial;       // workspace: per-part sums of the spline-record adjoints
     unsigned char *live;  // workspace: live[r * tiles + tile] = receive r can contribute to the tile
-    float2 *ranges;       // workspace: per tile the delay ranges of ntx transmits, nrx receives
-    float *depth;         // workspace: per tile the earliest delay of the middle transmit
-    int2 *windows;        // workspace: per part and channel the intervals written in partial
-    int *order;           // workspace: the tiles by depth
-    float *tau_tx, *tau_rx;  // workspace: Synthetic delays (ntx, np), (nrx, np), or null
+    // null where there is no room for them (adjoint_layout):
+    float2 *ranges;       // per tile the delay ranges of ntx transmits, nrx receives
+    float *depth;         // per tile the earliest delay of the middle transmit
+    int *order;           // the tiles by depth
+    float *tau_tx, *tau_rx;  // Synthetic delays (ntx, np), (nrx, np)
     const float *gk;      // set by launch_adjoint: gk_buf, or grad_out without pixel_index
 };
 // parts of the tiles whose channel adjoints are summed separately
 int adjoint_parts(long long nch, long long np);
-// the workspace: its size, and its pieces set in g (both may be null)
-size_t adjoint_layout(long long nframes, long long ntx, long long nrx, long long np, int nt,
-                      bool synthetic, char *ws, AdjArgs *g);
+size_t adjoint_workspace_bytes(long long nframes, long long ntx, long long nrx, long long np, int nt);
+// the pieces of a workspace of at least that size, set in g
+void adjoint_layout(char *ws, size_t bytes, AdjArgs *g);
 cudaError_t launch_adjoint(const AdjArgs &a, int dtype, cudaStream_t s);
 cudaError_t launch_das_synth_slow(const DasArgs &a, int sumtype, int dtype, cudaStream_t s);
 

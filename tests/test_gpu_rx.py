@@ -143,3 +143,28 @@ def test_delay_gradients_of_one_frame_and_of_several(ntx, nrx, npx, sumtype, dty
     rows = adjoint.das_synthetic_slowness(rf[0], slow0, syn, sumtype="tx_only").cpu().numpy()
     image = adjoint.das_synthetic_slowness(rf[0], slow0, syn, sumtype="tx_and_rx").cpu().numpy()
     np.testing.assert_array_equal(image, _block_sums(rows.reshape(nrx, npx)))
+
+
+@pytest.mark.parametrize("ntx,nrx,npx,nt", [(2, 1, 5000, 16), (1, 1, 1, 2), (3, 7, 300, 301), (5, 33, 4000, 64)])
+@pytest.mark.parametrize("sumtype", ["tx_and_rx", "tx_only"])
+@pytest.mark.parametrize("make", [_tabbed, _synthetic])
+def test_channel_gradients_in_the_least_workspace(ntx, nrx, npx, nt, sumtype, make, monkeypatch):
+    """With and without room for the delay ranges and tables: the same sums over other
+    parts, at most 5000 taps a sample in float32 (1e-5 of the largest sum)."""
+    bf = make(ntx, nrx, npx, nt, ntx + nrx)
+    rf = _channels(bf, 6)
+    slow = torch.full((npx,), 1 / 1540.0, device="cuda")
+
+    def grad():
+        x = rf.clone().requires_grad_(True)
+        out = (adjoint.das_synthetic_slowness(x, slow, bf, sumtype=sumtype) if make is _synthetic
+               else bf.differentiable(x, sumtype=sumtype))
+        g = torch.randn(out.shape, generator=torch.Generator().manual_seed(7)).cuda()
+        return torch.autograd.grad(out, x, g)[0]
+
+    full = grad()
+    def least(L, info, np_, synthetic, device):
+        n = L.pycbf_gb_adjoint_workspace_bytes(info, np_)
+        return torch.empty(n, dtype=torch.uint8, device=device), n
+    monkeypatch.setattr(adjoint, "_workspace", least)
+    assert bool(((grad() - full).abs() <= 1e-5 * full.abs().max()).all())
