@@ -41,12 +41,7 @@ SUMTYPES = ("tx_and_rx", "tx_only")
 _DTYPE = {torch.float32: _lib.F32, torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}
 
 
-def _ptr(t):
-    return ct.c_void_p(t.data_ptr()) if t is not None else None
-
-
-def _stream():
-    return ct.c_void_p(torch.cuda.current_stream().cuda_stream)
+_stream, _ptr = _lib.stream, _lib.ptr
 
 
 @dataclass(frozen=True)

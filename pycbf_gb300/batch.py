@@ -66,8 +66,7 @@ def assign_branches(costs: Sequence[float], nbranch: int) -> list:
     return out
 
 
-def _stream():
-    return ct.c_void_p(torch.cuda.current_stream().cuda_stream)
+_stream = _lib.stream
 
 
 class BatchBeamformer:

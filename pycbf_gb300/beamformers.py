@@ -59,12 +59,7 @@ def _require_cuda():
         raise BeamformerException("pycbf_gb300 needs a CUDA device; none is available")
 
 
-def _stream_ptr():
-    return ct.c_void_p(torch.cuda.current_stream().cuda_stream)
-
-
-def _ptr(t):
-    return ct.c_void_p(t.data_ptr()) if t is not None else None
+_stream_ptr, _ptr = _lib.stream, _lib.ptr
 
 
 def _to_host(out: torch.Tensor) -> np.ndarray:
@@ -673,7 +668,7 @@ class SyntheticBeamformer(Synthetic, _GPUBeamformer):
         dev["pnts"] = pnts
         self._dev = dev
         self._geom = _lib.SyntheticGeom(
-            **{k: _ptr(dev[k]).value for k in ("ovectx", "nvectx", "t0tx", "alatx", "doftx",
+            **{k: _ptr(dev[k]) for k in ("ovectx", "nvectx", "t0tx", "alatx", "doftx",
                                                 "cosalatx", "secalatx", "halfdofsintx", "ovecrx",
                                                 "nvecrx", "cosalarx", "pnts")},
             np=self.nop, c0=float(np.float32(self.c0)))

@@ -17,7 +17,7 @@ device, with no host round trip.
 """
 from __future__ import annotations
 
-import ctypes as ct
+import math
 from collections import OrderedDict
 
 import numpy as np
@@ -29,12 +29,7 @@ __all__ = ["Demodulator", "fft_tukey_demod", "zout_fft_tukey_demod", "percentile
            "log_compress", "bmode_compress", "tukey", "demod_matrix"]
 
 
-def _stream():
-    return ct.c_void_p(torch.cuda.current_stream().cuda_stream)
-
-
-def _p(t):
-    return ct.c_void_p(t.data_ptr()) if t is not None else None
+_stream, _p = _lib.stream, _lib.ptr
 
 
 def tukey(M: int, alpha: float = 0.25) -> np.ndarray:
@@ -170,12 +165,12 @@ class Demodulator:
         axis = axis % x.ndim
         if x.shape[axis] != self.n:
             raise ValueError(f"axis {axis} has {x.shape[axis]} samples, the demodulator {self.n}")
-        xm = x.movedim(axis, -1).contiguous()
+        xm = (x if axis == x.ndim - 1 else x.movedim(axis, -1)).contiguous()
         return xm, axis
 
     def _run(self, xm, want_iq, want_env):
         lead = xm.shape[:-1]
-        ncols = int(np.prod(lead)) if lead else 1
+        ncols = math.prod(lead)
         iq = torch.empty((*lead, self.M, 2), dtype=torch.float32, device=xm.device) if want_iq else None
         env = torch.empty((*lead, self.M), dtype=torch.float32, device=xm.device) if want_env else None
         st = self._lib.pycbf_gb_demod(_p(xm), ncols, self.n, _p(self._W), self.M, _p(iq), _p(env),
@@ -191,12 +186,12 @@ class Demodulator:
     def envelope(self, x, axis: int = -1) -> torch.Tensor:
         xm, axis = self._lines(x, axis)
         _, env = self._run(xm, False, True)
-        return env.movedim(-1, axis)
+        return env if axis == env.ndim - 1 else env.movedim(-1, axis)
 
     def bmode(self, x, axis: int = -1, q: float = 99.0, floor: float = 1e-10,
               image_ndim: int | None = None) -> torch.Tensor:
         env = self.envelope(x, axis).contiguous()
-        nseg = 1 if image_ndim is None else int(np.prod(env.shape[: env.ndim - image_ndim]))
+        nseg = 1 if image_ndim is None else math.prod(env.shape[: env.ndim - image_ndim])
         return bmode_compress(env, q, floor, nseg, out=env)[0]
 
 
