@@ -408,8 +408,7 @@ def main_ours(a):
     achieved = alg_bytes / das_s / 1e9
     roofline = {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                 "frac": achieved / hbm_peak, "traffic": None,
-                "kernel": ("das_staged_kernel<cubic, tx_and_rx, f32>" if bf._plan is not None
-                           else "das_kernel<tabbed, cubic, tx_and_rx, f32>"),
+                "kernel": "das_rx_kernel<tabbed, cubic, tx_and_rx, f32>",
                 "kernel_ms": 1e3 * das_s, "spline_ms": statistics.mean(spline_ms),
                 "peak_source": "measured" if peaks.get("hbm_gbs") else "fallback",
                 "algorithmic_bytes": alg_bytes}
@@ -542,7 +541,7 @@ def run_variants(a, w, dev, taps, ctx):
             nbytes = table_bytes + nf * (ntx * nrx * nt * x.element_size() + 4 * np_)
             res[name]["roofline"] = roofline_of(
                 t, nbytes, nf * das_flops(ctx["contrib"], taps), hbm, fp32p,
-                "das_staged_kernel (frame, tile) items + spline_coef_kernel")
+                "das_frames_kernel + spline_pairs_kernel")
             o = out.reshape(nf, -1)[:, torch.as_tensor(cols, device=dev)]
             errs = [rel_l2_t(o[k], scales[k] * f64) for k in range(nf)]
             res[name]["fp64_rel_l2"] = max(errs)
@@ -769,11 +768,11 @@ def run_synthetic_variants(a, dev, ctx):
     flops = das_flops(contrib, taps, delays=8 * (bf.ntx + bf.nrx) * np_)
     res["matrix_3d_fp16"] = {"value": taps / t, "unit": UNIT, "ms_per_call": 1e3 * t,
                              "frames_per_call": 8, "taps": taps, "contributing_taps": contrib,
-                             "storage": "float16", "launches_per_call": 2,
+                             "storage": "float16", "launches_per_call": 5,
                              "workload": "synthetic 3-D 32x32 matrix 25dw 2048s 128x128x256",
                              "roofline": roofline_of(t, io_bytes, flops, hbm, fp32p,
-                                                     "das_kernel<synthetic, cubic, tx_and_rx, f16> "
-                                                     "+ spline_coef_kernel")}
+                                                     "das_frames_kernel<synthetic, tx_and_rx, f16> "
+                                                     "(4 launches) + spline_pairs_kernel")}
     return res
 
 
@@ -911,7 +910,7 @@ def run_adjoint_variants(a, w, dev, taps, ctx):
                                                  "against float64 autograd in the tests",
                              "roofline": roofline_of(t_fa, nbytes, flops, ctx["hbm_peak"],
                                                      ctx["fp32_peak"],
-                                                     "spline + das_staged_kernel + adj_delay_kernel "
+                                                     "spline + das_rx_kernel + adj_delay_kernel "
                                                      "+ adj_scatter_kernel + adj_finalize_kernel")}
 
     sw = phantom.two_layer_pw_synthetic(device=dev)

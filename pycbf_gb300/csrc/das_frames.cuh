@@ -17,8 +17,9 @@
 // in das_rx_kernel.  Against a thread per pixel and all its receives (128 pixels, 16
 // warps an SM), with 11 transmits, 128 receives and 256 x 512 pixels from tables: four
 // float32 frames 591 -> 364 us, eight float16 857 -> 541; 64 x 256 pixels, eight frames
-// 567 -> 240 us; two 75-transmit synthetic frames 5.3 -> 4.7 ms; eight 3-D float16
-// volumes 53.8 -> 56.8 ms (the smaller tiles share fewer gathers in L1).
+// 567 -> 240 us; two synthetic frames of 75 transmits, 192 receives and 512 x 1024
+// pixels 5.3 -> 4.7 ms; eight 3-D float16 volumes 53.8 -> 56.8 ms (a third of the sectors
+// of their gathers hit L1 there, a ninth here; CTAs of 64 pixels gained 1 %).
 // The operations on one frame and their order are those of cubic_taps and
 // das_pixel, so the images are the single-frame ones bit for bit.
 #pragma once

@@ -15,7 +15,8 @@
 // used).  One float32 frame, cubic, 256 x 512 pixels and 128 receives unless said
 // otherwise, against the kernels before (synthetic: das_kernel; tables: das_staged_kernel
 // on its TMA windows up to 12 transmits, das_kernel beyond):
-//   synthetic, 75 transmits, 192 receives   3910 -> 2880 us (64 x 128 pixels 2350 -> 610)
+//   synthetic, 75 transmits, 192 receives,
+//           512 x 1024 pixels              3910 -> 2880 us (64 x 128 pixels 2350 -> 610)
 //   tables, 11 transmits                     170 ->  151 us (64 x 128 pixels 143 -> 40)
 //           1 / 5 / 8 transmits      90 / 121 / 138 -> 82 / 116 / 122 us
 //           11, 192 receives                 194 ->  187 us
