@@ -404,7 +404,7 @@ __host__ __device__ inline int cubic_column_padded(int ntx) {
 // instructions and 3.6 ms (20 a tap, half the issue slots; the rest waits on the
 // gathers) in das_kernel, against 3.84e9 and 4.9 ms with the tests and knots kept as bit
 // masks, 64-bit addresses and every constant fetched again; with the receives over
-// warps (das_rx_kernel) 2.7 ms.
+// warps (das_rx_kernel) 2.6 ms.
 // Every decision is the reference's: t0 <= x <= xmax and |w| >= thresh on the
 // rounded x and w, and the knot of the correctly rounded quotient.  h = s - j is
 // within 1/2 - eps_fast of zero unless the quotient is so near an integer that
