@@ -657,7 +657,8 @@ adj_finalize_kernel(const float *__restrict__ partial, int nparts, long long nch
     float *u = zv + stride;
     const float *p0 = partial + (size_t)ch * 2 * Lp;
     const size_t pstride = (size_t)nch * 2 * Lp;  // between parts
-    // the parts' samples into dst, parts in order, each from its window only
+    // the parts' samples into dst, parts in order, each from its window only; sample n is
+    // lane n % 32's in every part, so no lane adds to another's sum
     auto sum_parts = [&](float *dst, int off) {
         for (int n = lane; n < nt; n += 32) dst[n] = 0.f;
         int2 wins = make_int2(0, 0);  // of part q0 + lane
@@ -670,7 +671,8 @@ adj_finalize_kernel(const float *__restrict__ partial, int nparts, long long nch
             const float *src = p0 + q * pstride + off;
             if (win.x >= win.y) continue;
 #pragma unroll 4
-            for (int n = win.x + lane; n <= min(win.y, nt - 1); n += 32) dst[n] += src[n];
+            for (int n = (win.x & ~31) + lane; n <= min(win.y, nt - 1); n += 32)
+                if (n >= win.x) dst[n] += src[n];
         }
     };
     sum_parts(zv, Lp);

@@ -1,0 +1,43 @@
+"""Gradients at the edges of their kernels' division of the work (GPU)."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import adjoint_ref
+from pycbf_gb300 import adjoint
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, b):
+    a, b = a.detach().double().cpu(), b.detach().double().cpu()
+    return float(torch.linalg.norm(a - b) / torch.linalg.norm(b))
+
+
+@pytest.mark.parametrize("step", [37, 5, 32])
+def test_channel_gradient_from_parts_with_shifted_windows(step):
+    """Four parts of 2048 pixels whose windows of samples overlap and begin `step` samples
+    apart, so that a sample's place in the window differs from part to part: the sums
+    over the parts against float64 autograd (at most 4000 taps a sample; 1e-5 as for the
+    other channel gradients), and the same bits every time."""
+    ntx, nrx, npx, nt, t0, dt = 2, 3, 8192, 301, 1.3e-7, 4e-8
+    r = np.random.default_rng(step)
+    at = np.arange(npx) // 2048 * step + r.uniform(3, 120, npx)
+    f32 = lambda a: torch.as_tensor(np.asarray(a, np.float32))
+    tautx = f32(t0 + dt * (at + r.uniform(0, 2, (ntx, 1))))
+    taurx = f32(dt * r.uniform(0, 40, (nrx, 1)) + np.zeros((1, npx)))
+    apodtx, apodrx = f32(r.uniform(0.2, 1, (ntx, npx))), f32(r.uniform(0.2, 1, (nrx, npx)))
+    rf, g = f32(r.standard_normal((1, ntx, nrx, nt))), f32(r.standard_normal((1, npx)))
+
+    def grad():
+        x = rf.cuda().requires_grad_(True)
+        out = adjoint.das_tabbed(x, tautx.cuda(), taurx.cuda(), apodtx.cuda(), apodrx.cuda(), t0=t0, dt=dt)
+        return torch.autograd.grad(out, x, g.cuda())[0]
+
+    x64 = rf.double().requires_grad_(True)
+    ref = adjoint_ref.das_tabbed_ref(x64, *(t.double() for t in (tautx, taurx, apodtx, apodrx)), t0, dt)
+    want = torch.autograd.grad(ref, x64, g.double())[0]
+    got = grad()
+    assert _rel(got, want) <= 1e-5
+    for _ in range(20):
+        assert torch.equal(grad(), got)
