@@ -161,6 +161,7 @@ __global__ void __launch_bounds__(32 * kRxWarps, 4) adj_delay_kernel(const __gri
             trx = slow_delay(live, Drx, slow, 0.f);
         }
         float grx = 0.f;
+        bool tap = false;  // some tap of this pixel and receive counts
         // the forward's exact reject, by warps: no tap of the others passes its tests
         if (__any_sync(kFull, live)) {
             const float gp0 = nfr == 1 && SUM == PYCBF_GB_SUM_TX_ONLY
@@ -233,6 +234,7 @@ __global__ void __launch_bounds__(32 * kRxWarps, 4) adj_delay_kernel(const __gri
                             const float2 D = add2_rn(w2[p], make_float2(Drx, Drx));
                             if (ok[2 * p]) grx = fmaf(slope.x, D.x, grx);
                             if (ok[2 * p + 1]) grx = fmaf(slope.y, D.y, grx);
+                            tap = tap || ok[2 * p] || ok[2 * p + 1];
                         }
                     }
                     continue;
@@ -281,7 +283,7 @@ __global__ void __launch_bounds__(32 * kRxWarps, 4) adj_delay_kernel(const __gri
                     }
                 }
             }
-            if (ONE && !W) gs = fmaf(gq, grx, gs);
+            if (ONE && !W && tap) gs = fmaf(gq, grx, gs);  // else gq may be infinite or NaN
         }
         if (W && g.grad_taurx && valid) g.grad_taurx[(long long)r * np + i] = grx;
     }

@@ -5,6 +5,7 @@ import torch
 
 from oracle import adjoint_ref
 from pycbf_gb300 import adjoint
+from test_gpu_rx import DT, _channels, _synthetic, _tabbed
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +42,37 @@ def test_channel_gradient_from_parts_with_shifted_windows(step):
     assert _rel(got, want) <= 1e-5
     for _ in range(20):
         assert torch.equal(grad(), got)
+
+
+@pytest.mark.parametrize("nframes", [1, 2])
+@pytest.mark.parametrize("dtype", ["float32", "float16"])
+@pytest.mark.parametrize("make", [_tabbed, _synthetic])
+def test_upstream_gradient_of_pixels_without_taps_is_not_used(make, dtype, nframes):
+    """Receives that are masked, or whose taps all miss the record, leave exact zeros in
+    the per-receive images; whatever the upstream gradient is there, NaN included, every
+    gradient is the one that zeros there give, bit for bit."""
+    ntx, nrx, npx, nt = 3, 21, 333, 301
+    bf = make(ntx, nrx, npx, nt, 4)
+    rf = _channels(bf, 8, nframes if nframes > 1 else 0, DT[dtype])
+    slow = torch.full((npx,), 1 / 1500.0, device="cuda")
+    if make is _synthetic:
+        slow[::7] *= 1.6  # past the end of the record for the farther receives
+
+    def grads(fill):
+        x = rf.clone().requires_grad_(True)
+        if make is _synthetic:
+            leaves = [x, slow.clone().requires_grad_(True)]
+            out = adjoint.das_synthetic_slowness(*leaves, bf, sumtype="tx_only")
+        else:
+            ttx, atx, trx, arx = bf._tables
+            leaves = [x, ttx.clone().requires_grad_(True), trx.clone().requires_grad_(True)]
+            out = adjoint.das_tabbed(*leaves, atx, arx, t0=bf.t0, dt=bf.dt, thresh=bf.thresh,
+                                     sumtype="tx_only")
+        g = torch.randn(out.shape, generator=torch.Generator().manual_seed(9)).cuda()
+        empty = out == 0
+        assert 0 < int(empty.sum()) < empty.numel()
+        return torch.autograd.grad(out, leaves, torch.where(empty, torch.full_like(g, fill), g))
+
+    for zero, nan, inf in zip(*(grads(v) for v in (0.0, float("nan"), float("inf")))):
+        assert torch.equal(zero, nan) and torch.equal(zero, inf)
+        assert float(zero.abs().max()) > 0
