@@ -255,8 +255,10 @@ __global__ void __launch_bounds__(32 * kRxWarps, frames_ctas(GEOM, FG))
                 if (kEach) {
                     if (valid) a.out[((long long)(f0 + f) * nrx + r) * np + op] = v;
                 } else {
-                    if (SUM == PYCBF_GB_SUM_DMAS_SSR && !a.dmas_power)
-                        v = copysignf(sqrtf(fabsf(v)), v);
+                    if (SUM == PYCBF_GB_SUM_DMAS_SSR) {
+                        if (!a.dmas_power) v = copysignf(sqrtf(fabsf(v)), v);
+                        if (!live) v = __uint_as_float(kDeadSum);
+                    }
                     sums[(e * FG + f) * 32] = v;
                 }
             }
@@ -270,12 +272,8 @@ __global__ void __launch_bounds__(32 * kRxWarps, frames_ctas(GEOM, FG))
 #pragma unroll 8
                 for (int e = e0; e < e1; ++e) {
                     const float v = sums[(e * FG + w) * 32];
-                    if (SUM == PYCBF_GB_SUM_TX_AND_RX) {
-                        b += v;
-                    } else {
-                        acc = fmaf(v, s1, acc);
-                        s1 += v;
-                    }
+                    if (SUM == PYCBF_GB_SUM_TX_AND_RX) b += v;
+                    else dmas_add(v, acc, s1);
                 }
                 acc += b;
             }

@@ -1067,7 +1067,7 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
         if (SUM == PYCBF_GB_SUM_TX_AND_RX) bacc += accr;
         if (!CENSUS && SUM == PYCBF_GB_SUM_TX_ONLY && valid)
             a.out[((long long)f * nrx + r) * np + op] = accr;
-        if (SUM == PYCBF_GB_SUM_DMAS_SSR || SUM == PYCBF_GB_SUM_DMAS_POWER) {
+        if ((SUM == PYCBF_GB_SUM_DMAS_SSR || SUM == PYCBF_GB_SUM_DMAS_POWER) && live) {
             // pairwise sum over receives i<j of s_i s_j as sum_j s_j * (sum_{i<j} s_i):
             // no cancellation, two FMAs per receive
             const float s = (SUM == PYCBF_GB_SUM_DMAS_SSR) ? copysignf(sqrtf(fabsf(accr)), accr) : accr;

@@ -36,6 +36,17 @@ constexpr int kRxWarps = 8;
 template <int GEOM> constexpr int kRxRun = GEOM == GEOM_TABBED ? 64 : 256;
 constexpr size_t kRxSmemMax = 100 * 1024;  // two CTAs an SM
 
+// What DMAS keeps as the sum of a receive that does not reach a pixel, and then leaves out
+// (a zero would turn an infinite sum before it into NaN): a NaN that no arithmetic gives.
+constexpr unsigned kDeadSum = 0x7fc0dead;
+// one receive's sum into DMAS's image and running sum: the pairs i < j as s_j * sum_i s_i
+__device__ __forceinline__ void dmas_add(float s, float &acc, float &s1) {
+    if (__float_as_uint(s) != kDeadSum) {
+        acc = fmaf(s, s1, acc);
+        s1 += s;
+    }
+}
+
 inline size_t das_rx_smem(int geom, int ntx, int nrx) {
     const size_t rows = geom == GEOM_TABBED ? 5 * kRxRun<GEOM_TABBED>
                                             : std::min(nrx, kRxRun<GEOM_SYNTH>);
@@ -178,7 +189,9 @@ __global__ void __launch_bounds__(32 * kRxWarps, GEOM == GEOM_TABBED ? 4 : 3)
             }
             if (!__any_sync(kFull, live)) {
                 if (kEach && valid) a.out[((long long)f * nrx + r) * np + op] = 0.f;
-                if (!kEach) sums[(size_t)e * 32] = 0.f;
+                if (!kEach)
+                    sums[(size_t)e * 32] =
+                        SUM == PYCBF_GB_SUM_DMAS_SSR ? __uint_as_float(kDeadSum) : 0.f;
                 continue;
             }
             auto sum = S::zero();
@@ -202,7 +215,10 @@ __global__ void __launch_bounds__(32 * kRxWarps, GEOM == GEOM_TABBED ? 4 : 3)
             if (kEach) {
                 if (valid) a.out[((long long)f * nrx + r) * np + op] = v;
             } else {
-                if (SUM == PYCBF_GB_SUM_DMAS_SSR && !a.dmas_power) v = copysignf(sqrtf(fabsf(v)), v);
+                if (SUM == PYCBF_GB_SUM_DMAS_SSR) {
+                    if (!a.dmas_power) v = copysignf(sqrtf(fabsf(v)), v);
+                    if (!live) v = __uint_as_float(kDeadSum);
+                }
                 sums[(size_t)e * 32] = v;
             }
         }
@@ -221,11 +237,7 @@ __global__ void __launch_bounds__(32 * kRxWarps, GEOM == GEOM_TABBED ? 4 : 3)
         } else if (SUM == PYCBF_GB_SUM_DMAS_SSR) {
             if (w == 0) {
 #pragma unroll 8
-                for (int e = 0; e < n; ++e) {
-                    const float s = sums[(size_t)e * 32];
-                    acc = fmaf(s, s1, acc);
-                    s1 += s;
-                }
+                for (int e = 0; e < n; ++e) dmas_add(sums[(size_t)e * 32], acc, s1);
             }
             __syncthreads();
         }

@@ -775,7 +775,7 @@ __global__ void __launch_bounds__(kBlock, 5) das_staged_kernel(const __grid_cons
             if (SUM == PYCBF_GB_SUM_TX_AND_RX) bacc += accr;
             if (SUM == PYCBF_GB_SUM_TX_ONLY && valid)
                 a.out[((long long)f * nrx + r) * np + op] = accr;
-            if (SUM == PYCBF_GB_SUM_DMAS_SSR || SUM == PYCBF_GB_SUM_DMAS_POWER) {
+            if ((SUM == PYCBF_GB_SUM_DMAS_SSR || SUM == PYCBF_GB_SUM_DMAS_POWER) && live) {
                 const float sv = (SUM == PYCBF_GB_SUM_DMAS_SSR) ? copysignf(sqrtf(fabsf(accr)), accr) : accr;
                 acc = fmaf(sv, s1, acc);
                 s1 += sv;
