@@ -427,6 +427,7 @@ __global__ void __launch_bounds__(256) adj_rank_kernel(const float *__restrict__
 // masks (59 and 52 % of the issue slots), against 920 and 1271 for one CTA a channel
 // part whose warps took turns on full-length rows between barriers.
 constexpr int kSeg = 512;  // intervals of a warp's rows: 8 KB, seven CTAs an SM
+constexpr int kPartTiles = 16384;  // a part's tile list has to fit shared memory
 
 template <int GEOM, int SUM, bool TABLES>
 __global__ void __launch_bounds__(128, 5) adj_scatter_kernel(const __grid_constant__ AdjArgs g,
@@ -736,14 +737,11 @@ cudaError_t launch_scatter_one(const AdjArgs &g0, cudaStream_t s) {
         g.order = nullptr;
     }
     const size_t smem = 4 * kSeg * sizeof(float4) + per * sizeof(int);
-    if (smem > 48 * 1024) {
-        const int lim = (int)smem;
-        const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        err = cudaFuncSetAttribute(adj_scatter_kernel<GEOM, SUM, true>, attr, lim);
-        if (err == cudaSuccess && kSynth)
-            err = cudaFuncSetAttribute(adj_scatter_kernel<GEOM, SUM, !kSynth>, attr, lim);
-        if (err != cudaSuccess) return err;
-    }
+    const int most = (int)(4 * kSeg * sizeof(float4) + kPartTiles * sizeof(int));
+    err = cudaFuncSetAttribute(
+        tables ? adj_scatter_kernel<GEOM, SUM, true> : adj_scatter_kernel<GEOM, SUM, !kSynth>,
+        cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (err != cudaSuccess) return err;
     const long long groups = (long long)a.nframes * ((a.ntx + 3) / 4) * a.nrx;
     if (groups > 0x7fffffffLL) return cudaErrorInvalidValue;
     const dim3 grid((unsigned)groups, (unsigned)nparts);
@@ -809,8 +807,8 @@ int adjoint_parts(long long nch, long long np) {
     long long p = (11264 + nch - 1) / nch;
     p = std::min<long long>(p, std::max<long long>(1, np / 2048));
     p = std::max<long long>(1, std::min<long long>(p, 64));
-    // a part's tile list has to fit shared memory: 16,384 tiles
-    return (int)std::max<long long>(p, ((np + kBlock - 1) / kBlock + 16383) / 16384);
+    const long long tiles = (np + kBlock - 1) / kBlock;
+    return (int)std::max<long long>(p, (tiles + kPartTiles - 1) / kPartTiles);
 }
 
 static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }

@@ -76,3 +76,21 @@ def test_upstream_gradient_of_pixels_without_taps_is_not_used(make, dtype, nfram
     for zero, nan, inf in zip(*(grads(v) for v in (0.0, float("nan"), float("inf")))):
         assert torch.equal(zero, nan) and torch.equal(zero, inf)
         assert float(zero.abs().max()) > 0
+
+
+def test_channel_gradient_of_parts_of_4096_tiles():
+    """64 parts of 4096 tiles of 128 pixels, whose list in shared memory leaves no room for
+    the kernel's static part below the default limit.  The image is linear in the channel
+    data v, so <image(v), g> = <v, gradient>: sums of 8192 float32 taps a sample and part, 64
+    parts, and 64 samples give 4e-6 of |image| |g| / sqrt(pixels); 1e-4 allowed."""
+    npx, nt, t0, dt = 64 * 4096 * 128, 64, 0.0, 4e-8
+    gen = torch.Generator(device="cuda").manual_seed(10)
+    u = lambda a, b: torch.empty((1, npx), device="cuda").uniform_(a, b, generator=gen)
+    tautx, taurx, apodtx, apodrx = u(0, 40 * dt), u(0, 20 * dt), u(0.5, 1), u(0.5, 1)
+    v = torch.randn((1, 1, nt), generator=gen, device="cuda").requires_grad_(True)
+    out = adjoint.das_tabbed(v, tautx, taurx, apodtx, apodrx, t0=t0, dt=dt)
+    g = torch.randn(out.shape, generator=gen, device="cuda")
+    grad = torch.autograd.grad(out, v, g)[0].double()
+    image, g, v = out.detach().double(), g.double(), v.detach().double()
+    tol = 1e-4 * float(image.norm()) * float(g.norm()) / npx ** 0.5
+    assert abs(float((image * g).sum()) - float((v * grad).sum())) <= tol
