@@ -572,7 +572,6 @@ int pycbf_gb_slsc_with_kept(const float *im, const unsigned *kept, long long nfr
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr long long kMaxAdjTx = 128;  // three shared-memory columns per transmit (192 KB)
 
 int check_adjoint_common(const pycbf_gb_rfinfo *rf, const void *coef, int sumtype, bool synthetic) {
     int st = check_rf(rf, synthetic);

@@ -704,8 +704,7 @@ cudaError_t launch_delay_one(const AdjArgs &g, cudaStream_t s) {
                                                   : adj_delay_kernel<GEOM, SUM, T, false>;
     const size_t smem = delay_smem_bytes(GEOM, g.d.ntx);
     if (smem > 40 * 1024) {  // with the static part
-        cudaError_t err =
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t err = allow_smem(kern, delay_smem_bytes(GEOM, kMaxAdjTx));
         if (err != cudaSuccess) return err;
     }
     kern<<<(unsigned)((g.d.np + 31) / 32), 32 * kRxWarps, smem, s>>>(g);
@@ -737,10 +736,9 @@ cudaError_t launch_scatter_one(const AdjArgs &g0, cudaStream_t s) {
         g.order = nullptr;
     }
     const size_t smem = 4 * kSeg * sizeof(float4) + per * sizeof(int);
-    const int most = (int)(4 * kSeg * sizeof(float4) + kPartTiles * sizeof(int));
-    err = cudaFuncSetAttribute(
-        tables ? adj_scatter_kernel<GEOM, SUM, true> : adj_scatter_kernel<GEOM, SUM, !kSynth>,
-        cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    const size_t most = 4 * kSeg * sizeof(float4) + kPartTiles * sizeof(int);
+    err = allow_smem(
+        tables ? adj_scatter_kernel<GEOM, SUM, true> : adj_scatter_kernel<GEOM, SUM, !kSynth>, most);
     if (err != cudaSuccess) return err;
     const long long groups = (long long)a.nframes * ((a.ntx + 3) / 4) * a.nrx;
     if (groups > 0x7fffffffLL) return cudaErrorInvalidValue;
@@ -758,8 +756,7 @@ cudaError_t launch_scatter_one(const AdjArgs &g0, cudaStream_t s) {
     const size_t per_warp = sizeof(float) * 2 * (size_t)((a.nt + 4) & ~3);
     const int wpb = (int)std::min<size_t>(8, std::max<size_t>(1, (112 * 1024) / per_warp));
     const size_t fsmem = per_warp * wpb;
-    err = cudaFuncSetAttribute(adj_finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)fsmem);
+    err = allow_smem(adj_finalize_kernel, kSmemMax);
     if (err != cudaSuccess) return err;
     const long long blocks = (nch + wpb - 1) / wpb;
     adj_finalize_kernel<<<(unsigned)blocks, 32 * wpb, fsmem, s>>>(

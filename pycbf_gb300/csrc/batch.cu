@@ -227,21 +227,16 @@ size_t batch_full_smem_bytes(int max_ntx) {
     return (size_t)cubic_column_padded(std::max(max_ntx, 1)) * kBlock * sizeof(float);
 }
 
+constexpr size_t kBatchFixedSmem = 512;  // room for the kernels' static part
+static_assert(sizeof(BatchJob) + 32 <= kBatchFixedSmem, "");
+
 cudaError_t prepare_batch_das(int max_ntx) {
     const size_t smem = batch_full_smem_bytes(max_ntx);
-    if (smem > 227 * 1024) return cudaErrorInvalidValue;
-    const int lim = (int)std::max<size_t>(smem, 48 * 1024);
-    cudaError_t err =
-        cudaFuncSetAttribute(batch_das_full_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(batch_das_typed_kernel<float>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(batch_das_typed_kernel<__half>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(batch_das_typed_kernel<__nv_bfloat16>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    if (smem > kSmemMax) return cudaErrorInvalidValue;
+    cudaError_t err = allow_smem(batch_das_full_kernel, kSmemMax - kBatchFixedSmem);
+    if (err == cudaSuccess) err = allow_smem(batch_das_typed_kernel<float>, kSmemMax - kBatchFixedSmem);
+    if (err == cudaSuccess) err = allow_smem(batch_das_typed_kernel<__half>, kSmemMax - kBatchFixedSmem);
+    if (err == cudaSuccess) err = allow_smem(batch_das_typed_kernel<__nv_bfloat16>, kSmemMax - kBatchFixedSmem);
     return err;
 }
 

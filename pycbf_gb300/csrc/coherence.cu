@@ -453,8 +453,7 @@ cudaError_t launch_slsc(const float *im, const unsigned char *mask, const unsign
     bs = (bs / 32) * 32;
     if (bs < 32) return cudaErrorInvalidValue;
     const size_t smem = per_thread * bs;
-    cudaError_t err = cudaFuncSetAttribute(slsc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem);
+    cudaError_t err = allow_smem(slsc_kernel, kSmemMax);
     if (err != cudaSuccess) return err;
     const long long npix = (long long)nx * nz;
     const long long bx = (npix + bs - 1) / bs;

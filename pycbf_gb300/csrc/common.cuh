@@ -175,6 +175,17 @@ cudaError_t launch_spline_pairs(const SplineArgs &a, int dtype, cudaStream_t s);
 bool spline_pairs_fit(int nt);
 
 // ---------------------------------------------------------------------------
+// shared memory
+// ---------------------------------------------------------------------------
+constexpr size_t kSmemMax = 227 * 1024;  // of a CTA, the kernel's static part included
+// Raises a kernel's limit of dynamic shared memory to `most`: the same for every call of
+// that kernel, whatever the call needs.  Host threads share the limit, and one set to a
+// call's own size could be lowered by another thread's call before the launch.
+template <typename K> cudaError_t allow_smem(K *kern, size_t most) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
+// ---------------------------------------------------------------------------
 // delay-and-sum
 // ---------------------------------------------------------------------------
 // pixels (threads) per CTA of the delay-and-sum kernels: one table column each
@@ -303,6 +314,8 @@ struct AdjArgs {
     float *tau_tx, *tau_rx;  // Synthetic delays (ntx, np), (nrx, np)
     const float *gk;      // set by launch_adjoint: gk_buf, or grad_out without pixel_index
 };
+// ten shared-memory columns of 32 pixels per transmit and the table runs (192 KB)
+constexpr int kMaxAdjTx = 128;
 // parts of the tiles whose channel adjoints are summed separately
 int adjoint_parts(long long nch, long long np);
 size_t adjoint_workspace_bytes(long long nframes, long long ntx, long long nrx, long long np, int nt);

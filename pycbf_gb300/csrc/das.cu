@@ -22,7 +22,7 @@ cudaError_t launch_das_frames_bf16(const DasArgs &, int, int, int, cudaStream_t)
 
 bool das_frames_ok(const DasArgs &a, int sumtype) {
     return a.fast_axis && sumtype != PYCBF_GB_SUM_NONE && sumtype != PYCBF_GB_SUM_RX_ONLY &&
-           das_frames_smem(GEOM_TABBED, sumtype, 8, a.ntx) <= 200 * 1024;
+           das_frames_smem(GEOM_TABBED, sumtype, 8, a.ntx) <= kFramesSmemMax;
 }
 
 cudaError_t launch_das_frames(const DasArgs &a, int geom, int sumtype, int dtype, int fg,

@@ -134,6 +134,7 @@ __host__ __device__ constexpr int frames_run(int geom, int fg) {
     return geom == GEOM_SYNTH && fg == 2 ? 2 * kRxBlockSum : kRxBlockSum;
 }
 
+constexpr size_t kFramesSmemMax = 200 * 1024;
 inline size_t das_frames_smem(int geom, int sum, int fg, int ntx) {
     const size_t sums = sum == PYCBF_GB_SUM_TX_ONLY ? 0 : fg;
     const size_t rows = (sums + (geom == GEOM_TABBED ? 4 : 0)) * frames_run(geom, fg);
@@ -295,8 +296,7 @@ cudaError_t launch_das_frames_one(DasArgs a, cudaStream_t s) {
     auto kern = das_frames_kernel<GEOM, SUM, T, FG>;
     const size_t smem = das_frames_smem(GEOM, SUM, FG, a.ntx);
     if (smem > 40 * 1024) {  // with the static part
-        cudaError_t err =
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t err = allow_smem(kern, kFramesSmemMax);
         if (err != cudaSuccess) return err;
     }
     const dim3 grid((unsigned)((a.np + 31) / 32), (unsigned)(a.nframes / FG));

@@ -381,7 +381,7 @@ __device__ __forceinline__ void weight_range(float w, float &lo, float &hi) {
 // thread.  Cubic sums keep them as pairs, padded with infinite delays to whole
 // groups of kCubicGroup where that still fits; the padding of the last few
 // sizes below the limit does not, and their last transmits go one by one.
-constexpr size_t kColumnSmemMax = 227 * 1024;
+constexpr size_t kColumnSmemMax = kSmemMax;
 __host__ __device__ inline int cubic_column_padded(int ntx) {
     const int full = (ntx + kCubicGroup - 1) / kCubicGroup * kCubicGroup;
     return (size_t)full * kBlock * sizeof(float) <= kColumnSmemMax ? full : (ntx + 1) / 2 * 2;
@@ -1120,8 +1120,7 @@ cudaError_t launch_das_txm(const DasArgs &a, cudaStream_t s) {
     const size_t smem = das_smem_bytes(GEOM, SUM, a.ntx);
     auto kern = das_kernel<GEOM, KIND, SUM, T, CENSUS, TXM>;
     if (smem > 48 * 1024) {
-        cudaError_t err =
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t err = allow_smem(kern, kColumnSmemMax);
         if (err != cudaSuccess) return err;
     }
     const long long bx = (a.np + kBlock - 1) / kBlock;

@@ -250,8 +250,7 @@ cudaError_t launch_rx_one(const DasArgs &a, cudaStream_t s) {
     auto kern = das_rx_kernel<GEOM, KIND, SUM, T>;
     const size_t smem = das_rx_smem(GEOM, a.ntx, a.nrx);
     if (smem > 40 * 1024) {  // with the static part
-        cudaError_t err =
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t err = allow_smem(kern, kRxSmemMax);
         if (err != cudaSuccess) return err;
     }
     kern<<<dim3((unsigned)((a.np + 31) / 32), (unsigned)a.nframes), 32 * kRxWarps, smem, s>>>(a);

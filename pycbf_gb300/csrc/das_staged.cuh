@@ -65,6 +65,7 @@ constexpr int kUnstaged = 0x40000000;  // receive code flag: gathered from globa
 constexpr int kCodeFlags = kUnstaged;
 constexpr int kWinBits = 19;           // window start bits (the staged path needs nt <= 2^19)
 constexpr int kStagedMaxNt = 1 << kWinBits;
+constexpr int kStagedMaxRx = 4096;
 __host__ __device__ inline long long plan_tile_words(int nrx) {
     return 4 + (long long)kRxWords * nrx;
 }
@@ -930,9 +931,9 @@ template <int KIND, typename T>
 cudaError_t launch_plan_one(const DasArgs &a, int *plan, cudaStream_t s) {
     const long long tiles = (a.np + kBlock - 1) / kBlock;
     const size_t psmem = sizeof(int) * (size_t)a.nrx;
-    if (psmem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(tabbed_plan_kernel<KIND, T>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem);
+    const size_t fixed = (kTxReg + 1) * kBlock * sizeof(float);  // the kernel's static part
+    if (psmem + fixed > 48 * 1024) {
+        cudaError_t e = allow_smem(tabbed_plan_kernel<KIND, T>, kSmemMax - fixed);
         if (e != cudaSuccess) return e;
     }
     tabbed_plan_kernel<KIND, T><<<(unsigned)tiles, kBlock, psmem, s>>>(a, plan);
@@ -947,7 +948,7 @@ template <int KIND, int SUM, typename T>
 cudaError_t launch_staged_one(const DasArgs &a, const int *plan, int *status, cudaStream_t s) {
     auto kern = das_staged_kernel<KIND, SUM, T>;
     const int smem = (int)staged_smem_bytes(a.nrx);
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t err = allow_smem(kern, staged_smem_bytes(kStagedMaxRx));
     if (err != cudaSuccess) return err;
     int dev = 0, nsm = 0, per_sm = 0;
     if ((err = cudaGetDevice(&dev)) != cudaSuccess) return err;

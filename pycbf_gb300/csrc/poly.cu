@@ -141,8 +141,7 @@ cudaError_t launch_poly_t(const DasArgs &a, const void *rf, int interp, int k, c
     const size_t smem = interp == PYCBF_GB_INTERP_KORDER ? sizeof(float) * (size_t)k * k : 0;
     auto kern = poly_records_kernel<T>;
     if (smem > 48 * 1024) {
-        cudaError_t err =
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t err = allow_smem(kern, kSmemMax);
         if (err != cudaSuccess) return err;
     }
     kern<<<(unsigned)blocks, 256, smem, s>>>(static_cast<const T *>(rf), rec, nch, a.nt, a.dt,

@@ -222,8 +222,7 @@ static cudaError_t launch_spline_t(const SplineArgs &a, cudaStream_t s) {
         make_spline_table(&t);
         return t;
     }();
-    cudaError_t err = cudaFuncSetAttribute(spline_coef_kernel<T>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t err = allow_smem(spline_coef_kernel<T>, kSmemMax);
     if (err != cudaSuccess) return err;
     const long long blocks = (a.nch + ppb - 1) / ppb;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
@@ -246,8 +245,7 @@ static cudaError_t launch_spline_pairs_t(const SplineArgs &a, cudaStream_t s) {
         return t;
     }();
     auto kern = spline_pairs_kernel<T>;
-    cudaError_t err =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t err = allow_smem(kern, kSmemMax);
     if (err != cudaSuccess) return err;
     if (a.nch > 0x7fffffffLL || a.nframes % 2) return cudaErrorInvalidValue;
     kern<<<dim3((unsigned)a.nch, (unsigned)(a.nframes / 2)), 128, smem, s>>>(
@@ -278,8 +276,7 @@ cudaError_t launch_batch_spline(const BatchJob *jobs, int njobs, long long nch_t
         return t;
     }();
     if (set_attr) {
-        cudaError_t err = cudaFuncSetAttribute(batch_spline_kernel,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t err = allow_smem(batch_spline_kernel, kSmemMax);
         if (err != cudaSuccess) return err;
     }
     if (nch_total <= 0) return cudaSuccess;
