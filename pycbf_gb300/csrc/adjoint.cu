@@ -674,8 +674,8 @@ adj_finalize_kernel(const float *__restrict__ partial, int nparts, long long nch
             const float *src = p0 + q * pstride + off;
             if (win.x >= win.y) continue;
 #pragma unroll 4
-            for (int n = (win.x & ~31) + lane; n <= min(win.y, nt - 1); n += 32)
-                if (n >= win.x) dst[n] += src[n];
+            for (int n = win.x + ((lane - win.x) & 31); n <= min(win.y, nt - 1); n += 32)
+                dst[n] += src[n];
         }
     };
     sum_parts(zv, Lp);
