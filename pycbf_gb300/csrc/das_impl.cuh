@@ -380,11 +380,12 @@ __device__ __forceinline__ void weight_range(float w, float &lo, float &hi) {
 // The transmit delays of a pixel beyond kTxReg: a column of shared memory per
 // thread.  Cubic sums keep them as pairs, padded with infinite delays to whole
 // groups of kCubicGroup where that still fits; the padding of the last few
-// sizes below the limit does not, and their last transmits go one by one.
+// sizes below the limit does not, and their last transmits go one by one (an odd
+// one in half a row).
 constexpr size_t kColumnSmemMax = kSmemMax;
 __host__ __device__ inline int cubic_column_padded(int ntx) {
     const int full = (ntx + kCubicGroup - 1) / kCubicGroup * kCubicGroup;
-    return (size_t)full * kBlock * sizeof(float) <= kColumnSmemMax ? full : (ntx + 1) / 2 * 2;
+    return (size_t)full * kBlock * sizeof(float) <= kColumnSmemMax ? full : ntx;
 }
 
 // ---------------------------------------------------------------------------
@@ -840,7 +841,8 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
                 float apod;
                 if (k < ntx) tx_side(k, t.x, apod);
                 if (k + 1 < ntx) tx_side(k + 1, t.y, apod);
-                spair[(size_t)(k >> 1) * kBlock] = t;
+                if (k + 1 < ncol) spair[(size_t)(k >> 1) * kBlock] = t;
+                else stau[(size_t)k * kBlock] = t.x;
             }
         }
     } else {
@@ -1036,7 +1038,9 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
                     rec += kCubicGroup * chs;
                 }
                 for (; g < ntx; ++g) {  // an unpadded column's last transmits; no fast_axis: all
-                    const float2 t = spair[(size_t)(g >> 1) * kBlock];
+                    float2 t = make_float2(0.f, 0.f);
+                    if (g + 1 == ncol && !(g & 1)) t.x = stau[(size_t)g * kBlock];
+                    else t = spair[(size_t)(g >> 1) * kBlock];
                     float w = 1.f;
                     if (GEOM == GEOM_TABBED)
                         w = __fmul_rn(__ldg(a.apodtx + (long long)g * np + i), arx);
