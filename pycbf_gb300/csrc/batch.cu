@@ -166,7 +166,9 @@ batch_das_full_kernel(const BatchJob *__restrict__ jobs, const int2 *__restrict_
         __syncthreads();
         const int geom = s_job.geom, dtype = s_job.dtype;
         for (int sub = 0; sub < tiles_per_item; ++sub) {
-            const long long i = ((long long)it.y * tiles_per_item + sub) * kBlock + threadIdx.x;
+            const long long i0 = ((long long)it.y * tiles_per_item + sub) * kBlock;
+            if (i0 >= s_job.a.np) break;  // past the job's last tile
+            const long long i = i0 + threadIdx.x;
             if (geom == GEOM_TABBED) {
                 if (dtype == PYCBF_GB_F32) batch_pixel<GEOM_TABBED, float>(s_job.a, i, sm);
                 else if (dtype == PYCBF_GB_F16) batch_pixel<GEOM_TABBED, __half>(s_job.a, i, sm);
@@ -211,7 +213,9 @@ batch_das_typed_kernel(const BatchJob *__restrict__ jobs, const int2 *__restrict
         }
         const bool tabbed = s_job.geom == GEOM_TABBED;
         for (int sub = 0; sub < tiles_per_item; ++sub) {
-            const long long i = ((long long)it.y * tiles_per_item + sub) * kBlock + threadIdx.x;
+            const long long i0 = ((long long)it.y * tiles_per_item + sub) * kBlock;
+            if (i0 >= s_job.a.np) break;  // past the job's last tile
+            const long long i = i0 + threadIdx.x;
             if (tabbed) batch_pixel<GEOM_TABBED, T>(s_job.a, i, sm);
             else batch_pixel<GEOM_SYNTH, T>(s_job.a, i, sm);
         }

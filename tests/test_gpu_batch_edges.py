@@ -1,6 +1,7 @@
 """The batch queue at the edges of its work items (GPU)."""
 import numpy as np
 import pytest
+import torch
 
 from pycbf_gb300.batch import BatchBeamformer, BatchConfig
 from test_gpu_rx import _channels, _synthetic, _tabbed
@@ -19,3 +20,20 @@ def test_most_transmits_of_the_queue(make, ntx):
     got = batch([rf])[0].cpu().numpy()
     assert np.abs(got).max() > 0
     np.testing.assert_array_equal(got, bf(rf).ravel())
+
+
+@pytest.mark.parametrize("storages", [("float32",), ("float16",), ("float32", "float16")])
+def test_an_item_ends_with_its_job(storages):
+    """Jobs of one tile in items of one and of eight tiles (a kernel of one storage type and
+    that of several): the same work, so about the same time -- three times allowed, where
+    eight tiles' worth would take eight."""
+    bfs = [_tabbed(40, 64, 100, 301, 2, storage=storages[k % len(storages)]) for k in range(4)]
+    frames = [_channels(bf, 12) for bf in bfs]
+    us, images = [], []
+    for tiles in (1, 8):
+        batch = BatchBeamformer(bfs, config=BatchConfig(tx_chunk=0, tiles_per_item=tiles))
+        images.append([o.clone() for o in batch(frames)])
+        us.append(min(batch.time_config(batch.config, 20) for _ in range(5)))
+    assert us[1] <= 3 * us[0]
+    for a, b in zip(*images):
+        assert torch.equal(a, b)
