@@ -416,8 +416,9 @@ int pycbf_gb_das_tabbed_cubic_noalloc(const pycbf_gb_rfinfo *rf, const void *rfd
 /* are bitwise reproducible.  Apodization is not differentiated.           */
 /* workspace: at least pycbf_gb_adjoint_workspace_bytes bytes, 16-byte      */
 /* aligned; it may be NULL only when grad_rf and pixel_index are both      */
-/* NULL.  With 4 (ntx + nrx) np + 64 bytes more the Synthetic adjoint      */
-/* keeps its delays there instead of computing them per tap (same bits);   */
+/* NULL.  With 4 (ntx + nrx) np + 64 bytes more, where 4 (ntx + nrx) np is */
+/* at most 2^30, the Synthetic adjoint of the channel data keeps its       */
+/* delays there instead of computing them per tap (same bits);             */
 /* 8 (ntx + nrx + 1) np / 128 more serve a grad_rf smaller than that.      */
 /* ---------------------------------------------------------------------- */
 int pycbf_gb_das_synthetic_slowness(const pycbf_gb_rfinfo *rf, const void *coef,

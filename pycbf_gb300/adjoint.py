@@ -81,13 +81,21 @@ def _out_shape(rf4, np_, sumtype):
     return (nf, np_) if sumtype == _lib.SUMTYPE["tx_and_rx"] else (nf, nrx, np_)
 
 
-def _workspace(L, info, np_: int, synthetic: bool, device):
-    """The adjoint's workspace, with room for the tiles' delay ranges and the Synthetic
-    delay tables."""
+_TABLE_MAX = 1 << 30  # bytes of delay tables above which the library makes none
+
+
+def _workspace_bytes(L, info, np_: int, tables: bool) -> int:
+    """The least workspace, the tiles' delay ranges and, where the library makes them, the
+    Synthetic delay tables."""
     nel = info.ntx + info.nrx
     nws = L.pycbf_gb_adjoint_workspace_bytes(ct.byref(info), np_) + 8 * (nel + 1) * ((np_ + 127) // 128) + 64
-    if synthetic:
+    if tables and 4 * nel * np_ <= _TABLE_MAX:
         nws += 4 * nel * np_
+    return nws
+
+
+def _workspace(L, info, np_: int, tables: bool, device):
+    nws = _workspace_bytes(L, info, np_, tables)
     return torch.empty(nws, dtype=torch.uint8, device=device), nws
 
 
@@ -178,7 +186,7 @@ class _SyntheticDAS(torch.autograd.Function):
         g_s = torch.empty_like(slowness) if need_s else None
         ws, nws = None, 0
         if need_rf or ctx.pixel_index is not None:
-            ws, nws = _workspace(L, info, slowness.shape[0], True, dev)
+            ws, nws = _workspace(L, info, slowness.shape[0], need_rf, dev)  # tables: the data's
         if need_rf or need_s:
             st = L.pycbf_gb_das_synthetic_adjoint(
                 ct.byref(info), _ptr(coef), ct.byref(geom_struct), _ptr(slowness),
