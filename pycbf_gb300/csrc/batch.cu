@@ -88,8 +88,11 @@ __device__ __forceinline__ void batch_tile(const DasArgs &a, long long tile) {
                         sum = cubic_taps<GEOM, T, kCubicGroup>(a, tc, tt2 + g / 2, at2 + g / 2, trx,
                                                                arx, rg, (unsigned)chs, sum);
                     else
-                        sum = cubic_taps_clamped<GEOM, T, kCubicGroup>(
-                            a, tt2 + g / 2, at2 + g / 2, trx, arx, rg, chs, sum);
+#pragma unroll
+                        for (int k = 0; k < kCubicGroup; ++k)
+                            sum = cubic_tap_clamped<T, GEOM == GEOM_TABBED>(
+                                a, __fadd_rn(pair_lane(tt2 + g / 2, k), trx),
+                                __fmul_rn(pair_lane(at2 + g / 2, k), arx), rg + k * chs, sum);
                 }
             }
             bacc += CubicAcc<T>::total(sum);
@@ -140,7 +143,7 @@ batch_das_kernel(const BatchJob *__restrict__ jobs, const int2 *__restrict__ ite
 // type's registers apart from the others'.
 template <int GEOM, typename T>
 __device__ __noinline__ void batch_pixel(const DasArgs &a, long long i, float *sm) {
-    das_pixel<GEOM, PYCBF_GB_INTERP_CUBIC, PYCBF_GB_SUM_TX_AND_RX, T, false, kTxSmem>(a, i, 0, sm);
+    das_pixel<GEOM, PYCBF_GB_INTERP_CUBIC, PYCBF_GB_SUM_TX_AND_RX, T, false, kTxSmem, true>(a, i, 0, sm);
 }
 
 // The same queue, each pixel run by the single-frame kernel's body

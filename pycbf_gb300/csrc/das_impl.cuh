@@ -415,8 +415,12 @@ __host__ __device__ inline int cubic_column_padded(int ntx) {
 // A tap that counts has 0 <= j: x >= t0 gives s >= -1/2, which rounds to 0 or
 // more; and j <= nt - 1 where the fast quotient of xmax rounds to at most nt -
 // 1, which the host checks (DasArgs::fast_axis).  On the other time axes (one
-// float step of the delay longer than half a sample) the taps go one by one
-// through cubic_tap_clamped.
+// float step of the delay longer than two samples) the knot is clamped to nt - 1, as the
+// reference clamps it, and 2^29 samples a transmit and more take 64-bit offsets: FAST false.
+// There each tap by itself, with the quotient and a call, made das_kernel 2.7 times as
+// slow as it had been before the packed decisions: nearest, 128 receives, 256 x 512 pixels
+// from 1 s at 40 ns, 11 transmits 342 -> 912 us, now 293; 31 transmits 915 -> 1796, now 586;
+// linear on 129 records of 2^22 samples 225 -> 367, now 179.
 // ---------------------------------------------------------------------------
 constexpr unsigned kKnotBits = 0x4B400000u;  // 1.5 * 2^23 as an integer
 
@@ -464,8 +468,9 @@ struct TapConst {
 };
 
 // delay sums x, knots fj (as floats) and r (kKnotBits + j) of NP pairs of
-// transmits; a NaN or infinite x never counts, whatever its knot
-template <int NP>
+// transmits; a NaN or infinite x never counts, whatever its knot.  FAST false: knots past
+// the record (quotients of nt and more, whose floor the fast one may miss) become its last.
+template <int NP, bool FAST = true>
 __device__ __forceinline__ void knot_pairs(const DasArgs &a, const TapConst &c, const float2 *tt2,
                                            float trx, float2 *x2, float2 *fj2, unsigned *r) {
     const float2 trx2 = make_float2(trx, trx);
@@ -498,6 +503,27 @@ __device__ __forceinline__ void knot_pairs(const DasArgs &a, const TapConst &c, 
             }
         }
     }
+    if (!FAST) {
+        const unsigned last = (unsigned)(a.nt - 1);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            fj2[p].x = fminf(fj2[p].x, (float)last);
+            fj2[p].y = fminf(fj2[p].y, (float)last);
+            r[2 * p] = min(r[2 * p], kKnotBits + last);
+            r[2 * p + 1] = min(r[2 * p + 1], kKnotBits + last);
+        }
+    }
+}
+
+// records between transmits, and the k-th transmit's record r (knot_pairs)
+template <bool FAST> using ChannelStride = typename std::conditional<FAST, unsigned, long long>::type;
+template <typename R>
+__device__ __forceinline__ const R *tap_record(const R *rec, unsigned r, int k, unsigned chs) {
+    return rec + (r + ((unsigned)k * chs - kKnotBits));
+}
+template <typename R>
+__device__ __forceinline__ const R *tap_record(const R *rec, unsigned r, int k, long long chs) {
+    return rec + k * chs + (r - kKnotBits);
 }
 
 // b = (x - xlo) / dt with xlo = fl(t0 + fl(dt j)) for two transmits: the product
@@ -529,8 +555,8 @@ __device__ __forceinline__ float2 half_add(const float4 &c, float2 wy, float2 wz
 }
 
 // One tap with the IEEE quotient and its knot clamped to the channel, added
-// where it counts (time axes without fast_axis, transmits past the last whole
-// group of an unpadded column).
+// where it counts (transmits past the last whole group of an unpadded column, other time
+// axes in a batch).
 template <typename T, bool WEIGHTED>
 __device__ __noinline__ typename CubicAcc<T>::type cubic_tap_clamped(
     const DasArgs &a, float x, float w, const typename CoefRec<T>::raw *rec,
@@ -550,20 +576,20 @@ __device__ __noinline__ typename CubicAcc<T>::type cubic_tap_clamped(
 }
 
 // N taps gathered from global memory: transmits g .. g+N-1 of one receive, rec
-// the channel of transmit g, chs records between transmits (fast_axis: N chs <
-// 2^32).  Padding transmits carry infinite delays, which never count.  The
-// gather is predicated on the tap, so nothing is read for one that does not
-// count; its address is 64-bit rec plus 32-bit (j + k chs) records.
-template <int GEOM, typename T, int N>
+// the channel of transmit g, chs records between transmits.  Padding transmits carry
+// infinite delays, which never count.  The gather is predicated on the tap, so
+// nothing is read for one that does not count; its address is 64-bit rec plus,
+// with FAST (DasArgs::fast_axis: N chs < 2^32), 32-bit (j + k chs) records.
+template <int GEOM, typename T, int N, bool FAST = true>
 __device__ __forceinline__ typename CubicAcc<T>::type cubic_taps(
     const DasArgs &a, const TapConst &c, const float2 *tt2, const float2 *at2, float trx, float arx,
-    const typename CoefRec<T>::raw *rec, unsigned chs, typename CubicAcc<T>::type acc) {
+    const typename CoefRec<T>::raw *rec, ChannelStride<FAST> chs, typename CubicAcc<T>::type acc) {
     using raw = typename CoefRec<T>::raw;
     constexpr int NP = (N + 1) / 2;
     constexpr bool W = GEOM == GEOM_TABBED;
     float2 x2[NP], fj2[NP], w2[NP];
     unsigned r[2 * NP];
-    knot_pairs<NP>(a, c, tt2, trx, x2, fj2, r);
+    knot_pairs<NP, FAST>(a, c, tt2, trx, x2, fj2, r);
     bool ok[N];
     raw pv[N];
 #pragma unroll
@@ -576,7 +602,7 @@ __device__ __forceinline__ typename CubicAcc<T>::type cubic_taps(
             const float x = h ? x2[p].y : x2[p].x;
             ok[k] = (x >= c.t0) && (x <= c.xmax);
             if (W) ok[k] = ok[k] && (fabsf(h ? w2[p].y : w2[p].x) >= c.thresh);
-            if (ok[k]) pv[k] = __ldg(rec + (r[k] + ((unsigned)k * chs - kKnotBits)));
+            if (ok[k]) pv[k] = __ldg(tap_record(rec, r[k], k, chs));
         }
     }
 #pragma unroll
@@ -602,20 +628,6 @@ __device__ __forceinline__ typename CubicAcc<T>::type cubic_taps(
     return acc;
 }
 
-// the same taps one by one (time axes or channel strides without fast_axis)
-template <int GEOM, typename T, int N>
-__device__ __forceinline__ typename CubicAcc<T>::type cubic_taps_clamped(
-    const DasArgs &a, const float2 *tt2, const float2 *at2, float trx, float arx,
-    const typename CoefRec<T>::raw *rec, long long chs, typename CubicAcc<T>::type acc) {
-    constexpr bool W = GEOM == GEOM_TABBED;
-#pragma unroll
-    for (int k = 0; k < N; ++k)
-        acc = cubic_tap_clamped<T, W>(a, __fadd_rn(pair_lane(tt2, k), trx),
-                                      W ? __fmul_rn(pair_lane(at2, k), arx) : 1.f,
-                                      rec + (long long)k * chs, acc);
-    return acc;
-}
-
 // ---------------------------------------------------------------------------
 // Nearest and linear taps summed over the transmits of one receive, as cubic_taps:
 // the decisions of Kind<KIND>::index two transmits at a time, a redo of the taps whose
@@ -624,7 +636,7 @@ __device__ __forceinline__ typename CubicAcc<T>::type cubic_taps_clamped(
 // 251 x 509 pixels, linear 251 -> 164 us, nearest 206 -> 155; 75 Synthetic transmits, 192
 // receives, 128 x 1024 pixels, linear 2.83 -> 1.55 ms, nearest 2.23 -> 1.28.
 // ---------------------------------------------------------------------------
-// one tap, decided with the IEEE quotient (no fast_axis, unpadded columns)
+// one tap, decided with the IEEE quotient (unpadded columns)
 template <int KIND, typename T, bool WEIGHTED>
 __device__ __noinline__ float sample_tap_exact(const DasArgs &a, float x, float w, const T *ch,
                                                float acc) {
@@ -635,16 +647,16 @@ __device__ __noinline__ float sample_tap_exact(const DasArgs &a, float x, float 
     return WEIGHTED ? fmaf(w, v, acc) : acc + v;
 }
 
-template <int GEOM, int KIND, typename T, int N>
+template <int GEOM, int KIND, typename T, int N, bool FAST>
 __device__ __forceinline__ float sample_taps(const DasArgs &a, const TapConst &c, const float2 *tt2,
                                              const float2 *at2, float trx, float arx, const T *rec,
-                                             unsigned chs, float acc) {
+                                             ChannelStride<FAST> chs, float acc) {
     constexpr int NP = (N + 1) / 2;
     constexpr bool W = GEOM == GEOM_TABBED;
     float2 x2[NP], fj2[NP], w2[NP];
     unsigned r[2 * NP];
     if constexpr (KIND == PYCBF_GB_INTERP_LINEAR) {
-        knot_pairs<NP>(a, c, tt2, trx, x2, fj2, r);
+        knot_pairs<NP, FAST>(a, c, tt2, trx, x2, fj2, r);
     } else {
         // it = (int)(q + 1/2): the nearest integer, but 0 for all of -3/2 < q < 1/2
         const float2 trx2 = make_float2(trx, trx);
@@ -690,7 +702,7 @@ __device__ __forceinline__ float sample_taps(const DasArgs &a, const TapConst &c
                                                    : (fj >= -1.f) && (fj <= top);
             if (W) ok[k] = ok[k] && (fabsf(h ? w2[p].y : w2[p].x) >= c.thresh);
             if (ok[k]) {
-                const T *s = rec + (r[k] + ((unsigned)k * chs - kKnotBits));
+                const T *s = tap_record(rec, r[k], k, chs);
                 if constexpr (KIND == PYCBF_GB_INTERP_LINEAR)
                     pv[k] = make_float2(load_sample(s), fj < top ? load_sample(s + 1) : 0.f);
                 else
@@ -722,11 +734,12 @@ template <int GEOM, int KIND, typename T> struct TapSum {
     using Acc = float;
     static __device__ __forceinline__ Acc zero() { return 0.f; }
     static __device__ __forceinline__ float total(Acc v) { return v; }
-    template <int N>
+    template <int N, bool FAST>
     static __device__ __forceinline__ Acc taps(const DasArgs &a, const TapConst &c, const float2 *tt2,
                                                const float2 *at2, float trx, float arx,
-                                               const Rec *rec, unsigned chs, Acc acc) {
-        return sample_taps<GEOM, KIND, T, N>(a, c, tt2, at2, trx, arx, rec, chs, acc);
+                                               const Rec *rec, long long chs, Acc acc) {
+        return sample_taps<GEOM, KIND, T, N, FAST>(a, c, tt2, at2, trx, arx, rec,
+                                                   (ChannelStride<FAST>)chs, acc);
     }
     static __device__ __forceinline__ Acc tap(const DasArgs &a, float x, float w, const Rec *rec,
                                               Acc acc) {
@@ -738,11 +751,12 @@ template <int GEOM, typename T> struct TapSum<GEOM, PYCBF_GB_INTERP_CUBIC, T> {
     using Acc = typename CubicAcc<T>::type;
     static __device__ __forceinline__ Acc zero() { return CubicAcc<T>::zero(); }
     static __device__ __forceinline__ float total(Acc v) { return CubicAcc<T>::total(v); }
-    template <int N>
+    template <int N, bool FAST>
     static __device__ __forceinline__ Acc taps(const DasArgs &a, const TapConst &c, const float2 *tt2,
                                                const float2 *at2, float trx, float arx,
-                                               const Rec *rec, unsigned chs, Acc acc) {
-        return cubic_taps<GEOM, T, N>(a, c, tt2, at2, trx, arx, rec, chs, acc);
+                                               const Rec *rec, long long chs, Acc acc) {
+        return cubic_taps<GEOM, T, N, FAST>(a, c, tt2, at2, trx, arx, rec, (ChannelStride<FAST>)chs,
+                                            acc);
     }
     static __device__ __forceinline__ Acc tap(const DasArgs &a, float x, float w, const Rec *rec,
                                               Acc acc) {
@@ -759,6 +773,9 @@ constexpr int kTxAuto = 0, kTxRegs = 1, kTxSmem = 2;
 // One pixel (table column i of frame f) of the generic delay-and-sum: the
 // body of das_kernel, also run by the batched kernel for each of its jobs.
 // sm: the CTA's dynamic shared memory (das_smem_bytes), a column per thread.
+// FAST: the groups of taps are those of axes with fast_axis, and on others the taps go one
+// by one (the batched kernel: with both forms of the groups it spills, 60 bytes against
+// none); otherwise the groups are those of every axis.
 // cubic, linear and nearest sums over the transmits of a receive take cubic_taps and
 // sample_taps; the rest (census, per-tap outputs, other kinds) the general group
 template <int KIND, int SUM, bool CENSUS> __host__ __device__ constexpr bool fast_sum() {
@@ -767,7 +784,7 @@ template <int KIND, int SUM, bool CENSUS> __host__ __device__ constexpr bool fas
            !CENSUS && SUM != PYCBF_GB_SUM_NONE && SUM != PYCBF_GB_SUM_RX_ONLY;
 }
 
-template <int GEOM, int KIND, int SUM, typename T, bool CENSUS, int TXM = kTxAuto>
+template <int GEOM, int KIND, int SUM, typename T, bool CENSUS, int TXM = kTxAuto, bool FAST = false>
 __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, float *sm) {
     using K = Kind<KIND, T>;
     constexpr bool kFast = fast_sum<KIND, SUM, CENSUS>();
@@ -796,7 +813,7 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
     float *stau = sm + tid;
     float2 *spair = reinterpret_cast<float2 *>(sm) + tid;  // kFast: the column in pairs
     const int ncol = kFast && !in_regs ? cubic_column_padded(ntx) : ntx;
-    const int nfast = a.fast_axis ? ncol / kCubicGroup * kCubicGroup : 0;  // taps by whole groups
+    const int ngroups = FAST && !a.fast_axis ? 0 : ncol / kCubicGroup * kCubicGroup;  // taps by whole groups
     const TapConst tc(a);
     // Tabbed transmit weights beyond kTxReg are read from the table per
     // receive (L1-resident: a tile's rows), which halves the shared memory of
@@ -1007,20 +1024,13 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
                 for (int g = 0; g < kTxReg; g += kCubicGroup) {
                     if (g < ntx) {
                         const Rec *rg = rec + (long long)g * chs;
-                        if (a.fast_axis)
-                            sum = S::template taps<kCubicGroup>(a, tc, tt2 + g / 2, at2 + g / 2, trx,
-                                                                arx, rg, (unsigned)chs, sum);
-                        else
-#pragma unroll
-                            for (int k = 0; k < kCubicGroup; ++k)
-                                sum = S::tap(a, __fadd_rn(pair_lane(tt2 + g / 2, k), trx),
-                                             __fmul_rn(pair_lane(at2 + g / 2, k), arx),
-                                             rg + (long long)k * chs, sum);
+                        sum = S::template taps<kCubicGroup, FAST>(a, tc, tt2 + g / 2, at2 + g / 2,
+                                                                  trx, arx, rg, chs, sum);
                     }
                 }
             } else {
                 int g = 0;
-                for (; g < nfast; g += kCubicGroup) {
+                for (; g < ngroups; g += kCubicGroup) {
                     float2 t2[kCubicGroup / 2], w2[kCubicGroup / 2];
 #pragma unroll
                     for (int p = 0; p < kCubicGroup / 2; ++p) {
@@ -1033,11 +1043,10 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
                         for (int k = 0; k < kCubicGroup; ++k)
                             w[k] = __ldg(a.apodtx + (long long)min(g + k, ntx - 1) * np + i);
                     }
-                    sum = S::template taps<kCubicGroup>(a, tc, t2, w2, trx, arx, rec, (unsigned)chs,
-                                                        sum);
+                    sum = S::template taps<kCubicGroup, FAST>(a, tc, t2, w2, trx, arx, rec, chs, sum);
                     rec += kCubicGroup * chs;
                 }
-                for (; g < ntx; ++g) {  // an unpadded column's last transmits; no fast_axis: all
+                for (; g < ntx; ++g) {  // the others: an unpadded column's last transmits
                     float2 t = make_float2(0.f, 0.f);
                     if (g + 1 == ncol && !(g & 1)) t.x = stau[(size_t)g * kBlock];
                     else t = spair[(size_t)(g >> 1) * kBlock];

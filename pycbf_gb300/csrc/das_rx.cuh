@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(32 * kRxWarps, GEOM == GEOM_TABBED ? 4 : 3)
                     for (int k = 0; k < kCubicGroup; ++k)
                         v[k] = __ldg(a.apodtx + (long long)min(g + k, ntx - 1) * np + i);
                 }
-                sum = S::template taps<kCubicGroup>(a, tc, t2, w2, trx, arx, rec, (unsigned)chs, sum);
+                sum = S::template taps<kCubicGroup, true>(a, tc, t2, w2, trx, arx, rec, chs, sum);
             }
             float v = S::total(sum);
             if (kEach) {

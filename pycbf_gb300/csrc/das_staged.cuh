@@ -743,13 +743,9 @@ __global__ void __launch_bounds__(kBlock, 5) das_staged_kernel(const __grid_cons
 #pragma unroll
                         for (int g = 0; g < kTxReg; g += kTapGroup)
                             if (g < ntx)
-                                sum = a.fast_axis
-                                          ? cubic_taps<GEOM_TABBED, T, kTapGroup>(
-                                                a, tc, tt2 + g / 2, at2 + g / 2, trx, arx,
-                                                rec + (long long)g * chs, (unsigned)chs, sum)
-                                          : cubic_taps_clamped<GEOM_TABBED, T, kTapGroup>(
-                                                a, tt2 + g / 2, at2 + g / 2, trx, arx,
-                                                rec + (long long)g * chs, chs, sum);
+                                sum = cubic_taps<GEOM_TABBED, T, kTapGroup, false>(
+                                    a, tc, tt2 + g / 2, at2 + g / 2, trx, arx, rec + (long long)g * chs,
+                                    chs, sum);
                     }
                     accr = CubicAcc<T>::total(sum);
                 } else {
