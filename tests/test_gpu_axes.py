@@ -70,3 +70,34 @@ def test_long_records_give_the_rows_of_short_ones(kind, ntx, nrx, nt):
     assert float(want.abs().max()) > 0 and torch.equal(rows, want)
     del rf, rows, want
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("kind", ["cubic", "linear", "nearest"])
+@pytest.mark.parametrize("storage", ["float32", "float16"])
+@pytest.mark.parametrize("staged", [True, False])
+@pytest.mark.parametrize("wide", [0.02, 0.5])
+def test_coarse_axes_gather_the_records_of_the_taps(kind, storage, staged, wide):
+    """The images above cannot tell which records a cubic or linear sum read; NaN samples
+    can: 0 x NaN shows in exactly the pixels and receives whose taps ('none', decided one
+    by one) read a record of theirs.  With a staging plan (windows that fit a stage, and
+    longer ones that do not) and without."""
+    ntx, nrx, npx, nt, t0, dt = 5, 70, 333, 2072, 1.0, 5.5e-8
+    r = np.random.default_rng(3)
+    span = nt * dt
+    kw = dict(tautx=t0 + r.uniform(-0.05, 0.6) * span + r.uniform(0, wide, (ntx, npx)) * span,
+              taurx=r.uniform(0, 0.3, (nrx, 1)) * span + r.uniform(0, 0.01, (nrx, npx)) * span,
+              apodtx=r.uniform(-1, 1, (ntx, npx)), apodrx=r.choice([0.0, 0.012, 1.0], (nrx, npx)), t0=t0,
+              dt=dt, nt=nt, interp={"kind": kind}, storage=storage, pixel_order="natural")
+    rf = r.standard_normal((ntx, nrx, nt)).astype(np.float32)
+    for ch in r.integers(0, ntx * nrx, 60):
+        at = r.integers(0, nt)
+        rf.reshape(-1, nt)[ch, at:at + 100] = np.nan
+    rf = torch.as_tensor(rf, device="cuda").to(getattr(torch, storage))
+    taps = pg.TabbedBeamformer(sumtype="none", **kw)(rf).reshape(ntx, nrx, npx)
+    bf = pg.TabbedBeamformer(sumtype="tx_only", stage_channels=staged, **kw)
+    rows = bf(rf).reshape(nrx, npx)
+    want = np.isnan(taps).any(0)
+    assert 0 < want.sum() < want.size
+    np.testing.assert_array_equal(np.isnan(rows), want)
+    if staged:
+        assert bf.kernel_status() == 0
