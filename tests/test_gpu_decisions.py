@@ -1,0 +1,47 @@
+"""Sums over transmits against the sums of their taps (GPU): das_rx_kernel and the kernel of
+several frames decide taps two at a time; sumtype 'none' writes every tap, decided one by
+one by other code."""
+import numpy as np
+import pytest
+import torch
+
+import pycbf_gb300 as pg
+from test_gpu_rx import DT
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind,storage,frames", [
+    ("cubic", "float32", 1), ("cubic", "float16", 1), ("cubic", "bfloat16", 1), ("linear", "float32", 1),
+    ("linear", "float16", 1), ("linear", "bfloat16", 1), ("nearest", "float32", 1), ("nearest", "float16", 1),
+    ("cubic", "float32", 2), ("cubic", "float32", 4), ("cubic", "float16", 8), ("cubic", "bfloat16", 3)])
+@pytest.mark.parametrize("ntx,nrx,npx", [(1, 1, 33), (4, 65, 70), (11, 130, 257), (30, 9, 100)])
+def test_sums_are_those_of_their_taps(kind, storage, frames, ntx, nrx, npx):
+    """Delays on and next to the samples and half-samples, before, at and past both ends,
+    NaN and infinite; weights on either side of the threshold, NaN among them.  A tap's value
+    is at most |w| times 4 samples' worth of products, each rounded a few times, and
+    ntx of them are added in float32: (ntx + 8) 2^-22 of them all."""
+    nt, t0, dt, thresh = 301, 1.3e-7, 4e-8, 0.01
+    r = np.random.default_rng(ntx + nrx)
+    f32 = lambda a: np.asarray(a, np.float32)
+    quant = lambda lo, hi, shape: (r.integers(2 * lo, 2 * hi, shape) / 2 + r.choice([0, 0, 1e-4, -1e-4, 0.3], shape))
+    tautx, taurx = f32(t0 + dt * quant(-30, 200, (ntx, npx))), f32(dt * quant(0, 140, (nrx, npx)))
+    for table in (tautx, taurx):
+        table[r.random(table.shape) < 0.02] = np.nan
+        table[r.random(table.shape) < 0.02] = np.inf
+    apodtx = f32(r.choice([1.0, 0.1, -0.1, 0.0], (ntx, npx)))
+    apodtx[r.random(apodtx.shape) < 0.02] = np.nan
+    edge = np.nextafter(np.float32(0.1), np.float32(1))
+    apodrx = f32(r.choice([1.0, 0.1, float(edge), 0.0999, 0.01, -0.5, 0.0], (nrx, npx)))
+    kw = dict(tautx=tautx, taurx=taurx, apodtx=apodtx, apodrx=apodrx, t0=t0, dt=dt, nt=nt, thresh=thresh,
+              interp={"kind": kind}, storage=storage)
+    rf = torch.as_tensor(r.standard_normal((frames, ntx, nrx, nt)), dtype=torch.float32).to(DT[storage]).cuda()
+    taps = pg.TabbedBeamformer(sumtype="none", **kw)(rf).reshape(frames, ntx, nrx, npx).astype(np.float64)
+    assert np.abs(taps).max() > 0
+    weight = (np.abs(apodtx)[:, None] * np.abs(apodrx)[None]).astype(np.float64)
+    bound = (ntx + 8) * 2.0 ** -22 * 4 * float(rf.float().abs().max()) * np.nansum(weight, 0)
+    rows = pg.TabbedBeamformer(sumtype="tx_only", **kw)(rf).reshape(frames, nrx, npx)
+    assert np.all(np.abs(rows - taps.sum(1)) <= bound)
+    image = pg.TabbedBeamformer(sumtype="tx_and_rx", **kw)(rf).reshape(frames, npx)
+    total = (nrx + 8) * 2.0 ** -23 * np.abs(taps).sum((1, 2)) + bound.sum(0)
+    assert np.all(np.abs(image - taps.sum((1, 2))) <= total)
