@@ -688,7 +688,10 @@ __device__ __forceinline__ float sample_taps(const DasArgs &a, const TapConst &c
         }
     }
     bool ok[N];
-    typename Kind<KIND, T>::P pv[N];
+    // samples as they are stored: a conversion next to the load would wait for it, and with
+    // two samples a tap the loads of a group would go one after another (float16, linear,
+    // 11 transmits, 128 receives, 256 x 512 pixels: 241 us, now 187)
+    T lo[N], hi[N];
     const float top = (float)(a.nt - 1);
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
@@ -703,10 +706,8 @@ __device__ __forceinline__ float sample_taps(const DasArgs &a, const TapConst &c
             if (W) ok[k] = ok[k] && (fabsf(h ? w2[p].y : w2[p].x) >= c.thresh);
             if (ok[k]) {
                 const T *s = tap_record(rec, r[k], k, chs);
-                if constexpr (KIND == PYCBF_GB_INTERP_LINEAR)
-                    pv[k] = make_float2(load_sample(s), fj < top ? load_sample(s + 1) : 0.f);
-                else
-                    pv[k] = load_sample(s);
+                lo[k] = __ldg(s);
+                if (KIND == PYCBF_GB_INTERP_LINEAR) hi[k] = fj < top ? __ldg(s + 1) : T{};
             }
         }
     }
@@ -718,9 +719,9 @@ __device__ __forceinline__ float sample_taps(const DasArgs &a, const TapConst &c
             const float2 K = add2_rn(
                 fma2_rn(c.dt2, make_float2(__fadd_rn(fj, 1.f), fj), c.nz2), c.t02);
             const float2 ab = mul2_rn(sub2_rn(K, make_float2(x, x)), make_float2(c.inv2.x, -c.inv2.x));
-            v = fmaf(ab.x, pv[k].x, ab.y * pv[k].y);
+            v = fmaf(ab.x, load_sample_reg(lo[k]), ab.y * load_sample_reg(hi[k]));
         } else {
-            v = pv[k];
+            v = load_sample_reg(lo[k]);
         }
         if (ok[k]) acc = W ? fmaf(pair_lane(w2, k), v, acc) : acc + v;
     }
