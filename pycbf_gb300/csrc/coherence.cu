@@ -10,8 +10,11 @@ namespace pgb {
 // the pairs (s, s+L) of the separated images are multiplied and summed as
 // sign(p) sqrt|p| (signed square root) or p (power); the reference kernel
 // (pycbf/gpu/__advanced_engines__.cu:17-61) does the same with one thread and
-// one atomicAdd per (lag, s, pixel).
+// one atomicAdd per (lag, s, pixel).  The images of kDmasPairs pairs are loaded
+// together: it waits for its loads, the more so with the few warps that fit
+// beside dmas_short_kernel's ring, whose longer lag lists it serves.
 // ---------------------------------------------------------------------------
+constexpr int kDmasPairs = 8;
 __device__ __forceinline__ void dmas_pixel(const float *__restrict__ im, long long nsep,
                                            long long np, const int *__restrict__ lags, int nlag,
                                            int power, int sumlags, long long ip,
@@ -23,9 +26,21 @@ __device__ __forceinline__ void dmas_pixel(const float *__restrict__ im, long lo
         const long long lag = __ldg(lags + l);
         float acc = 0.f;
         if (lag >= 0) {
-            for (long long s = 0; s + lag < nsep; ++s) {
-                const float p = __fmul_rn(__ldg(col + s * np), __ldg(col + (s + lag) * np));
-                acc += power ? p : copysignf(sqrtf(fabsf(p)), p);
+            const float *a = col, *b = col + lag * np;
+            for (long long left = nsep - lag; left > 0; left -= kDmasPairs) {
+                float u[kDmasPairs], v[kDmasPairs];
+#pragma unroll
+                for (int k = 0; k < kDmasPairs; ++k) {
+                    u[k] = k < left ? __ldg(a) : 0.f;
+                    v[k] = k < left ? __ldg(b) : 0.f;
+                    a += np;
+                    b += np;
+                }
+#pragma unroll
+                for (int k = 0; k < kDmasPairs; ++k) {
+                    const float p = __fmul_rn(u[k], v[k]);
+                    if (k < left) acc += power ? p : copysignf(sqrtf(fabsf(p)), p);
+                }
             }
         }
         if (sumlags) tot += acc;

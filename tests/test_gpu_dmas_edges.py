@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import pycbf_gb300 as pg
+from pycbf_gb300 import _lib
 
 pytestmark = pytest.mark.gpu
 BIG = 3e38
@@ -47,3 +48,34 @@ def test_masked_receive_after_an_infinite_sum(geometry, kind, kw, dmastype):
     rf[..., 1, :] = BIG
     out = bf(rf, out_as_numpy=False)
     assert bool((out == float("inf")).all())
+
+
+@pytest.mark.parametrize("lags", [[40], [30, 60], [0, 1, 25], [-1, 24, 200, 5], [24, 24, 1],
+                                  list(range(10, 26)), list(range(60))])
+@pytest.mark.parametrize("nsep", [1, 7, 8, 41, 128])
+@pytest.mark.parametrize("power", [0, 1])
+@pytest.mark.parametrize("sumlags", [0, 1])
+def test_lag_lists_of_any_length(lags, nsep, power, sumlags):
+    """Lists within and beyond the short kernel's lags, with lags that have no pairs, two
+    frames: at most nsep float32 additions a lag and 60 lags, each product and root rounded
+    a few times, (nsep + 70) 2^-24 of the magnitudes."""
+    npx, nf = 131, 2
+    gen = torch.Generator(device="cuda").manual_seed(nsep)
+    im = torch.randn((nf, nsep, npx), generator=gen, device="cuda")
+    out = torch.full((nf, npx) if sumlags else (nf, len(lags), npx), float("nan"), device="cuda")
+    dev = torch.as_tensor(lags, dtype=torch.int32, device="cuda")
+    L = _lib.load()
+    _lib.check(L.pycbf_gb_dmas(_lib.ptr(im), nf, nsep, npx, _lib.ptr(dev), len(lags), power, sumlags,
+                               _lib.ptr(out), _lib.stream()), "dmas")
+    x = im.double()
+    want, size = [], []
+    for lag in lags:
+        n = max(nsep - lag, 0) if lag >= 0 else 0
+        p = x[:, :n] * x[:, nsep - n:]
+        t = p if power else p.sign() * p.abs().sqrt()
+        want.append(t.sum(1))
+        size.append(t.abs().sum(1))
+    want, size = torch.stack(want, 1), torch.stack(size, 1)
+    if sumlags:
+        want, size = want.sum(1), size.sum(1)
+    assert bool(((out.double() - want).abs() <= (nsep + 70) * 2.0 ** -24 * size).all())
