@@ -137,7 +137,7 @@ bool staged_ok(const pycbf_gb_rfinfo *rf, int interp, int sumtype, const void *d
 int launch_tabbed(const pycbf_gb_rfinfo *rf, DasArgs &a, int interp, int sumtype, const void *plan,
                   cudaStream_t s) {
     if (plan && staged_ok(rf, interp, sumtype, a.data) &&
-        (a.stall_test || !das_rx_ok(a, interp, sumtype))) {
+        (a.stall_test || !a.fast_axis)) {
         if (sumtype == PYCBF_GB_SUM_TX_ONLY) {  // rows of receives no pixel of a tile uses stay 0
             const size_t bytes = sizeof(float) * (size_t)rf->nframes * rf->nrx * (size_t)a.np;
             int st = cuda_status(cudaMemsetAsync(a.out, 0, bytes, s));
@@ -202,7 +202,7 @@ int prepare_data(const pycbf_gb_rfinfo *rf, const void *rfdata, int interp, void
 // frames of that table 0.54 against 0.70 ms; eight 3-D volumes, 3.4 GB, 65 against 57 ms).
 int take_frame_groups(pycbf_gb_rfinfo *rf, const void **rfdata, int geom, DasArgs &a, int sumtype,
                       void **workspace, size_t *workspace_bytes, cudaStream_t s) {
-    if (rf->nframes < 2 || !das_frames_ok(a, sumtype) || !spline_pairs_fit(rf->nt))
+    if (rf->nframes < 2 || !das_frames_ok(a, geom, sumtype) || !spline_pairs_fit(rf->nt))
         return PYCBF_GB_OK;
     if (!*workspace || *workspace_bytes < pycbf_gb_workspace_bytes(rf, PYCBF_GB_INTERP_CUBIC))
         return PYCBF_GB_EWORKSPACE;

@@ -887,7 +887,7 @@ template <typename T>
 static cudaError_t launch_synth_slow_t(const DasArgs &a, int sumtype, cudaStream_t s) {
     constexpr int CU = PYCBF_GB_INTERP_CUBIC, GE = GEOM_SYNTH_SLOW;
     constexpr int BOTH = PYCBF_GB_SUM_TX_AND_RX, EACH = PYCBF_GB_SUM_TX_ONLY;
-    if (das_rx_ok(a, CU, sumtype))
+    if (das_rx_ok(a, GE, CU, sumtype))
         return sumtype == BOTH ? launch_rx_one<GE, CU, BOTH, T>(a, s) : launch_rx_one<GE, CU, EACH, T>(a, s);
     return sumtype == BOTH ? launch_das_one<GE, CU, BOTH, T, false>(a, s)
                            : launch_das_one<GE, CU, EACH, T, false>(a, s);

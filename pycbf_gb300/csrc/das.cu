@@ -20,8 +20,17 @@ cudaError_t launch_das_frames_f32(const DasArgs &, int, int, int, cudaStream_t);
 cudaError_t launch_das_frames_f16(const DasArgs &, int, int, int, cudaStream_t);
 cudaError_t launch_das_frames_bf16(const DasArgs &, int, int, int, cudaStream_t);
 
-bool das_frames_ok(const DasArgs &a, int sumtype) {
-    return a.fast_axis && sumtype != PYCBF_GB_SUM_NONE && sumtype != PYCBF_GB_SUM_RX_ONLY &&
+// Receives enough for the kernels that spread them over warps.  From tables of one or two,
+// most of a CTA's warps would only help to fetch the transmits' column and das_kernel is the
+// faster one: a call of 256 x 512 pixels, 2048 samples, one receive and 13 / 31 / 75 / 300
+// transmits 47 / 49 / 61 / 400 us against 56 / 66 / 97 / 580, two receives 49 / 54 / 71 / 558
+// against 58 / 67 / 108 / 583 (three 51 / 56 / 80 / 694 against 58 / 68 / 112 / 590).
+// Synthetic transmit delays are dearer to compute: 75 of them and one receive 88 us spread
+// over warps or not, 300 215 against 537.
+static bool receives_ok(const DasArgs &a, int geom) { return geom != GEOM_TABBED || a.nrx > 2; }
+
+bool das_frames_ok(const DasArgs &a, int geom, int sumtype) {
+    return a.fast_axis && receives_ok(a, geom) && sumtype != PYCBF_GB_SUM_NONE && sumtype != PYCBF_GB_SUM_RX_ONLY &&
            das_frames_smem(GEOM_TABBED, sumtype, 8, a.ntx) <= kFramesSmemMax;
 }
 
@@ -63,16 +72,17 @@ cudaError_t launch_rx_f16(const DasArgs &, int, int, int, cudaStream_t);
 cudaError_t launch_rx_bf16(const DasArgs &, int, int, int, cudaStream_t);
 
 // Sums over transmits of the kinds with packed decisions, on time axes that allow them
-// (fast_axis), at every size: das_rx_kernel is the faster one throughout (its figures are
-// beside it).  The other axes are das_kernel's and, with a staging plan,
-// das_staged_kernel's (nearest, 11 transmits, 128 receives, 256 x 512 pixels from 1 s at
-// 40 ns: 178 us staged, 293 not).
-bool das_rx_ok(const DasArgs &a, int interp, int sumtype) {
+// (fast_axis): das_rx_kernel is the faster one at every size (its figures are beside it)
+// but the fewest receives.  Those and the other axes are das_kernel's; on other axes with a
+// staging plan, das_staged_kernel's (nearest, 11 transmits, 128 receives, 256 x 512 pixels
+// from 1 s at 40 ns: 178 us staged, 293 not; on ordinary axes with one or two receives the
+// plan's launches cost more than the windows save, 47 against 41 us).
+bool das_rx_ok(const DasArgs &a, int geom, int interp, int sumtype) {
     if (interp != PYCBF_GB_INTERP_CUBIC && interp != PYCBF_GB_INTERP_LINEAR &&
         interp != PYCBF_GB_INTERP_NEAREST)
         return false;
-    return a.fast_axis && sumtype != PYCBF_GB_SUM_NONE && sumtype != PYCBF_GB_SUM_RX_ONLY &&
-           das_rx_smem(GEOM_TABBED, a.ntx, a.nrx) <= kRxSmemMax;
+    return a.fast_axis && receives_ok(a, geom) && sumtype != PYCBF_GB_SUM_NONE &&
+           sumtype != PYCBF_GB_SUM_RX_ONLY && das_rx_smem(GEOM_TABBED, a.ntx, a.nrx) <= kRxSmemMax;
 }
 
 static cudaError_t launch_das_rx(const DasArgs &a, int geom, int interp, int sumtype, int dtype,
@@ -87,7 +97,7 @@ static cudaError_t launch_das_rx(const DasArgs &a, int geom, int interp, int sum
 
 cudaError_t launch_das(const DasArgs &a, int geom, int interp, int sumtype, int dtype, bool census,
                        cudaStream_t s) {
-    if (!census && geom != GEOM_SYNTH_SLOW && das_rx_ok(a, interp, sumtype))
+    if (!census && geom != GEOM_SYNTH_SLOW && das_rx_ok(a, geom, interp, sumtype))
         return launch_das_rx(a, geom, interp, sumtype, dtype, s);
     if (geom == GEOM_TABBED) {
         switch (dtype) {

@@ -854,7 +854,17 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
                 }
             }
         } else {
-            for (int k = 0; k < ncol; k += 2) {
+            int k = 0;
+            constexpr int kAhead = GEOM == GEOM_TABBED ? 4 : 1;  // pairs of table rows in flight
+#pragma unroll kAhead
+            for (; k + 1 < ntx; k += 2) {
+                float2 t;
+                float apod;
+                tx_side(k, t.x, apod);
+                tx_side(k + 1, t.y, apod);
+                spair[(size_t)(k >> 1) * kBlock] = t;
+            }
+            for (; k < ncol; k += 2) {
                 float2 t = make_float2(inf, inf);
                 float apod;
                 if (k < ntx) tx_side(k, t.x, apod);

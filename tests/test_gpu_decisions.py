@@ -45,3 +45,30 @@ def test_sums_are_those_of_their_taps(kind, storage, frames, ntx, nrx, npx):
     image = pg.TabbedBeamformer(sumtype="tx_and_rx", **kw)(rf).reshape(frames, npx)
     total = (nrx + 8) * 2.0 ** -23 * np.abs(taps).sum((1, 2)) + bound.sum(0)
     assert np.all(np.abs(image - taps.sum((1, 2))) <= total)
+
+
+@pytest.mark.parametrize("kind,storage,frames", [
+    ("cubic", "float32", 1), ("cubic", "float16", 1), ("linear", "float32", 1), ("linear", "bfloat16", 1),
+    ("nearest", "float32", 1), ("cubic", "float32", 3), ("cubic", "float16", 2)])
+@pytest.mark.parametrize("sumtype", ["tx_only", "tx_and_rx"])
+@pytest.mark.parametrize("ones", [False, True])
+@pytest.mark.parametrize("ntx,nrx,npx", [(1, 1, 129), (12, 2, 40), (13, 1, 300), (75, 2, 131), (302, 1, 65), (454, 2, 33)])
+def test_few_receives_give_the_rows_of_more(kind, storage, frames, sumtype, ones, ntx, nrx, npx):
+    """One and two receives go to another kernel than three: the sums of a call whose
+    further receives have no weight, bit for bit."""
+    nt, dt = 301, 4e-8
+    r = np.random.default_rng(ntx)
+    more = 3
+    taurx, apodrx = r.uniform(0, 140, (more, npx)) * dt, r.choice([0.0, 0.012, 1.0], (more, npx))
+    apodrx[nrx:] = 0
+    tautx = r.uniform(-30, 200, (ntx, npx)) * dt
+    apodtx = np.ones((ntx, npx)) if ones else r.uniform(-1, 1, (ntx, npx))
+    rf = torch.as_tensor(r.standard_normal((frames, ntx, more, nt)), dtype=torch.float32).to(DT[storage]).cuda()
+    kw = dict(tautx=tautx, apodtx=apodtx, t0=0.0, dt=dt, nt=nt, interp={"kind": kind}, storage=storage,
+              sumtype=sumtype)
+    want = pg.TabbedBeamformer(taurx=taurx, apodrx=apodrx, **kw)(rf)
+    got = pg.TabbedBeamformer(taurx=taurx[:nrx], apodrx=apodrx[:nrx], **kw)(rf[:, :, :nrx].contiguous())
+    if sumtype == "tx_only":
+        want = want.reshape(frames, more, npx)[:, :nrx]
+    assert np.abs(got).max() > 0
+    np.testing.assert_array_equal(got.reshape(want.shape), want)
