@@ -325,7 +325,7 @@ def main_ours(a):
     pidx = ct.c_void_p(bf._pixel_index.data_ptr()) if bf._pixel_index is not None else None
     P = lambda t: ct.c_void_p(t.data_ptr())
     args_spline = (ct.byref(info), P(rf), P(ws), nws)
-    plan = ct.c_void_p(bf._plan.data_ptr()) if bf._plan is not None else None
+    plan = ct.c_void_p(bf._staging_plan.data_ptr()) if bf._staging_plan is not None else None
     args_das = (ct.byref(info), P(ws), P(tautx), P(apodtx), P(taurx), P(apodrx), bf.nop, pidx,
                 ct.c_float(0.01), 3, plan, P(out))
     flush = torch.empty(64 * 1024 * 1024, dtype=torch.float32, device=dev)  # 256 MiB > L2

@@ -164,9 +164,9 @@ int pycbf_gb_spline_coefficients(const pycbf_gb_rfinfo *rf, const void *rfdata, 
 /* locality-friendly order).  plan: NULL, or a staging plan built by       */
 /* pycbf_gb_tabbed_plan for these tables, this thresh and this interp;     */
 /* with it, ntx <= 12 and sumtype tx_only / tx_and_rx / dmas, the kernel   */
-/* for time axes coarser than float32 delays (every tap decided exactly)   */
-/* stages channel windows in shared memory by TMA (same results).  out is  */
-/* written, not accumulated.                                               */
+/* for the time axes of pycbf_gb_tabbed_plan_used stages channel windows   */
+/* in shared memory by TMA (same results).  out is written, not            */
+/* accumulated.                                                            */
 /* ---------------------------------------------------------------------- */
 int pycbf_gb_das_tabbed(const pycbf_gb_rfinfo *rf, const void *rfdata, const float *tautx,
                         const float *apodtx, const float *taurx, const float *apodrx,
@@ -187,6 +187,10 @@ int pycbf_gb_das_tabbed(const pycbf_gb_rfinfo *rf, const void *rfdata, const flo
 /* on the GPU.  Images are sums over blocks of 64 receives (in order) of    */
 /* each block's sequential sum, with or without a plan.                     */
 size_t pycbf_gb_tabbed_plan_bytes(long long np, int ntx, int nrx);
+/* 1 if delay-and-sum calls with this rfinfo and interp read a plan (float32 */
+/* delays in steps of more than two samples, 2^29 samples a transmit and     */
+/* more), 0 if they ignore it.                                               */
+int pycbf_gb_tabbed_plan_used(const pycbf_gb_rfinfo *rf, int interp);
 int pycbf_gb_tabbed_plan(const pycbf_gb_rfinfo *rf, const float *tautx, const float *apodtx,
                          const float *taurx, const float *apodrx, long long np, int interp,
                          float thresh, void *plan, size_t plan_bytes, void *stream);

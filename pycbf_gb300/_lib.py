@@ -27,8 +27,8 @@ SUMTYPE = {"none": 0, "tx_only": 1, "rx_only": 2, "tx_and_rx": 3, "dmas_ssr": 4,
 EXPORTS = (
     "pycbf_gb_abi_version", "pycbf_gb_status_string", "pycbf_gb_last_cuda_error",
     "pycbf_gb_workspace_bytes", "pycbf_gb_spline_coefficients", "pycbf_gb_das_tabbed",
-    "pycbf_gb_das_tabbed_prefiltered", "pycbf_gb_tabbed_plan_bytes", "pycbf_gb_tabbed_plan",
-    "pycbf_gb_das_synthetic", "pycbf_gb_tap_census_tabbed", "pycbf_gb_tap_census_synthetic",
+    "pycbf_gb_das_tabbed_prefiltered", "pycbf_gb_tabbed_plan_bytes", "pycbf_gb_tabbed_plan_used",
+    "pycbf_gb_tabbed_plan", "pycbf_gb_das_synthetic", "pycbf_gb_tap_census_tabbed", "pycbf_gb_tap_census_synthetic",
     "pycbf_gb_synthetic_rx_mask", "pycbf_gb_dmas", "pycbf_gb_slsc", "pycbf_gb_slsc_kept_bytes",
     "pycbf_gb_slsc_kept", "pycbf_gb_slsc_with_kept", "pycbf_gb_fp32_probe",
     "pycbf_gb_das_tabbed_cubic_noalloc", "pycbf_gb_das_synthetic_slowness",
@@ -105,6 +105,7 @@ def load() -> ct.CDLL:
                                           vp, sz, vp]
         L.pycbf_gb_tabbed_plan_bytes.argtypes = [ll, i, i]
         L.pycbf_gb_tabbed_plan_bytes.restype = sz
+        L.pycbf_gb_tabbed_plan_used.argtypes = [P(RFInfo), i]
         L.pycbf_gb_tabbed_plan.argtypes = [P(RFInfo), vp, vp, vp, vp, ll, i, f, vp, sz, vp]
         L.pycbf_gb_das_tabbed_prefiltered.argtypes = [P(RFInfo), vp, vp, vp, vp, vp, ll, vp, f, i,
                                                       vp, vp, vp]

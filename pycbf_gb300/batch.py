@@ -152,7 +152,7 @@ class BatchBeamformer:
             _lib.check(st, "pycbf_gb_spline_coefficients")
             st = L.pycbf_gb_das_tabbed_prefiltered(
                 ct.byref(info), _ptr(coef), _ptr(tautx), _ptr(apodtx), _ptr(taurx), _ptr(apodrx),
-                bf.nop, _ptr(bf._pixel_index), float(np.float32(bf.thresh)), 3, _ptr(bf._plan),
+                bf.nop, _ptr(bf._pixel_index), float(np.float32(bf.thresh)), 3, _ptr(bf._staging_plan),
                 _ptr(out), stream)
             _lib.check(st, "pycbf_gb_das_tabbed_prefiltered")
         else:

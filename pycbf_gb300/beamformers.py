@@ -518,10 +518,22 @@ class TabbedBeamformer(Tabbed, _GPUBeamformer):
             apodtx, apodrx = apodtx[:, perm].contiguous(), apodrx[:, perm].contiguous()
             self._pixel_index = perm.to(torch.int32).contiguous()
         self._tables = (tautx, apodtx, taurx, apodrx)
-        self._plan = None
-        if (self.stage_channels and self.ntx <= 12 and self._interp_code <= _lib.INTERP["cubic"]
-                and self._usf == 1):
-            self._plan = self._build_plan(tautx, apodtx, taurx, apodrx)
+        self._staging_plan = None  # what calls on this time axis read, if anything
+        if self._can_stage() and self._lib.pycbf_gb_tabbed_plan_used(ct.byref(self._rfinfo(1)),
+                                                                     self._interp_code):
+            self._staging_plan = self._build_plan(*self._tables)
+
+    def _can_stage(self):
+        return (self.stage_channels and self.ntx <= 12 and self._interp_code <= _lib.INTERP["cubic"]
+                and self._usf == 1)
+
+    @property
+    def _plan(self):
+        """The staging plan of the tables, None where they cannot have one; on the axes whose
+        calls do not read it, built when first asked for."""
+        if self._staging_plan is None and self._can_stage():
+            self._staging_plan = self._build_plan(*self._tables)
+        return self._staging_plan
 
     def _build_plan(self, tautx, apodtx, taurx, apodrx):
         """The staging plan of these (kernel-order) tables, on the current stream."""
@@ -547,7 +559,7 @@ class TabbedBeamformer(Tabbed, _GPUBeamformer):
         st = self._lib.pycbf_gb_das_tabbed(
             ct.byref(info), _ptr(rf), _ptr(tautx), _ptr(apodtx), _ptr(taurx), _ptr(apodrx),
             self.nop, _ptr(self._pixel_index), self._interp_code, float(np.float32(self.thresh)),
-            sumtype_code, _ptr(self._plan), _ptr(out), _ptr(ws), nws, _stream_ptr())
+            sumtype_code, _ptr(self._staging_plan), _ptr(out), _ptr(ws), nws, _stream_ptr())
         _lib.check(st, "pycbf_gb_das_tabbed")
 
     def differentiable(self, txrxt, tautx=None, taurx=None, sumtype=None):
@@ -568,7 +580,7 @@ class TabbedBeamformer(Tabbed, _GPUBeamformer):
             ktx, kap_tx, krx, kap_rx = self._tables
             return adjoint.das_tabbed(rf, ktx, krx, kap_tx, kap_rx, t0=self.t0, dt=self.dt,
                                       thresh=self.thresh, sumtype=sumtype or self.sumtype,
-                                      pixel_index=self._pixel_index, plan=self._plan)
+                                      pixel_index=self._pixel_index, plan=self._staging_plan)
         # caller-owned delay tables: run in the caller's pixel order, so that
         # no permutation (and no scatter of its gradient) is needed
         ntx_, nap_tx, nrx_, nap_rx = self._natural_tables()
@@ -595,13 +607,13 @@ class TabbedBeamformer(Tabbed, _GPUBeamformer):
     def kernel_status(self) -> int:
         """0, or 1 if a staged launch gave up a bounded wait (its outputs are
         NaN).  Sticky until reset_kernel_status()."""
-        if self._plan is None:
+        if self._staging_plan is None:
             return 0
-        return int(self._plan[:4].view(torch.int32)[0].item())
+        return int(self._staging_plan[:4].view(torch.int32)[0].item())
 
     def reset_kernel_status(self) -> None:
-        if self._plan is not None:
-            self._plan[:4].zero_()
+        if self._staging_plan is not None:
+            self._staging_plan[:4].zero_()
 
     def tap_census(self):
         """Per pixel (original order): contributing taps and the sum of their sample indices."""

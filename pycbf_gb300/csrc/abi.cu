@@ -296,6 +296,15 @@ int pycbf_gb_spline_coefficients(const pycbf_gb_rfinfo *rf, const void *rfdata, 
                         static_cast<cudaStream_t>(stream), &data, &eff);
 }
 
+int pycbf_gb_tabbed_plan_used(const pycbf_gb_rfinfo *rf, int interp) {
+    if (check_rf(rf, false, true) || interp < 0 ||
+        !staged_ok(rf, interp, PYCBF_GB_SUM_TX_AND_RX, nullptr))
+        return 0;
+    DasArgs a = {};
+    fill_time_axis(a, rf);
+    return !a.fast_axis;
+}
+
 size_t pycbf_gb_tabbed_plan_bytes(long long np, int ntx, int nrx) {
     if (np <= 0 || ntx <= 0 || nrx <= 0) return 0;
     return sizeof(int) * (size_t)tabbed_plan_words(np, ntx, nrx);
