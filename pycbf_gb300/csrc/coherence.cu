@@ -67,8 +67,10 @@ dmas_kernel(const float *__restrict__ im, long long nsep, long long np, const in
 // sends the whole launch to the loop above.
 constexpr int kDmasRing = 32, kDmasThreads = 128, kDmasAhead = 8;
 
+// Seven CTAs an SM, as many as the ring allows, are asked for: the general loop would take
+// the registers of the seventh (five lags 59.5 against 58 us).
 template <int NL>
-__global__ void __launch_bounds__(kDmasThreads)
+__global__ void __launch_bounds__(kDmasThreads, NL <= 8 ? 7 : 6)
 dmas_short_kernel(const float *__restrict__ im, long long nsep, long long np,
                   const int *__restrict__ lags, int nlag, int power, int sumlags,
                   float *__restrict__ out) {
