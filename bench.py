@@ -733,11 +733,11 @@ def run_synthetic_variants(a, dev, ctx):
     base_flops = das_flops(contrib, ntx * nrx * np_, delays=(ntx + nrx) * np_)
     K = 2 * 3 + 1
     slsc_flops = np_ * (2 * K * sum(nrx - m for m in range(1, 17)) + 4 * K * nrx)
-    extra = {"synthetic_das": (0, "das_kernel<synthetic, cubic, tx_and_rx, f32> + spline_coef_kernel"),
-             "synthetic_dmas": (3 * np_ * nrx, "das_kernel<synthetic, cubic, dmas_ssr, f32> + "
+    extra = {"synthetic_das": (0, "das_rx_kernel<synthetic, cubic, tx_and_rx, f32> + spline_coef_kernel"),
+             "synthetic_dmas": (3 * np_ * nrx, "das_rx_kernel<synthetic, cubic, dmas_ssr, f32> + "
                                                "spline_coef_kernel (all-pairs sum fused)"),
-             "synthetic_slsc": (slsc_flops, "das_kernel<synthetic, cubic, tx_only, f32> + "
-                                            "slsc_kernel + spline_coef_kernel")}
+             "synthetic_slsc": (slsc_flops, "das_rx_kernel<synthetic, cubic, tx_only, f32> + "
+                                            "slsc_reg_kernel + spline_coef_kernel")}
     launches = {"synthetic_das": 2, "synthetic_dmas": 2, "synthetic_slsc": 3}
     for name, bf in cases.items():
         call = lambda: bf(rf, out_as_numpy=False)
@@ -964,7 +964,7 @@ def run_adjoint_variants(a, w, dev, taps, ctx):
                           "interp": "cubic", "sumtype": "tx_only",
                           "roofline": roofline_of(t_fa, s_bytes, s_flops, ctx["hbm_peak"],
                                                   ctx["fp32_peak"],
-                                                  "spline + das_kernel<slowness> + adj_delay_kernel "
+                                                  "spline + das_rx_kernel<slowness> + adj_delay_kernel "
                                                   "+ adj_scatter_kernel + adj_finalize_kernel")}
     return res
 

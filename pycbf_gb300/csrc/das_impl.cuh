@@ -394,7 +394,7 @@ __host__ __device__ inline int cubic_column_padded(int ntx) {
 //
 // What bounds them is the issue rate: a tap is one gather and a handful of
 // float operations, and the L1 or shared-memory pipe is busy about a third of
-// the time.  So a tap is kept to ~14 instructions:
+// the time.  So a tap is kept to 20 instructions, 14 of them its decisions:
 //   x   = fl(tautx + taurx)                      packed, two transmits each
 //   s   = (x - t0) * 1/dt - 1/2                  packed subtract, packed fma
 //   j   = s rounded to an integer: s + 1.5 * 2^23 holds it in its low bits,

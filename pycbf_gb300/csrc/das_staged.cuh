@@ -1,6 +1,5 @@
 // Tabbed delay-and-sum with channel windows staged in shared memory by TMA, for the
-// time axes whose taps take the exact decisions (das_rx_kernel is the faster one on the
-// others: das.cu).
+// time axes without fast_axis (das_rx_kernel is the faster one on the others: das.cu).
 //
 // The pixels of a CTA (a "tile": 128 consecutive table columns, which the
 // host stores in Morton order of their delays) need, for each (tx, rx)
