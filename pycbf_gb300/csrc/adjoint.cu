@@ -381,7 +381,9 @@ __global__ void __launch_bounds__(kBlock) adj_range_kernel(const __grid_constant
             if (!tx) g.live[(long long)r * tiles + tile] = any ? 1 : 0;
         }
     };
-    for (int t = w; t < a.ntx; t += kWarps) element(t);
+    // every share needs the Tabbed weights; the transmits are the first share's otherwise
+    if (GEOM == GEOM_TABBED || blockIdx.y == 0)
+        for (int t = w; t < a.ntx; t += kWarps) element(t);
     if (GEOM == GEOM_TABBED) {  // the largest weight over every warp's transmits
 #pragma unroll
         for (int m = 0; m < M; ++m) s_amax[w][lane + 32 * m] = amax[m];

@@ -213,8 +213,8 @@ struct DasArgs {
     // of the IEEE quotient
     float eps_fast;
     float neg_zero;     // -0: added to a product in an fma it keeps the product's own rounding
-    // cubic_taps applies: the fast knot of every x <= xmax is at most nt - 1, and a
-    // group's transmits are less than 2^32 records apart
+    // groups of taps need no clamp and 32-bit offsets: the fast knot of every x <= xmax is at
+    // most nt - 1, and a group's transmits are less than 2^32 records apart
     int fast_axis;
     // das_frames_kernel: the receives of this launch (TX_AND_RX: the sum of those
     // before r0, a block boundary, is in out), and whether DMAS sums plain products
