@@ -239,7 +239,7 @@ static_assert(sizeof(BatchJob) + 32 <= kBatchFixedSmem, "");
 
 cudaError_t prepare_batch_das(int max_ntx) {
     const size_t smem = batch_full_smem_bytes(max_ntx);
-    if (smem > kSmemMax) return cudaErrorInvalidValue;
+    if (smem > kSmemMax - kBatchFixedSmem) return cudaErrorInvalidValue;
     cudaError_t err = allow_smem(batch_das_full_kernel, kSmemMax - kBatchFixedSmem);
     if (err == cudaSuccess) err = allow_smem(batch_das_typed_kernel<float>, kSmemMax - kBatchFixedSmem);
     if (err == cudaSuccess) err = allow_smem(batch_das_typed_kernel<__half>, kSmemMax - kBatchFixedSmem);

@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 import torch
 
+from pycbf_gb300 import _lib
 from pycbf_gb300.batch import BatchBeamformer, BatchConfig
 from test_gpu_rx import _channels, _synthetic, _tabbed
 
@@ -20,6 +21,12 @@ def test_most_transmits_of_the_queue(make, ntx):
     got = batch([rf])[0].cpu().numpy()
     assert np.abs(got).max() > 0
     np.testing.assert_array_equal(got, bf(rf).ravel())
+
+
+def test_one_transmit_more_is_refused_when_planned():
+    """Not at the first run: the plan's own call."""
+    with pytest.raises(_lib.GPUError, match="pycbf_gb_batch_plan"):
+        BatchBeamformer([_tabbed(454, 2, 40, 64, 1)], config=BatchConfig(tx_chunk=0))
 
 
 @pytest.mark.parametrize("storages", [("float32",), ("float16",), ("float32", "float16")])
