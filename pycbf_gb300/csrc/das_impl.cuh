@@ -467,6 +467,10 @@ struct TapConst {
           thresh(in_register(a.thresh)) {}
 };
 
+struct NoTapConst {  // for the kernels without groups of taps
+    __device__ __forceinline__ explicit NoTapConst(const DasArgs &) {}
+};
+
 // delay sums x, knots fj (as floats) and r (kKnotBits + j) of NP pairs of
 // transmits; a NaN or infinite x never counts, whatever its knot.  FAST false: knots past
 // the record (quotients of nt and more, whose floor the fast one may miss) become its last.
@@ -792,10 +796,17 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
     constexpr unsigned kFull = 0xffffffffu;
     const int tid = threadIdx.x;
     const long long np = a.np;
-    // threads past the end walk the last pixel along (the receive loop votes per
-    // warp) and write nothing
-    const bool valid = i < np;
-    if (!valid) i = np - 1;
+    // The receive loop votes per warp where it pays: sums by groups of taps, Synthetic
+    // masks of outputs per transmit.  There threads past the end walk the last pixel along
+    // and write nothing.  Elsewhere they leave (a vote and its clamped threads cost outputs
+    // per tap 3 to 10 %: 11 Synthetic transmits, 64 receives, 64 x 128 pixels, nearest 105
+    // us with, 95 without).
+    constexpr bool kVote = kFast || (GEOM == GEOM_SYNTH && SUM != PYCBF_GB_SUM_NONE);
+    const bool valid = !kVote || i < np;
+    if (i >= np) {
+        if (!kVote) return;
+        i = np - 1;
+    }
     const int ntx = a.ntx, nrx = a.nrx;
     const long long op = a.pixel_index ? (long long)__ldg(a.pixel_index + i) : i;
     const bool in_regs = TXM == kTxAuto ? ntx <= kTxReg : TXM == kTxRegs;
@@ -815,7 +826,7 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
     float2 *spair = reinterpret_cast<float2 *>(sm) + tid;  // kFast: the column in pairs
     const int ncol = kFast && !in_regs ? cubic_column_padded(ntx) : ntx;
     const int ngroups = FAST && !a.fast_axis ? 0 : ncol / kCubicGroup * kCubicGroup;  // taps by whole groups
-    const TapConst tc(a);
+    const typename std::conditional<kFast, TapConst, NoTapConst>::type tc(a);
     // Tabbed transmit weights beyond kTxReg are read from the table per
     // receive (L1-resident: a tile's rows), which halves the shared memory of
     // the column form and so raises the CTAs per SM (two -> five at 75 transmits)
@@ -895,7 +906,8 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
     }
     // Tabbed weights beyond kTxReg: one value for every transmit of every pixel of the warp
     // (apodtx all ones), or read from the table per tap
-    const bool one_weight = GEOM == GEOM_TABBED && __all_sync(kFull, amin == atop);
+    bool one_weight = false;
+    if (kFast && GEOM == GEOM_TABBED) one_weight = __all_sync(kFull, amin == atop);
 
     float acc = 0.f, s1 = 0.f;
     float bacc = 0.f;  // TX_AND_RX: sequential sum of the current block of kRxBlockSum receives
@@ -908,7 +920,7 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
             trx = __ldg(a.taurx + (long long)r * np + i);
             arx = __ldg(a.apodrx + (long long)r * np + i);
         } else if (GEOM == GEOM_SYNTH) {
-            trx = synth_rx_delay_warp(a, r, pnt);
+            trx = kVote ? synth_rx_delay_warp(a, r, pnt) : synth_rx_delay(a, r, pnt);
             arx = 1.f;
         } else {
             float D;
@@ -919,7 +931,6 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
     };
     float trx_next = 0.f, arx_next = 0.f;
     if (GEOM == GEOM_TABBED && nrx > 0) rx_side(0, trx_next, arx_next);
-
     for (int r = 0; r < nrx; ++r) {
         if (SUM == PYCBF_GB_SUM_TX_AND_RX && r > 0 && r % kRxBlockSum == 0) {
             acc += bacc;  // the image is the sum of the blocks' sums, in block order
@@ -939,9 +950,9 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
         bool live;
         if (GEOM == GEOM_TABBED) live = __fmul_rn(amax, fabsf(arx)) >= a.thresh;
         else live = trx != inf;
-        // a warp leaves a receive together; the taps of a pixel that it cannot reach
-        // fail their own tests (weight below thresh, infinite delay)
-        if (SUM != PYCBF_GB_SUM_NONE && !__any_sync(kFull, live)) {
+        // a warp that votes leaves a receive together; the taps of a pixel that it cannot
+        // reach fail their own tests (weight below thresh, infinite delay)
+        if (SUM != PYCBF_GB_SUM_NONE && !(kVote ? __any_sync(kFull, live) : live)) {
             if (!CENSUS && SUM == PYCBF_GB_SUM_TX_ONLY && valid)
                 a.out[((long long)f * nrx + r) * np + op] = 0.f;
             continue;
