@@ -73,14 +73,23 @@ __global__ void adj_gather_kernel(const float *__restrict__ gout, const int *__r
 // weights, so a tap is its decisions, a gather, the slope of its cubic and two
 // multiply-adds; otherwise the frames' products are summed per tap, and the knots of
 // other axes are quotients.
-template <int GEOM, int SUM, typename T, bool ONE>
-__global__ void __launch_bounds__(32 * kRxWarps, 4) adj_delay_kernel(const __grid_constant__ AdjArgs g) {
+//
+// WARPS: eight, for tables of up to kFewRx receives four, or one or two for as many
+// receives: each warp's running sums are a column of shared memory, which idle warps would
+// hold too.  The whole call of 75 transmits, 512 samples, 256 x 512 pixels and 1 / 3 / 5 / 8
+// receives 336 / 386 / 489 / 590 us, 458 / 619 / 717 / 810 with eight warps (373 / 482 / 661
+// / 890 with a thread per pixel).
+constexpr int kFewRx = 8;
+template <int WARPS> constexpr int kDelayRun = WARPS < kRxWarps ? WARPS : kRxRun<GEOM_TABBED>;
+
+template <int GEOM, int SUM, typename T, bool ONE, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 32 / WARPS) adj_delay_kernel(const __grid_constant__ AdjArgs g) {
     using rec = typename CoefRec<T>::raw;
-    constexpr int G = kCubicGroup, kRun = kRxRun<GEOM_TABBED>;
+    constexpr int G = kCubicGroup, kRun = kDelayRun<WARPS>;
     constexpr bool W = GEOM == GEOM_TABBED;
     const DasArgs &a = g.d;
     extern __shared__ float2 smp[];
-    __shared__ float s_part[kRxWarps][32];  // largest weights; then dL/dslowness
+    __shared__ float s_part[WARPS][32];  // largest weights; then dL/dslowness
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long np = a.np;
     long long i = (long long)blockIdx.x * 32 + lane;
@@ -91,10 +100,10 @@ __global__ void __launch_bounds__(32 * kRxWarps, 4) adj_delay_kernel(const __gri
     const float inf = __int_as_float(0x7f800000);
     const TapConst tc(a);
     float2 *stau = smp + lane, *sw = stau + (size_t)npair * 32,
-           *sg = sw + (size_t)npair * 32 * (1 + w);  // Tabbed: [kRxWarps][npair][32]
-    float *tabs = reinterpret_cast<float *>(smp + (size_t)npair * 32 * (2 + kRxWarps)) + lane;
+           *sg = sw + (size_t)npair * 32 * (1 + w);  // Tabbed: [WARPS][npair][32]
+    float *tabs = reinterpret_cast<float *>(smp + (size_t)npair * 32 * (2 + WARPS)) + lane;
     auto fetch_run = [&](int r0, int buf) {
-        rx_fetch_run<kRun, kRxWarps>(a, tabs + (size_t)buf * 2 * kRun * 32, r0, min(kRun, nrx - r0), w, i);
+        rx_fetch_run<kRun, WARPS>(a, tabs + (size_t)buf * 2 * kRun * 32, r0, min(kRun, nrx - r0), w, i);
     };
     if (W) fetch_run(0, 0);
 
@@ -105,7 +114,7 @@ __global__ void __launch_bounds__(32 * kRxWarps, 4) adj_delay_kernel(const __gri
         slow = __ldg(a.slow + i);
     }
     float amax = 0.f;
-    for (int p = w; p < npair; p += kRxWarps) {
+    for (int p = w; p < npair; p += WARPS) {
         float tau[2] = {inf, inf}, wt[2] = {0.f, 0.f};  // padding: never counts
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -131,7 +140,7 @@ __global__ void __launch_bounds__(32 * kRxWarps, 4) adj_delay_kernel(const __gri
     __syncthreads();
     if (W) {
 #pragma unroll
-        for (int k = 0; k < kRxWarps; ++k) amax = fmaxf(amax, s_part[k][lane]);
+        for (int k = 0; k < WARPS; ++k) amax = fmaxf(amax, s_part[k][lane]);
     }
     const long long chs = (long long)nrx * nt;
     unsigned off[G];
@@ -140,9 +149,9 @@ __global__ void __launch_bounds__(32 * kRxWarps, 4) adj_delay_kernel(const __gri
 
     const float gpix = nfr == 1 && SUM == PYCBF_GB_SUM_TX_AND_RX ? __ldg(g.gk + i) : 0.f;
     float gs = 0.f;
-    // receive r by warp r % kRxWarps (a run is a multiple of kRxWarps)
+    // receive r by warp r % WARPS (a run is a multiple of WARPS)
     int buf = 1;
-    for (int r = w; r < nrx; r += kRxWarps) {
+    for (int r = w; r < nrx; r += WARPS) {
         float trx, arx = 1.f, Drx = 0.f;
         bool live;
         if (W) {
@@ -292,17 +301,17 @@ __global__ void __launch_bounds__(32 * kRxWarps, 4) adj_delay_kernel(const __gri
     if (!valid) return;
     if (W && g.grad_tautx) {
         const float2 *part = sw + (size_t)npair * 32;
-        for (int p = w; p < npair; p += kRxWarps) {
+        for (int p = w; p < npair; p += WARPS) {
             float2 d = part[(size_t)p * 32];
 #pragma unroll
-            for (int k = 1; k < kRxWarps; ++k) d = add2_rn(d, part[((size_t)k * npair + p) * 32]);
+            for (int k = 1; k < WARPS; ++k) d = add2_rn(d, part[((size_t)k * npair + p) * 32]);
             if (2 * p < ntx) g.grad_tautx[(long long)(2 * p) * np + i] = d.x;
             if (2 * p + 1 < ntx) g.grad_tautx[(long long)(2 * p + 1) * np + i] = d.y;
         }
     }
     if (!W && w == 0 && g.grad_slow) {
 #pragma unroll
-        for (int k = 1; k < kRxWarps; ++k) gs += s_part[k][lane];
+        for (int k = 1; k < WARPS; ++k) gs += s_part[k][lane];
         g.grad_slow[i] = gs;
     }
 }
@@ -694,23 +703,33 @@ adj_finalize_kernel(const float *__restrict__ partial, int nparts, long long nch
 }
 
 
-size_t delay_smem_bytes(int geom, int ntx) {
+template <int WARPS> size_t delay_smem_bytes(int geom, int ntx) {
     const size_t column = (size_t)((ntx + 3) / 4 * 4) * 32 * sizeof(float);
-    return geom == GEOM_TABBED ? (2 + kRxWarps) * column + 4 * kRxRun<GEOM_TABBED> * 32 * sizeof(float)
+    return geom == GEOM_TABBED ? (2 + WARPS) * column + 4 * kDelayRun<WARPS> * 32 * sizeof(float)
                                : 2 * column;
+}
+
+template <int GEOM, int SUM, typename T, int WARPS>
+cudaError_t launch_delay_warps(const AdjArgs &g, cudaStream_t s) {
+    auto kern = g.d.fast_axis && g.d.nframes == 1 ? adj_delay_kernel<GEOM, SUM, T, true, WARPS>
+                                                  : adj_delay_kernel<GEOM, SUM, T, false, WARPS>;
+    const size_t smem = delay_smem_bytes<WARPS>(GEOM, g.d.ntx);
+    if (smem > 40 * 1024) {  // with the static part
+        cudaError_t err = allow_smem(kern, delay_smem_bytes<WARPS>(GEOM, kMaxAdjTx));
+        if (err != cudaSuccess) return err;
+    }
+    kern<<<(unsigned)((g.d.np + 31) / 32), 32 * WARPS, smem, s>>>(g);
+    return cudaGetLastError();
 }
 
 template <int GEOM, int SUM, typename T>
 cudaError_t launch_delay_one(const AdjArgs &g, cudaStream_t s) {
-    auto kern = g.d.fast_axis && g.d.nframes == 1 ? adj_delay_kernel<GEOM, SUM, T, true>
-                                                  : adj_delay_kernel<GEOM, SUM, T, false>;
-    const size_t smem = delay_smem_bytes(GEOM, g.d.ntx);
-    if (smem > 40 * 1024) {  // with the static part
-        cudaError_t err = allow_smem(kern, delay_smem_bytes(GEOM, kMaxAdjTx));
-        if (err != cudaSuccess) return err;
+    if constexpr (GEOM == GEOM_TABBED) {
+        if (g.d.nrx == 1) return launch_delay_warps<GEOM, SUM, T, 1>(g, s);
+        if (g.d.nrx == 2) return launch_delay_warps<GEOM, SUM, T, 2>(g, s);
+        if (g.d.nrx <= kFewRx) return launch_delay_warps<GEOM, SUM, T, 4>(g, s);
     }
-    kern<<<(unsigned)((g.d.np + 31) / 32), 32 * kRxWarps, smem, s>>>(g);
-    return cudaGetLastError();
+    return launch_delay_warps<GEOM, SUM, T, kRxWarps>(g, s);
 }
 
 template <int GEOM, int SUM>
@@ -726,7 +745,7 @@ cudaError_t launch_scatter_one(const AdjArgs &g0, cudaStream_t s) {
     // and a quotient per tap again)
     const bool tables = GEOM == GEOM_TABBED || (g.tau_tx && g.tau_rx);
     constexpr bool kSynth = GEOM != GEOM_TABBED;
-    const dim3 rgrid((unsigned)tiles, 4);
+    const dim3 rgrid((unsigned)tiles, (unsigned)std::min(4, (a.nrx + 3) / 4));
     if (tables) adj_range_kernel<GEOM, kSynth><<<rgrid, kBlock, 0, s>>>(g);
     else adj_range_kernel<GEOM, false><<<rgrid, kBlock, 0, s>>>(g);
     cudaError_t err = cudaGetLastError();

@@ -94,3 +94,36 @@ def test_channel_gradient_of_parts_of_4096_tiles():
     image, g, v = out.detach().double(), g.double(), v.detach().double()
     tol = 1e-4 * float(image.norm()) * float(g.norm()) / npx ** 0.5
     assert abs(float((image * g).sum()) - float((v * grad).sum())) <= tol
+
+
+@pytest.mark.parametrize("nframes", [1, 2])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("sumtype", ["tx_only", "tx_and_rx"])
+@pytest.mark.parametrize("ntx,nrx,npx", [(1, 1, 33), (5, 3, 300), (13, 4, 129), (75, 2, 64), (128, 4, 31), (12, 8, 65), (75, 5, 97)])
+def test_delay_gradients_of_few_receives(nframes, dtype, sumtype, ntx, nrx, npx):
+    """Up to eight receives go to kernels of fewer warps: their delay gradients against those
+    of a call whose further receives have no weight.  A receive's own are the same bits, and
+    up to four receives, one a warp, so are the transmits'; beyond, the receives' terms are
+    added in another order: each sum of n terms is off by at most (n - 1) 2^-24 of the sum of
+    their magnitudes, here those of single-receive calls."""
+    nt, dt, more = 301, 4e-8, 9
+    r = np.random.default_rng(ntx)
+    cuda = lambda a: torch.as_tensor(np.asarray(a, np.float32)).cuda()
+    taurx, apodrx = r.uniform(0, 140, (more, npx)) * dt, r.choice([0.0, 0.02, 1.0], (more, npx))
+    apodrx[nrx:] = 0
+    tautx, apodtx = r.uniform(-30, 200, (ntx, npx)) * dt, r.uniform(-1, 1, (ntx, npx))
+    rf = cuda(r.standard_normal((nframes, ntx, more, nt))).to(DT[dtype])
+    g = cuda(r.standard_normal((nframes, more, npx) if sumtype == "tx_only" else (nframes, npx)))
+
+    def grads(a, b):
+        leaves = [cuda(t).requires_grad_(True) for t in (tautx, taurx[a:b])]
+        out = adjoint.das_tabbed(rf[:, :, a:b].contiguous(), *leaves, cuda(apodtx), cuda(apodrx[a:b]),
+                                 t0=0.0, dt=dt, sumtype=sumtype)
+        up = g[:, a:b].contiguous() if sumtype == "tx_only" else g
+        return torch.autograd.grad(out, leaves, up.reshape(out.shape))
+
+    (few_tx, few_rx), (tx, rx) = grads(0, nrx), grads(0, more)
+    assert float(few_tx.abs().max()) > 0 and float(few_rx.abs().max()) > 0
+    assert torch.equal(few_rx, rx[:nrx])
+    bound = 0 if nrx <= 4 else 2 * (nrx - 1) * 2.0 ** -24 * sum(grads(k, k + 1)[0].abs() for k in range(nrx))
+    assert bool(((few_tx - tx).abs() <= bound).all())
