@@ -796,12 +796,14 @@ __device__ __forceinline__ void das_pixel(const DasArgs &a, long long i, int f, 
     constexpr unsigned kFull = 0xffffffffu;
     const int tid = threadIdx.x;
     const long long np = a.np;
-    // The receive loop votes per warp where it pays: sums by groups of taps, Synthetic
-    // masks of outputs per transmit.  There threads past the end walk the last pixel along
-    // and write nothing.  Elsewhere they leave (a vote and its clamped threads cost outputs
-    // per tap 3 to 10 %: 11 Synthetic transmits, 64 receives, 64 x 128 pixels, nearest 105
-    // us with, 95 without).
-    constexpr bool kVote = kFast || (GEOM == GEOM_SYNTH && SUM != PYCBF_GB_SUM_NONE);
+    // The receive loop votes per warp where it pays: sums by groups of taps, outputs per
+    // transmit (but akima's).  There threads past the end walk the last pixel along and write
+    // nothing.  Elsewhere they leave: a vote and its clamped threads cost outputs per tap 4
+    // to 11 % (11 transmits, 64 receives, 64 x 128 pixels: nearest 103 us with, 91 without,
+    // Synthetic 105 and 95), akima's per transmit 4 % (256 x 512 pixels, 25 transmits 694
+    // and 664; nearest from float16 455 and 470).
+    constexpr bool kVote = kFast || (GEOM == GEOM_SYNTH && SUM != PYCBF_GB_SUM_NONE) ||
+                           (SUM == PYCBF_GB_SUM_RX_ONLY && KIND <= PYCBF_GB_INTERP_CUBIC);
     const bool valid = !kVote || i < np;
     if (i >= np) {
         if (!kVote) return;
