@@ -202,16 +202,17 @@ int prepare_data(const pycbf_gb_rfinfo *rf, const void *rfdata, int interp, void
 // frames of that table 0.54 against 0.70 ms; eight 3-D volumes, 3.4 GB, 65 against 57 ms).
 int take_frame_groups(pycbf_gb_rfinfo *rf, const void **rfdata, int geom, DasArgs &a, int sumtype,
                       void **workspace, size_t *workspace_bytes, cudaStream_t s) {
-    if (rf->nframes < 2 || !das_frames_ok(a, geom, sumtype) || !spline_pairs_fit(rf->nt))
+    const int gdt = rf->dtype == PYCBF_GB_I16 ? PYCBF_GB_F32 : rf->dtype;
+    const size_t nch = (size_t)rf->ntx * rf->nrx, frame = nch * rf->nt;
+    const size_t rec = gdt == PYCBF_GB_F32 ? 16 : 8;
+    const int most = gdt != PYCBF_GB_F32 && 8 * frame * rec <= ((size_t)1 << 30) ? 8 : 4;
+    if (rf->nframes < 2 || !das_frames_ok(a, geom, sumtype, (int)std::min<long long>(most, rf->nframes)) ||
+        !spline_pairs_fit(rf->nt))
         return PYCBF_GB_OK;
     if (!*workspace || *workspace_bytes < pycbf_gb_workspace_bytes(rf, PYCBF_GB_INTERP_CUBIC))
         return PYCBF_GB_EWORKSPACE;
     if (reinterpret_cast<uintptr_t>(*workspace) % 16) return PYCBF_GB_EINVAL;
-    const int gdt = rf->dtype == PYCBF_GB_I16 ? PYCBF_GB_F32 : rf->dtype;
-    const size_t nch = (size_t)rf->ntx * rf->nrx, frame = nch * rf->nt;
-    const size_t rec = gdt == PYCBF_GB_F32 ? 16 : 8;
     const size_t img = sumtype == PYCBF_GB_SUM_TX_ONLY ? (size_t)rf->nrx * a.np : (size_t)a.np;
-    const int most = gdt != PYCBF_GB_F32 && 8 * frame * rec <= ((size_t)1 << 30) ? 8 : 4;
     while (rf->nframes >= 2) {
         int fg = most;
         while (fg > rf->nframes) fg /= 2;

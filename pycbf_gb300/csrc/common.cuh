@@ -239,8 +239,9 @@ cudaError_t launch_das(const DasArgs &a, int geom, int interp, int sumtype, int 
                        cudaStream_t s);
 // whether launch_das takes das_rx_kernel (but for a slowness geometry)
 bool das_rx_ok(const DasArgs &a, int geom, int interp, int sumtype);
-// cubic sums over transmits of a.nframes frames (a multiple of fg) from grouped records
-bool das_frames_ok(const DasArgs &a, int geom, int sumtype);
+// cubic sums over transmits of a.nframes frames (a multiple of fg) from grouped records; ok:
+// whether they are to be taken, in groups of up to `group`
+bool das_frames_ok(const DasArgs &a, int geom, int sumtype, int group);
 cudaError_t launch_das_frames(const DasArgs &a, int geom, int sumtype, int dtype, int fg,
                               cudaStream_t s);
 cudaError_t launch_synth_rx_mask(const DasArgs &a, unsigned char *mask, cudaStream_t s);

@@ -20,17 +20,46 @@ cudaError_t launch_das_frames_f32(const DasArgs &, int, int, int, cudaStream_t);
 cudaError_t launch_das_frames_f16(const DasArgs &, int, int, int, cudaStream_t);
 cudaError_t launch_das_frames_bf16(const DasArgs &, int, int, int, cudaStream_t);
 
-// Receives enough for the kernels that spread them over warps.  From tables of one or two,
-// most of a CTA's warps would only help to fetch the transmits' column and das_kernel is the
-// faster one: a call of 256 x 512 pixels, 2048 samples, one receive and 13 / 31 / 75 / 300
-// transmits 47 / 49 / 61 / 400 us against 56 / 66 / 97 / 580, two receives 49 / 54 / 71 / 558
-// against 58 / 67 / 108 / 583 (three 51 / 56 / 80 / 694 against 58 / 68 / 112 / 590).
-// Synthetic transmit delays are dearer to compute: 75 of them and one receive 88 us spread
-// over warps or not, 300 215 against 537.
-static bool receives_ok(const DasArgs &a, int geom) { return geom != GEOM_TABBED || a.nrx > 2; }
+// The kernels that spread a pixel's receives over warps (das_rx_kernel, das_frames_kernel)
+// fill the GPU from few pixels and hide latency with many receives.  With few receives on an
+// image that fills it anyway most of their warps only help to fetch the transmits' column,
+// and das_kernel, a thread per pixel, is the faster one: up to kFewRx receives that grow with
+// the pixels (it walks them one after another).  us of a call, 2048 samples, das_kernel /
+// das_rx_kernel:
+//   tables      pixels   receives 1         4         8        16
+//   5 tx        128 x 256   15 / 18   18 / 19   20 / 19   25 / 21
+//               256 x 512   17 / 29   21 / 31   25 / 33   33 / 37
+//              512 x 1024   26 / 68   35 / 78   46 / 84   90 / 115   (24 receives 144 / 138)
+//   75 tx       128 x 256   25 / 31   45 / 37   69 / 40  124 / 55
+//               256 x 512   37 / 78  70 / 103 114 / 127 204 / 160
+//              512 x 1024 105 / 296 172 / 376 256 / 436 448 / 518     (24 receives 625 / 621)
+//   300 tx      256 x 512 373 / 580 740 / 708
+//   Synthetic, 5 / 75 tx, 256 x 512 pixels, 4 receives 25 / 31 and 96 / 78 (every thread
+//   computes its own transmit delays there: the more of them, the fewer receives)
+// Up to twelve transmits and 16 to 64 receives on 512 x 1024 pixels and more are faster from
+// staged windows than with either (5 transmits, 24 receives 103 us), but a staging plan
+// holds the launch's queue, so it serves one stream at a time, and takes 64 bytes a tile and
+// receive.
+static bool few_receives(const DasArgs &a, int geom) {
+    constexpr long long kFewRx = 16;
+    const long long px = a.np * a.nframes, rx = a.nrx, tx = a.ntx;
+    if (geom == GEOM_SYNTH_SLOW) return false;  // 2 receives 423 us spread over warps, 450 not
+    const bool regs = tx <= kTxReg;  // no column of shared memory: more warps an SM
+    if (geom == GEOM_TABBED)
+        return rx == 1 || (rx <= kFewRx && rx * (regs ? 8192 : 128 * std::max(tx, 128LL)) <= px);
+    // Synthetic: 48 receives of 5 transmits at 512 x 1024 pixels 176 us on either, 64 225 / 215
+    return px >= 40000 && tx <= 100 && rx <= 48 && rx * (regs ? 8192 : 1365 * tx) <= px;
+}
 
-bool das_frames_ok(const DasArgs &a, int geom, int sumtype) {
-    return a.fast_axis && receives_ok(a, geom) && sumtype != PYCBF_GB_SUM_NONE && sumtype != PYCBF_GB_SUM_RX_ONLY &&
+// Groups of frames share the decisions of a tap, so das_kernel is left fewer receives: groups
+// of two or four float32 frames, 11 transmits, 256 x 512 pixels, 8 receives 42 / 44 and 64 /
+// 66 us a call, 16 receives 63 / 53 and 105 / 76; of eight float16 frames, 2 receives 60 / 60,
+// 4 82 / 68; three frames, two launches each of two kernels, 128 x 128 pixels, 5 transmits, 2
+// receives 16 / 31.  Synthetic groups are the faster ones throughout.
+bool das_frames_ok(const DasArgs &a, int geom, int sumtype, int group) {
+    const long long few = group == 8 ? 2 : a.nframes == 3 ? 8 : std::max(2LL, std::min(a.np / 16384, 8LL));
+    if (geom == GEOM_TABBED && a.nrx <= few) return false;
+    return a.fast_axis && sumtype != PYCBF_GB_SUM_NONE && sumtype != PYCBF_GB_SUM_RX_ONLY &&
            das_frames_smem(GEOM_TABBED, sumtype, 8, a.ntx) <= kFramesSmemMax;
 }
 
@@ -72,16 +101,15 @@ cudaError_t launch_rx_f16(const DasArgs &, int, int, int, cudaStream_t);
 cudaError_t launch_rx_bf16(const DasArgs &, int, int, int, cudaStream_t);
 
 // Sums over transmits of the kinds with packed decisions, on time axes that allow them
-// (fast_axis): das_rx_kernel is the faster one at every size (its figures are beside it)
-// but the fewest receives.  Those and the other axes are das_kernel's; on other axes with a
-// staging plan, das_staged_kernel's (nearest, 11 transmits, 128 receives, 256 x 512 pixels
-// from 1 s at 40 ns: 178 us staged, 293 not; on ordinary axes with one or two receives the
-// plan's launches cost more than the windows save, 47 against 41 us).
+// (fast_axis): das_rx_kernel's (its figures are beside it) but for few receives.  Those and
+// the other axes are das_kernel's; on other axes with a staging plan, das_staged_kernel's
+// (nearest, 11 transmits, 128 receives, 256 x 512 pixels from 1 s at 40 ns: 178 us staged,
+// 293 not).
 bool das_rx_ok(const DasArgs &a, int geom, int interp, int sumtype) {
     if (interp != PYCBF_GB_INTERP_CUBIC && interp != PYCBF_GB_INTERP_LINEAR &&
         interp != PYCBF_GB_INTERP_NEAREST)
         return false;
-    return a.fast_axis && receives_ok(a, geom) && sumtype != PYCBF_GB_SUM_NONE &&
+    return a.fast_axis && !few_receives(a, geom) && sumtype != PYCBF_GB_SUM_NONE &&
            sumtype != PYCBF_GB_SUM_RX_ONLY && das_rx_smem(GEOM_TABBED, a.ntx, a.nrx) <= kRxSmemMax;
 }
 

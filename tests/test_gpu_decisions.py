@@ -72,3 +72,45 @@ def test_few_receives_give_the_rows_of_more(kind, storage, frames, sumtype, ones
         want = want.reshape(frames, more, npx)[:, :nrx]
     assert np.abs(got).max() > 0
     np.testing.assert_array_equal(got.reshape(want.shape), want)
+
+
+@pytest.mark.parametrize("kind,storage,frames", [
+    ("cubic", "float32", 1), ("cubic", "float16", 1), ("linear", "float32", 1), ("nearest", "float32", 1),
+    ("nearest", "float32", 2), ("cubic", "float32", 2), ("cubic", "float16", 8)])
+@pytest.mark.parametrize("geom,ntx,npx,few", [
+    ("tabbed", 12, 16384, 2), ("tabbed", 13, 32767, 1), ("tabbed", 13, 32769, 2), ("tabbed", 140, 53760, 3),
+    ("synthetic", 5, 40001, 4), ("synthetic", 31, 84630, 2)])
+def test_receives_that_fit_one_thread_give_the_rows_of_more(kind, storage, frames, geom, ntx, npx, few):
+    """How many receives one thread a pixel walks goes by the pixels and transmits; beyond, they
+    are spread over warps: the sums per receive on both sides of that number, and the images
+    as the sums of those, bit for bit."""
+    nt, dt = 301, 4e-8
+    r = np.random.default_rng(ntx)
+    common = dict(t0=0.0, dt=dt, nt=nt, interp={"kind": kind}, storage=storage, pixel_order="natural")
+    xe = 3e-4 * (np.arange(few + 1) - few / 2)
+    tables = dict(tautx=r.uniform(-30, 200, (ntx, npx)) * dt, apodtx=r.uniform(-1, 1, (ntx, npx)))
+    taurx, apodrx = r.uniform(0, 140, (few + 1, npx)) * dt, r.choice([0.0, 0.012, 1.0], (few + 1, npx))
+    pnts = np.stack([r.uniform(-1e-3, 1e-3, npx), r.uniform(1e-3, 8e-3, npx)], 1)
+    up = np.array([0.0, 1.0])
+
+    def run(nrx, sumtype):
+        if geom == "tabbed":
+            bf = pg.TabbedBeamformer(taurx=taurx[:nrx], apodrx=apodrx[:nrx], sumtype=sumtype, **tables, **common)
+        else:
+            src = np.stack([np.linspace(-4e-3, 4e-3, ntx), np.full(ntx, -8e-3)], 1)
+            bf = pg.SyntheticBeamformer(
+                ovectx=src, nvectx=np.tile(up, (ntx, 1)), doftx=np.zeros(ntx), alatx=np.full(ntx, 0.9),
+                t0tx=np.full(ntx, -8e-3 / 1540), ovecrx=np.stack([xe[:nrx], np.zeros(nrx)], 1),
+                nvecrx=np.tile(up, (nrx, 1)), alarx=np.full(nrx, 0.45), c0=1540.0, pnts=pnts, sumtype=sumtype,
+                **common)
+        return bf(rf[:, :, :nrx].contiguous()).reshape((frames, nrx, npx) if sumtype == "tx_only" else (frames, npx))
+
+    rf = torch.as_tensor(r.standard_normal((frames, ntx, few + 1, nt)), dtype=torch.float32).to(DT[storage]).cuda()
+    more = run(few + 1, "tx_only")
+    assert np.abs(more).max(axis=(0, 2)).min() > 0
+    np.testing.assert_array_equal(run(few, "tx_only"), more[:, :few])
+    for nrx in (few, few + 1):
+        image = np.zeros((frames, npx), np.float32)
+        for k in range(nrx):
+            image = image + more[:, k]
+        np.testing.assert_array_equal(run(nrx, "tx_and_rx"), image)
