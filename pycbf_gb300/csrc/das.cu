@@ -23,9 +23,9 @@ cudaError_t launch_das_frames_bf16(const DasArgs &, int, int, int, cudaStream_t)
 // The kernels that spread a pixel's receives over warps (das_rx_kernel, das_frames_kernel)
 // fill the GPU from few pixels and hide latency with many receives.  With few receives on an
 // image that fills it anyway most of their warps only help to fetch the transmits' column,
-// and das_kernel, a thread per pixel, is the faster one: up to kFewRx receives that grow with
-// the pixels (it walks them one after another).  us of a call, 2048 samples, das_kernel /
-// das_rx_kernel:
+// and das_kernel, a thread per pixel, is the faster one: up to 16 receives, more of them the
+// more pixels there are (it walks them one after another) and fewer the longer the column of
+// transmits that each thread holds.  us of a call, 2048 samples, das_kernel / das_rx_kernel:
 //   tables      pixels   receives 1         4         8        16
 //   5 tx        128 x 256   15 / 18   18 / 19   20 / 19   25 / 21
 //               256 x 512   17 / 29   21 / 31   25 / 33   33 / 37
@@ -33,6 +33,8 @@ cudaError_t launch_das_frames_bf16(const DasArgs &, int, int, int, cudaStream_t)
 //   75 tx       128 x 256   25 / 31   45 / 37   69 / 40  124 / 55
 //               256 x 512   37 / 78  70 / 103 114 / 127 204 / 160
 //              512 x 1024 105 / 296 172 / 376 256 / 436 448 / 518     (24 receives 625 / 621)
+//   200 tx      256 x 512          286 / 345 447 / 408
+//              512 x 1024          822 / 1165 1234 / 1366 2142 / 1607
 //   300 tx      256 x 512 373 / 580 740 / 708
 //   Synthetic, 5 / 75 tx, 256 x 512 pixels, 4 receives 25 / 31 and 96 / 78 (every thread
 //   computes its own transmit delays there: the more of them, the fewer receives)
@@ -41,12 +43,13 @@ cudaError_t launch_das_frames_bf16(const DasArgs &, int, int, int, cudaStream_t)
 // holds the launch's queue, so it serves one stream at a time, and takes 64 bytes a tile and
 // receive.
 static bool few_receives(const DasArgs &a, int geom) {
-    constexpr long long kFewRx = 16;
     const long long px = a.np * a.nframes, rx = a.nrx, tx = a.ntx;
-    if (geom == GEOM_SYNTH_SLOW) return false;  // 2 receives 423 us spread over warps, 450 not
+    if (geom == GEOM_SYNTH_SLOW) return false;  // gradients of the slowness: the rest of the step is far larger
     const bool regs = tx <= kTxReg;  // no column of shared memory: more warps an SM
-    if (geom == GEOM_TABBED)
-        return rx == 1 || (rx <= kFewRx && rx * (regs ? 8192 : 128 * std::max(tx, 128LL)) <= px);
+    if (geom == GEOM_TABBED) {
+        const long long each = regs ? 8192 : rx == 2 ? 12288 : std::max(12288LL, 160 * tx - 8192);
+        return rx == 1 || (rx <= std::min(16LL, std::max(2LL, 1500 / tx)) && rx * each <= px);
+    }
     // Synthetic: 48 receives of 5 transmits at 512 x 1024 pixels 176 us on either, 64 225 / 215
     return px >= 40000 && tx <= 100 && rx <= 48 && rx * (regs ? 8192 : 1365 * tx) <= px;
 }
@@ -54,10 +57,11 @@ static bool few_receives(const DasArgs &a, int geom) {
 // Groups of frames share the decisions of a tap, so das_kernel is left fewer receives: groups
 // of two or four float32 frames, 11 transmits, 256 x 512 pixels, 8 receives 42 / 44 and 64 /
 // 66 us a call, 16 receives 63 / 53 and 105 / 76; of eight float16 frames, 2 receives 60 / 60,
-// 4 82 / 68; three frames, two launches each of two kernels, 128 x 128 pixels, 5 transmits, 2
-// receives 16 / 31.  Synthetic groups are the faster ones throughout.
+// 4 82 / 68.  Three, five or seven frames are two or three launches each of two kernels: three,
+// 128 x 128 pixels, 5 transmits, 2 receives 16 / 31.  Synthetic groups are the faster ones throughout.
 bool das_frames_ok(const DasArgs &a, int geom, int sumtype, int group) {
-    const long long few = group == 8 ? 2 : a.nframes == 3 ? 8 : std::max(2LL, std::min(a.np / 16384, 8LL));
+    const bool odd = a.nframes < 8 && a.nframes % 2;
+    const long long few = group == 8 ? 2 : odd ? 8 : std::max(2LL, std::min(a.np / 16384, 8LL));
     if (geom == GEOM_TABBED && a.nrx <= few) return false;
     return a.fast_axis && sumtype != PYCBF_GB_SUM_NONE && sumtype != PYCBF_GB_SUM_RX_ONLY &&
            das_frames_smem(GEOM_TABBED, sumtype, 8, a.ntx) <= kFramesSmemMax;

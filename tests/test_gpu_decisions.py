@@ -78,7 +78,7 @@ def test_few_receives_give_the_rows_of_more(kind, storage, frames, sumtype, ones
     ("cubic", "float32", 1), ("cubic", "float16", 1), ("linear", "float32", 1), ("nearest", "float32", 1),
     ("nearest", "float32", 2), ("cubic", "float32", 2), ("cubic", "float16", 8)])
 @pytest.mark.parametrize("geom,ntx,npx,few", [
-    ("tabbed", 12, 16384, 2), ("tabbed", 13, 32767, 1), ("tabbed", 13, 32769, 2), ("tabbed", 140, 53760, 3),
+    ("tabbed", 12, 16384, 2), ("tabbed", 13, 24575, 1), ("tabbed", 13, 24577, 2), ("tabbed", 140, 42624, 3),
     ("synthetic", 5, 40001, 4), ("synthetic", 31, 84630, 2)])
 def test_receives_that_fit_one_thread_give_the_rows_of_more(kind, storage, frames, geom, ntx, npx, few):
     """How many receives one thread a pixel walks goes by the pixels and transmits; beyond, they
